@@ -13,8 +13,9 @@
 //   WG3        correction.  Thread r owns the FP32 output row r in registers (as packed FP32 pairs)
 //              and everything that is sequential over tiles: running maximum, denominator, per-tile
 //              weights, O = O * o_scale + float(P.V) * w, capture statistics, epilogue and store.
-//   WG4        warp 16: TMA producer (Q, K ring, V ring); warp 17: one thread issues the QK^T MMAs,
-//              up to four tiles ahead of the read-back; warp 18: one thread issues the P.V MMAs.
+//   WG4        warp 16: TMA producer (Q, K ring, V ring); warp 17: issues the QK^T MMAs, up to four
+//              tiles ahead of the read-back; warp 18: issues the P.V MMAs.  Both walk their loop as
+//              whole converged warps and elect one lane for the MMAs.
 // Tensor memory (512 columns) is four accumulator buffers of 128 columns.  Tile it owns buffer
 // it % 4 from its Q.K^T until its P.V result has been read back: the scores are written there, the
 // softmax group reads them, P.V overwrites the same columns and the correction group takes the
@@ -50,6 +51,7 @@ constexpr int kVStages = 3;           // V ring depth
 constexpr int kTile = 128 * 128;      // bytes of one 128 x 128 INT8 tile
 constexpr int kThreads = 640;
 constexpr int kSoftmaxGroups = 3;     // softmax warpgroups; tile it is handled by group it % 3
+constexpr int kIssueWarp = 16;        // producer; +1 issues Q.K^T (and owns tensor memory), +2 P.V
 constexpr int kBuffers = 4;           // tensor-memory accumulator buffers; tile it uses it % 4
 // What a launch produces besides the output: nothing, the reference's capture workspace, or the
 // retained-mass selection of every query block.
@@ -101,7 +103,7 @@ struct SmemLayout {
   static constexpr int rowstate = mask_stage + kMaskStageBytes;  // float [5][128]: m, d[4] (capture)
   static constexpr int v_affine = rowstate + 5 * 128 * 4;  // float [2][128]: V scales, V centres
   static constexpr int bars = v_affine + 2 * 128 * 4;      // 8-byte mbarriers
-  static constexpr int n_bars = 1 + 2 * kKStages + 2 * kVStages + 7 * 4 + 3;  // one spare
+  static constexpr int n_bars = 1 + 2 * kKStages + 2 * kVStages + 6 * 4 + 3;  // one spare
   static constexpr int tmem_slot = bars + n_bars * 8;
   static constexpr int gave_up = tmem_slot + 8;            // site of the first expired wait, or 0
   static constexpr int total = tmem_slot + 16;
@@ -161,8 +163,8 @@ struct Bars {
   uint32_t base;
   static constexpr int QFULL = 0, KFULL = 1, KEMPTY = KFULL + kKStages, VFULL = KEMPTY + kKStages,
                        VEMPTY = VFULL + kVStages, SFULL = VEMPTY + kVStages,
-                       BUFFREE = SFULL + kBuffers, PFULL = BUFFREE + kBuffers, PFREE = PFULL + 4,
-                       OFULL = PFREE + 4, STATFREE = OFULL + kBuffers, WFULL = STATFREE + 4,
+                       BUFFREE = SFULL + kBuffers, PFULL = BUFFREE + kBuffers, SLOTFREE = PFULL + 4,
+                       OFULL = SLOTFREE + 4, WFULL = OFULL + kBuffers,
                        PAIRS = WFULL + 4;  // two: the selection epilogue's bulk copies
   // Tensor memory is four accumulator buffers of 128 columns; tile it owns buffer it % 4 for its
   // whole life: Q.K^T writes the scores there (SFULL), the softmax group reads them, P.V then
@@ -170,7 +172,12 @@ struct Bars {
   // hands the buffer back once it has it in registers (BUFFREE).  Three tiles can be in the
   // softmax stage while a fourth is in P.V / read-back, so no stage waits for another tile's
   // accumulator.  The probability tiles and the per-row statistics have four slots
-  // (it % L::kSlots).
+  // (it % L::kSlots), handed back together (SLOTFREE) by the correction group when it has read the
+  // statistics: it does that after P.V of the tile has completed, so the probabilities are free too.
+  // Where a warpgroup hands something over its warps arrive once each (mbar_arrive_warp): 4 arrivals
+  // on the barrier's word instead of 128.
+  // Measured with the uniform issue warps below, dense 32K (B1 Hq16 Hkv4 D128): 6.50 -> 6.39 ms of
+  // attention, 65536 64-key tiles with a bias at head_dim 64 0.91 -> 0.82 ms.
   __device__ __forceinline__ uint32_t operator()(int i) const { return base + 8u * i; }
 };
 
@@ -192,8 +199,6 @@ __device__ __forceinline__ void softmax_tile_int(uint32_t tmem_row, const float 
                                                  uint16_t* sums, PackMultipliers mul,
                                                  int max_floor = INT_MIN,
                                                  const uint32_t* keep = nullptr) {
-  // (With kScoresInt the bits mark the keys that exist in a ragged last tile; the others go into
-  // the exponent pass as -1e30, the value the general path gives them.)
   // Pass 1 lands two 32-column chunks per wait (nothing else is live yet, so 64 landing registers
   // are free); pass 2 walks the chunks backwards so that it starts on chunk 3, which is still in
   // registers, and every later chunk is fetched underneath the previous chunk's exponentials.
@@ -253,7 +258,7 @@ __device__ __forceinline__ void softmax_tile_int(uint32_t tmem_row, const float 
     if constexpr (KEEPBITS) {
 #pragma unroll
       for (int i = 0; i < 32; ++i)
-        if (((keep[c] >> i) & 1u) == 0u) x[i] = KIND == kScoresScaled ? -INFINITY : -1.0e30f;
+        if (((keep[c] >> i) & 1u) == 0u) x[i] = -INFINITY;
     }
     if (c > 0) tmem_load32(tmem_row + 32 * (c - 1), raw);
     uint32_t P[8], s4[8];
@@ -583,10 +588,9 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
   // 0 every path; 1 boolean per-query masks read as bits; 2 no mask, not causal, positive scale;
   // 3 causal without mask, positive scale; 4 any other per-query mask; 5 masks broadcast over the
   // queries (their entries are read as 16-byte pieces shared by all rows); 6 as 2 with a key length
-  // that is a whole number of tiles (no ragged last tile: the integer fast path alone); 7 as 2 with
-  // a ragged last tile, which takes the integer fast path with the existing keys marked by bits.
-  constexpr bool BOOLROWS = VARIANT == 1, WHOLE = VARIANT == 6, RAGGED = VARIANT == 7,
-                 PLAIN = VARIANT == 2 || WHOLE || RAGGED, CAUSAL = VARIANT == 3,
+  // that is a whole number of tiles (no ragged last tile: the integer fast path alone).
+  constexpr bool BOOLROWS = VARIANT == 1, WHOLE = VARIANT == 6,
+                 PLAIN = VARIANT == 2 || WHOLE, CAUSAL = VARIANT == 3,
                  MASKED = VARIANT == 4, KEYMASK = VARIANT == 5;
   constexpr bool kHasInt = VARIANT == 0 || PLAIN, kHasScaled = VARIANT == 0 || CAUSAL,
                  kHasMasked = VARIANT == 0 || BOOLROWS || MASKED || KEYMASK,
@@ -596,7 +600,10 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t sbase = smem_u32(smem);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // (the shuffle tells the compiler that the warp index is the same in all lanes; the capture and
+  // selection kernels lose 2-4 % to the register allocation that follows from it)
+  const int warp = CAPTURE ? int(threadIdx.x >> 5) : __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0);
+  const int lane = threadIdx.x & 31;
   const int wg = warp >> 2;
   const int n_k = (a.k_len + CTA_K - 1) / CTA_K, n_q = (a.q_len + 127) / 128;
   // Launch order is query block fastest, then (head, half), then batch.  With a split tail the grid
@@ -640,23 +647,23 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
     for (int b = 0; b < kBuffers; ++b) {
       mbar_init(bar(Bars::SFULL + b), 1);
       mbar_init(bar(Bars::OFULL + b), 1);
-      mbar_init(bar(Bars::BUFFREE + b), 128);
+      mbar_init(bar(Bars::BUFFREE + b), 4);
     }
     for (int i = 0; i < 4; ++i) {
-      mbar_init(bar(Bars::STATFREE + i), 128);
-      mbar_init(bar(Bars::PFULL + i), 128);
-      mbar_init(bar(Bars::PFREE + i), 1);
+      mbar_init(bar(Bars::SLOTFREE + i), 4);
+      mbar_init(bar(Bars::PFULL + i), 4);
       mbar_init(bar(Bars::WFULL + i), 128);
     }
     if constexpr (MODE == kSelect)
       for (int i = 0; i < 2; ++i) mbar_init(bar(Bars::PAIRS + i), 1);
     mbar_init_fence();
   }
-  if (warp == 17) tmem_alloc(sbase + L::tmem_slot, 512);
+  if (warp == kIssueWarp + 1) tmem_alloc(sbase + L::tmem_slot, 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(smem + L::tmem_slot);
+  const uint32_t tmem =
+      __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(smem + L::tmem_slot), 0);
   // everything above needs no result of the kernels before this one; everything below does
   chain_wait();
 
@@ -666,7 +673,8 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
 
   if (wg == 4) {
     regs_dec<kRegsIssue>();
-    if (warp == 16 && lane == 0) {
+    const int n_iter = __shfl_sync(0xffffffffu, seq.n_iter, 0);
+    if (warp == kIssueWarp && lane == 0) {
       // ---------------------------------------------------------------- producer
       tma_prefetch_descriptor(&map_q);
       tma_prefetch_descriptor(&map_k);
@@ -712,54 +720,70 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
         for (int it = max(0, v_issued - L::kVSt); it < v_issued; ++it)
           mbar_drain(bar(Bars::VFULL + it % L::kVSt), (it / L::kVSt) & 1);
       }
-    } else if (warp == 17 && lane == 0) {
+    } else if (warp == kIssueWarp + 1) {
       // ---------------------------------------------------------------- MMA issue: S = Q.K^T
       // Tile it goes to buffer it % 4 as soon as the correction group has read that buffer's
-      // previous tile (it - 4) out.  Issuing the two GEMMs from two threads halves the per-tile
-      // barrier round-trips on each.
+      // previous tile (it - 4) out.  Issuing the two GEMMs from two warps halves the per-tile barrier round trips on
+      // each.  The whole warp walks the loop and one lane is elected for the MMAs: with control flow
+      // that is uniform over the warp the descriptors and barrier addresses stay in uniform
+      // registers, and this warp, which gets few issue slots beside the softmax warps of its
+      // scheduler, has a short instruction stream (with one thread per loop the P.V issue alone took
+      // 800 to 1300 cycles of a tile's 1700).
       constexpr uint32_t idesc_qk = idesc_i8(true, true, CTA_K);
+      RingPos<L::kKSt> ks;
+      RingPos<kBuffers> sb;
       bool ok = mbar_wait<true>(bar(Bars::QFULL), 0, gave_up, 201);
-      for (int it = 0; it < seq.n_iter && ok; ++it) {
-        const int b = it % kBuffers, u = it / kBuffers, s = it % L::kKSt, r = it / L::kKSt;
-        ok = mbar_wait2<true>(bar(Bars::KFULL + s), r & 1, bar(Bars::BUFFREE + b), (u & 1) ^ 1,
-                              gave_up, 202);
-        if (!ok) break;
+      for (int it = 0; it < n_iter; ++it) {
+        ok = ok && mbar_wait2<true>(bar(Bars::KFULL + ks.stage), ks.phase,
+                                    bar(Bars::BUFFREE + sb.stage), sb.phase ^ 1, gave_up, 202);
+        if (!__all_sync(0xffffffffu, ok)) break;
         tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
-        for (int panel = 0; panel < L::kPanels; ++panel) {
-          const uint64_t desc_q = smem_desc_kmajor<L::kPanelBytes>(sbase + L::q + panel * kTile);
-          const uint64_t desc_k = smem_desc_kmajor<L::kPanelBytes>(
-              sbase + L::k + s * L::kKStage + panel * L::kKPanel);
+          for (int panel = 0; panel < L::kPanels; ++panel) {
+            const uint64_t desc_q = smem_desc_kmajor<L::kPanelBytes>(sbase + L::q + panel * kTile);
+            const uint64_t desc_k = smem_desc_kmajor<L::kPanelBytes>(
+                sbase + L::k + ks.stage * L::kKStage + panel * L::kKPanel);
 #pragma unroll
-          for (int kk = 0; kk < L::kPanelBytes / 32; ++kk)
-            mma_i8(tmem + 128 * b, desc_q + 2 * kk, desc_k + 2 * kk, idesc_qk, (panel | kk) > 0);
+            for (int kk = 0; kk < L::kPanelBytes / 32; ++kk)
+              mma_i8(tmem + 128 * sb.stage, desc_q + 2 * kk, desc_k + 2 * kk, idesc_qk,
+                     (panel | kk) > 0);
+          }
+          mma_commit(bar(Bars::SFULL + sb.stage));
+          mma_commit(bar(Bars::KEMPTY + ks.stage));
         }
-        mma_commit(bar(Bars::SFULL + b));
-        mma_commit(bar(Bars::KEMPTY + s));
+        __syncwarp();
+        ks.next();
+        sb.next();
       }
-    } else if (warp == 18 && lane == 0) {
+    } else if (warp == kIssueWarp + 2) {
       // ---------------------------------------------------------------- MMA issue: P.V
       constexpr uint32_t idesc_pv = idesc_i8(false, true, L::kOut);
+      RingPos<L::kVSt> vs;
+      RingPos<L::kSlots> ps;
+      RingPos<kBuffers> ob;
       bool ok = true;
-      for (int it = 0; it < seq.n_iter && ok; ++it) {
-        const int s = it % L::kVSt, r = it / L::kVSt;
-        const int slot = it % L::kSlots, j = it / L::kSlots;
-        ok = mbar_wait2<true>(bar(Bars::PFULL + slot), j & 1, bar(Bars::VFULL + s), r & 1,
-                              gave_up, 204);
-        if (!ok) break;
-        const int b = it % kBuffers;
-        const uint32_t tmem_o = tmem + 128 * b;  // the tile's scores have all been read by now
+      for (int it = 0; it < n_iter; ++it) {
+        ok = mbar_wait2<true>(bar(Bars::VFULL + vs.stage), vs.phase, bar(Bars::PFULL + ps.stage),
+                              ps.phase, gave_up, 204);
+        if (!__all_sync(0xffffffffu, ok)) break;
         tc_fence_after();
-        const uint64_t desc_p = smem_desc_k128(sbase + L::p + slot * kTile);
-        const uint64_t desc_v = smem_desc_k128(sbase + L::v + s * kTile);
-        // a 64-key tile is the first or second half (64 bytes per row) of its 128-key V slab
-        const uint32_t v_k0 = CTA_K == 64 ? 4u * (seq.tile(it) & 1) : 0u;
+        if (elect_one()) {
+          const uint64_t desc_p = smem_desc_k128(sbase + L::p + ps.stage * kTile);
+          const uint64_t desc_v = smem_desc_k128(sbase + L::v + vs.stage * kTile);
+          // a 64-key tile is the first or second half (64 bytes per row) of its 128-key V slab
+          const uint32_t v_k0 = CTA_K == 64 ? 4u * (seq.tile(it) & 1) : 0u;
 #pragma unroll
-        for (int kk = 0; kk < CTA_K / 32; ++kk)
-          mma_i8(tmem_o, desc_p + 2 * kk, desc_v + v_k0 + 2 * kk, idesc_pv, kk > 0);
-        mma_commit(bar(Bars::OFULL + b));
-        mma_commit(bar(Bars::VEMPTY + s));
-        mma_commit(bar(Bars::PFREE + slot));
+          for (int kk = 0; kk < CTA_K / 32; ++kk)
+            mma_i8(tmem + 128 * ob.stage, desc_p + 2 * kk, desc_v + v_k0 + 2 * kk,
+                   idesc_pv, kk > 0);
+          mma_commit(bar(Bars::OFULL + ob.stage));
+          mma_commit(bar(Bars::VEMPTY + vs.stage));
+        }
+        __syncwarp();
+        vs.next();
+        ps.next();
+        ob.next();
       }
     }
   } else if (wg < kSoftmaxGroups) {
@@ -853,8 +877,8 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       if constexpr (BOOLROWS) {
         if (!last && row_ok) mask_row_load64(bool_row + tile * CTA_K, mask_bytes);
       }
-      ok = mbar_wait3(bar(Bars::PFREE + slot), ((it / L::kSlots) & 1) ^ 1, bar(Bars::STATFREE + slot),
-                      ((it / L::kSlots) & 1) ^ 1, bar(Bars::SFULL + sb), u & 1, gave_up, 301);
+      ok = mbar_wait2(bar(Bars::SLOTFREE + slot), ((it / L::kSlots) & 1) ^ 1, bar(Bars::SFULL + sb),
+                      u & 1, gave_up, 301);
       if (!ok) break;
       tc_fence_after();
       // causal: tiles that end at or before the CTA's first query are fully visible
@@ -864,19 +888,7 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       if (WHOLE || (kHasInt && int_scores && (!last || a.k_len % CTA_K == 0)))
         softmax_tile_int<CAPTURE, CTA_K, kScoresInt>(tmem_row, sc, p_row, row_in & 7, stat,
                                                      my_sums, pack_mul, last ? -50000 : INT_MIN);
-      else if (RAGGED) {
-        // last visited tile of a call without mask or causal rule: the keys that exist, as bits
-        if constexpr (RAGGED) {
-          uint32_t keep[CTA_K / 32];
-#pragma unroll
-          for (int c = 0; c < CTA_K / 32; ++c) {
-            const int exist = a.k_len - (tile * CTA_K + 32 * c);
-            keep[c] = exist >= 32 ? 0xffffffffu : exist <= 0 ? 0u : (1u << exist) - 1u;
-          }
-          softmax_tile_int<CAPTURE, CTA_K, kScoresInt, true>(tmem_row, sc, p_row, row_in & 7, stat,
-                                                             my_sums, pack_mul, -50000, keep);
-        }
-      } else if (kHasScaled && below_diagonal && !last)
+      else if (kHasScaled && below_diagonal && !last)
         softmax_tile_int<CAPTURE, CTA_K, kScoresScaled>(tmem_row, sc, p_row, row_in & 7, stat,
                                                         my_sums, pack_mul);
       else if (BOOLROWS && !last) {
@@ -902,7 +914,7 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       // are in shared memory: P.V may now overwrite the buffer
       tc_fence_before();
       fence_async_smem();
-      mbar_arrive(bar(Bars::PFULL + slot));
+      mbar_arrive_warp(bar(Bars::PFULL + slot));
       if constexpr (CAPTURE) {
         // With capture every tile needs the reference's exact running maximum and four denominator
         // partials per row (they decide block masses and tile sets bit for bit): a strictly
@@ -1039,13 +1051,13 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
         const float2 wf = stats[slot * 128 + row_in];
         w = wf.x;
         o_scale = wf.y;
-        mbar_arrive(bar(Bars::STATFREE + slot));
+        mbar_arrive_warp(bar(Bars::SLOTFREE + slot));
       } else {
         ok = mbar_wait(bar(Bars::OFULL + ob), (it / kBuffers) & 1, gave_up, 401);
         if (!ok) break;
         tc_fence_after();
         const float2 stat = stats[slot * 128 + row_in];
-        mbar_arrive(bar(Bars::STATFREE + slot));
+        mbar_arrive_warp(bar(Bars::SLOTFREE + slot));
         st.m = fmaxf(st.m, stat.x);
         if (st.m > m_o + 8.0f) {
           o_scale = ex2_approx(m_o - st.m);
@@ -1071,7 +1083,7 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
           tmem_load16(tmem_o + lane_base + 16 * (c + 1), acc);
         } else {
           tc_fence_before();
-          mbar_arrive(bar(Bars::BUFFREE + ob));  // Q.K^T of tile it + 4 may take the buffer
+          mbar_arrive_warp(bar(Bars::BUFFREE + ob));  // Q.K^T of tile it + 4 may take the buffer
         }
         if (rescale) {
 #pragma unroll
@@ -1320,7 +1332,7 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 17) {
+  if (warp == kIssueWarp + 1) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
   }
@@ -1604,9 +1616,6 @@ int attention_tc(const AttentionArgs& a, cudaStream_t stream, bool every_path) {
     }
     if (plain) {
       if (a.k_len % K == 0) return launch_tc<kDense, K, HD, 6>(a, map_q, map_k, map_v, stream);
-      // measured: the bit form of the ragged last tile gains at head_dim 128 (a 1000-key call
-      // 45 -> 34 us, long calls 0.5-1.5 %) and loses 1-4 % at head_dim 64 and 256
-      if constexpr (HD == 128) return launch_tc<kDense, K, HD, 7>(a, map_q, map_k, map_v, stream);
       return launch_tc<kDense, K, HD, 2>(a, map_q, map_k, map_v, stream);
     }
     if (a.mask != nullptr)

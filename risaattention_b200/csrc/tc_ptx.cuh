@@ -29,6 +29,11 @@ __device__ __forceinline__ void mbar_init_fence() {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// One arrival for a converged warp: every lane's earlier work comes before it.
+__device__ __forceinline__ void mbar_arrive_warp(uint32_t bar) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
+}
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                : "memory");
@@ -132,6 +137,31 @@ __device__ __forceinline__ bool mbar_wait3(uint32_t b0, uint32_t p0, uint32_t b1
          (r1 || mbar_wait<SPIN>(b1, p1, gave_up, site + 1)) &&
          (r2 || mbar_wait<SPIN>(b2, p2, gave_up, site + 2));
 }
+
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t elected;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xffffffff;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(elected));
+  return elected != 0;
+}
+// Position in a ring of N stages: the stage and the parity of its current round.
+template <int N>
+struct RingPos {
+  int stage = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ void next() {
+    if (++stage == N) {
+      stage = 0;
+      phase ^= 1;
+    }
+  }
+};
 
 // ---- proxies / fences --------------------------------------------------------------------------
 __device__ __forceinline__ void fence_async_smem() {
