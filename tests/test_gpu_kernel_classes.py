@@ -75,6 +75,31 @@ def test_class_kernels_give_the_bits_of_the_all_paths_kernel(head_dim, k_len, ki
         assert own[0][:, :, 3].count_nonzero() == 0 and torch.isneginf(own[1][:, :, 3]).all()
 
 
+@pytest.mark.parametrize("head_dim,k_len", [(64, 1024), (64, 130), (128, 1500), (128, 1025),
+                                            (128, 640), (256, 1279)])
+@pytest.mark.parametrize("kind", ["lengths", "strided", "per_head", "nothing", "everything"])
+def test_key_masks_read_as_bits_give_the_bits_of_the_all_paths_kernel(head_dim, k_len, kind):
+    """Boolean masks broadcast over the queries: tiles that are wholly visible, cut by a sequence end
+    (at, before and after a tile's edge), wholly hidden; keys that are not contiguous; masks of their
+    own per head.  Same codes and operations as the general path, so every bit is compared."""
+    q, k, v, g = _inputs(head_dim, 300, k_len, seed=head_dim + k_len)
+    ramp = torch.arange(k_len, device="cuda")
+    if kind == "lengths":
+        mask = (ramp < torch.tensor([k_len - 3, k_len // 128 * 64], device="cuda")[:, None])
+        mask = mask[:, None, None, :]
+    elif kind == "strided":
+        mask = (torch.rand(2, 1, 1, 2 * k_len, device="cuda", generator=g) > 0.3)[..., ::2]
+    elif kind == "per_head":
+        mask = (ramp >= 63 + torch.arange(4, device="cuda")[:, None])[None, :, None, :]
+    else:
+        mask = torch.full((1, 1, 1, k_len), kind == "everything", device="cuda")
+    own, every = _both(lambda: risa.int8_attention(q, k, v, attn_mask=mask, return_lse=True))
+    assert torch.equal(own[0], every[0])
+    assert torch.equal(own[1].view(torch.int32), every[1].view(torch.int32))
+    if kind == "nothing":
+        assert own[0].count_nonzero() == 0 and torch.isneginf(own[1]).all()
+
+
 @pytest.mark.parametrize("head_dim", [64, 128])
 def test_class_kernels_in_pattern_construction_and_reuse(head_dim):
     """Capture, in-pass selection and sparse reuse of calls without mask or causal rule run in the
