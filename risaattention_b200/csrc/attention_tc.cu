@@ -47,12 +47,12 @@ namespace {
 using namespace tc;
 
 constexpr int kKStages = 3;           // K ring depth (K runs two tiles ahead of V)
-constexpr int kVStages = 3;           // V ring depth
+constexpr int kVStages = 6;           // most V stages a ring has (SmemLayout::kVSt)
 constexpr int kTile = 128 * 128;      // bytes of one 128 x 128 INT8 tile
 constexpr int kThreads = 640;
 constexpr int kSoftmaxGroups = 3;     // softmax warpgroups; tile it is handled by group it % 3
 constexpr int kIssueWarp = 16;        // producer; +1 issues Q.K^T (and owns tensor memory), +2 P.V
-constexpr int kBuffers = 4;           // tensor-memory accumulator buffers; tile it uses it % 4
+constexpr int kMaxBuffers = 8;        // tensor-memory accumulator buffers (SmemLayout::kBuffers)
 // What a launch produces besides the output: nothing, the reference's capture workspace, or the
 // retained-mass selection of every query block.
 enum Mode : int { kDense = 0, kCapture = 1, kSelect = 2 };
@@ -85,10 +85,16 @@ struct SmemLayout {
   static constexpr int kPanels = D == 256 ? 2 : 1;         // column panels of a Q / K tile
   static constexpr int kPanelBytes = D == 64 ? 64 : 128;   // bytes per row of a panel
   static constexpr int kKSt = D == 256 ? 2 : kKStages;     // K ring depth
-  static constexpr int kVSt = D == 256 ? 2 : kVStages;     // V ring depth
-  static constexpr int kSlots = D == 256 ? 3 : 4;          // P tiles and per-row statistics
-  static constexpr int kQBytes = kPanels * kTile;          // the Q tile
-  static constexpr int kKPanel = CTA_K * 128;              // one column panel of a K stage
+  static constexpr int kVSt = D == 256 ? 2 : D == 64 ? 6 : CTA_K == 64 ? 4 : 3;  // V ring depth
+  // Tensor memory: accumulator buffers as wide as the wider of the scores and the output, so 64-key
+  // tiles at head_dim 64 have eight of 64 columns, everything else four of 128.
+  static constexpr int kBuffers = D == 64 ? 8 : 4;
+  static constexpr int kBufferCols = 512 / kBuffers;
+  static constexpr int kSlots = D == 256 ? 3 : kBuffers;   // P tiles and per-row statistics
+  static constexpr int kQBytes = kPanels * 128 * kPanelBytes;  // the Q tile
+  static constexpr int kKPanel = CTA_K * kPanelBytes;      // one column panel of a K stage
+  static constexpr int kVStage = kOut * 128;               // one V stage
+  static constexpr int kPTile = 128 * CTA_K;               // one P tile: rows of CTA_K bytes
   static constexpr int kKStage = kPanels * kKPanel;        // one K stage
   static constexpr int kMaskStageWords = 32 * 33;          // 32 x 32 values, rows padded to 33
   static constexpr int kMaskStageBytes =
@@ -96,14 +102,15 @@ struct SmemLayout {
   static constexpr int q = 0;
   static constexpr int k = q + kQBytes;
   static constexpr int v = k + kKSt * kKStage;
-  static constexpr int p = v + kVSt * kTile;
-  static constexpr int stats = p + kSlots * kTile;         // float2 [slots][128]: tile max, U8 sum
-  static constexpr int sums = stats + 4 * 128 * 8;         // uint16 [slots][128][CTA_K / 4] (capture)
-  static constexpr int mask_stage = sums + 4 * 128 * (CTA_K / 2);
+  static constexpr int p = v + kVSt * kVStage;
+  static constexpr int stats = p + kSlots * kPTile;        // float2 [slots][128]: tile max, U8 sum
+  static constexpr int sums = stats + kSlots * 128 * 8;    // uint16 [slots][128][CTA_K / 4] (capture)
+  static constexpr int sums_bytes = (kSlots < 4 ? 4 : kSlots) * 128 * (CTA_K / 2);
+  static constexpr int mask_stage = sums + sums_bytes;
   static constexpr int rowstate = mask_stage + kMaskStageBytes;  // float [5][128]: m, d[4] (capture)
   static constexpr int v_affine = rowstate + 5 * 128 * 4;  // float [2][128]: V scales, V centres
   static constexpr int bars = v_affine + 2 * 128 * 4;      // 8-byte mbarriers
-  static constexpr int n_bars = 1 + 2 * kKStages + 2 * kVStages + 6 * 4 + 3;  // one spare
+  static constexpr int n_bars = 1 + 2 * kKStages + 2 * kVStages + 6 * kMaxBuffers + 2;
   static constexpr int tmem_slot = bars + n_bars * 8;
   static constexpr int gave_up = tmem_slot + 8;            // site of the first expired wait, or 0
   static constexpr int total = tmem_slot + 16;
@@ -163,9 +170,10 @@ struct Bars {
   uint32_t base;
   static constexpr int QFULL = 0, KFULL = 1, KEMPTY = KFULL + kKStages, VFULL = KEMPTY + kKStages,
                        VEMPTY = VFULL + kVStages, SFULL = VEMPTY + kVStages,
-                       BUFFREE = SFULL + kBuffers, PFULL = BUFFREE + kBuffers, SLOTFREE = PFULL + 4,
-                       OFULL = SLOTFREE + 4, WFULL = OFULL + kBuffers,
-                       PAIRS = WFULL + 4;  // two: the selection epilogue's bulk copies
+                       BUFFREE = SFULL + kMaxBuffers, PFULL = BUFFREE + kMaxBuffers,
+                       SLOTFREE = PFULL + kMaxBuffers, OFULL = SLOTFREE + kMaxBuffers,
+                       WFULL = OFULL + kMaxBuffers,
+                       PAIRS = WFULL + kMaxBuffers;  // two: the selection epilogue's bulk copies
   // Tensor memory is four accumulator buffers of 128 columns; tile it owns buffer it % 4 for its
   // whole life: Q.K^T writes the scores there (SFULL), the softmax group reads them, P.V then
   // overwrites the same columns with the tile's integer output (OFULL) and the correction group
@@ -650,12 +658,12 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       mbar_init(bar(Bars::VFULL + s), 1);
       mbar_init(bar(Bars::VEMPTY + s), 1);
     }
-    for (int b = 0; b < kBuffers; ++b) {
+    for (int b = 0; b < L::kBuffers; ++b) {
       mbar_init(bar(Bars::SFULL + b), 1);
       mbar_init(bar(Bars::OFULL + b), 1);
       mbar_init(bar(Bars::BUFFREE + b), 4);
     }
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < L::kSlots; ++i) {
       mbar_init(bar(Bars::SLOTFREE + i), 4);
       mbar_init(bar(Bars::PFULL + i), 4);
       mbar_init(bar(Bars::WFULL + i), 128);
@@ -680,51 +688,64 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
   if (wg == 4) {
     regs_dec<kRegsIssue>();
     const int n_iter = __shfl_sync(0xffffffffu, seq.n_iter, 0);
-    if (warp == kIssueWarp && lane == 0) {
-      // ---------------------------------------------------------------- producer
-      tma_prefetch_descriptor(&map_q);
-      tma_prefetch_descriptor(&map_k);
-      tma_prefetch_descriptor(&map_v);
-      mbar_expect_tx(bar(Bars::QFULL), 128 * D);
+    // Two producers, one for Q and K and one for V: K is consumed as soon as an accumulator buffer is
+    // free, V only after the softmax, so one warp that waited for both would hold K back.  Like the
+    // MMA warps they walk their loops converged and elect a lane for the copies.
+    if (warp == kIssueWarp) {
+      // ---------------------------------------------------------------- producer: Q, K
+      if (elect_one()) {
+        tma_prefetch_descriptor(&map_q);
+        tma_prefetch_descriptor(&map_k);
+        mbar_expect_tx(bar(Bars::QFULL), 128 * D);
 #pragma unroll
-      for (int panel = 0; panel < L::kPanels; ++panel)
-        tma_load_3d(sbase + L::q + panel * kTile, &map_q, bar(Bars::QFULL), 128 * panel, bx * 128,
-                    int(bh));
-      bool ok = true;
-      int k_issued = 0, v_issued = 0;
-      // K runs two tiles ahead of V, matching the order in which the MMA warp consumes them.
-      for (int step = 0; step < seq.n_iter + 2 && ok; ++step) {
-        if (step < seq.n_iter) {
-          const int s = step % L::kKSt, r = step / L::kKSt;
-          ok = mbar_wait<true>(bar(Bars::KEMPTY + s), (r & 1) ^ 1, gave_up, 101);
-          if (!ok) break;
-          mbar_expect_tx(bar(Bars::KFULL + s), CTA_K * D);
+        for (int panel = 0; panel < L::kPanels; ++panel)
+          tma_load_3d(sbase + L::q + panel * kTile, &map_q, bar(Bars::QFULL), 128 * panel, bx * 128,
+                      int(bh));
+      }
+      RingPos<L::kKSt> ks;
+      int it = 0;
+      for (; it < n_iter; ++it) {
+        const bool ok = mbar_wait<true>(bar(Bars::KEMPTY + ks.stage), ks.phase ^ 1, gave_up, 101);
+        if (!__all_sync(0xffffffffu, ok)) break;
+        const int row0 = seq.tile(it) * CTA_K;
+        if (elect_one()) {
+          mbar_expect_tx(bar(Bars::KFULL + ks.stage), CTA_K * D);
 #pragma unroll
           for (int panel = 0; panel < L::kPanels; ++panel)
-            tma_load_3d(sbase + L::k + s * L::kKStage + panel * L::kKPanel, &map_k,
-                        bar(Bars::KFULL + s), 128 * panel, seq.tile(step) * CTA_K, int(kvh));
-          k_issued = step + 1;
+            tma_load_3d(sbase + L::k + ks.stage * L::kKStage + panel * L::kKPanel, &map_k,
+                        bar(Bars::KFULL + ks.stage), 128 * panel, row0, int(kvh));
         }
-        const int it = step - 2;
-        if (it >= 0) {
-          const int s = it % L::kVSt, r = it / L::kVSt;
-          ok = mbar_wait<true>(bar(Bars::VEMPTY + s), (r & 1) ^ 1, gave_up, 102);
-          if (!ok) break;
-          // V always arrives as the 128-key slab that holds the tile (64-key tiles use half of it):
-          // rows stay 128 bytes wide, so one swizzle mode and one descriptor form serve both widths
-          mbar_expect_tx(bar(Bars::VFULL + s), L::kOut * 128);
-          tma_load_3d(sbase + L::v + s * kTile, &map_v, bar(Bars::VFULL + s),
-                      (seq.tile(it) * CTA_K) & ~127, L::kOut * half, int(kvh));
-          v_issued = it + 1;
-        }
+        __syncwarp();
+        ks.next();
       }
-      if (!ok) {
+      if (it < n_iter) {
         // drain: every issued load must land before shared memory can be released
         mbar_drain(bar(Bars::QFULL), 0);
-        for (int it = max(0, k_issued - L::kKSt); it < k_issued; ++it)
-          mbar_drain(bar(Bars::KFULL + it % L::kKSt), (it / L::kKSt) & 1);
-        for (int it = max(0, v_issued - L::kVSt); it < v_issued; ++it)
-          mbar_drain(bar(Bars::VFULL + it % L::kVSt), (it / L::kVSt) & 1);
+        for (int j = max(0, it - L::kKSt); j < it; ++j)
+          mbar_drain(bar(Bars::KFULL + j % L::kKSt), (j / L::kKSt) & 1);
+      }
+    } else if (warp == kIssueWarp + 3) {
+      // ---------------------------------------------------------------- producer: V
+      if (elect_one()) tma_prefetch_descriptor(&map_v);
+      RingPos<L::kVSt> vs;
+      int it = 0;
+      for (; it < n_iter; ++it) {
+        const bool ok = mbar_wait<true>(bar(Bars::VEMPTY + vs.stage), vs.phase ^ 1, gave_up, 102);
+        if (!__all_sync(0xffffffffu, ok)) break;
+        // V always arrives as the 128-key slab that holds the tile (64-key tiles use half of it):
+        // rows stay 128 bytes wide, so one swizzle mode and one descriptor form serve both widths
+        const int key0 = (seq.tile(it) * CTA_K) & ~127;
+        if (elect_one()) {
+          mbar_expect_tx(bar(Bars::VFULL + vs.stage), L::kVStage);
+          tma_load_3d(sbase + L::v + vs.stage * L::kVStage, &map_v, bar(Bars::VFULL + vs.stage),
+                      key0, L::kOut * half, int(kvh));
+        }
+        __syncwarp();
+        vs.next();
+      }
+      if (it < n_iter) {
+        for (int j = max(0, it - L::kVSt); j < it; ++j)
+          mbar_drain(bar(Bars::VFULL + j % L::kVSt), (j / L::kVSt) & 1);
       }
     } else if (warp == kIssueWarp + 1) {
       // ---------------------------------------------------------------- MMA issue: S = Q.K^T
@@ -737,7 +758,7 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       // 800 to 1300 cycles of a tile's 1700).
       constexpr uint32_t idesc_qk = idesc_i8(true, true, CTA_K);
       RingPos<L::kKSt> ks;
-      RingPos<kBuffers> sb;
+      RingPos<L::kBuffers> sb;
       bool ok = mbar_wait<true>(bar(Bars::QFULL), 0, gave_up, 201);
       for (int it = 0; it < n_iter; ++it) {
         ok = ok && mbar_wait2<true>(bar(Bars::KFULL + ks.stage), ks.phase,
@@ -752,7 +773,7 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
                 sbase + L::k + ks.stage * L::kKStage + panel * L::kKPanel);
 #pragma unroll
             for (int kk = 0; kk < L::kPanelBytes / 32; ++kk)
-              mma_i8(tmem + 128 * sb.stage, desc_q + 2 * kk, desc_k + 2 * kk, idesc_qk,
+              mma_i8(tmem + L::kBufferCols * sb.stage, desc_q + 2 * kk, desc_k + 2 * kk, idesc_qk,
                      (panel | kk) > 0);
           }
           mma_commit(bar(Bars::SFULL + sb.stage));
@@ -767,7 +788,7 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       constexpr uint32_t idesc_pv = idesc_i8(false, true, L::kOut);
       RingPos<L::kVSt> vs;
       RingPos<L::kSlots> ps;
-      RingPos<kBuffers> ob;
+      RingPos<L::kBuffers> ob;
       bool ok = true;
       for (int it = 0; it < n_iter; ++it) {
         ok = mbar_wait2<true>(bar(Bars::VFULL + vs.stage), vs.phase, bar(Bars::PFULL + ps.stage),
@@ -775,13 +796,13 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
         if (!__all_sync(0xffffffffu, ok)) break;
         tc_fence_after();
         if (elect_one()) {
-          const uint64_t desc_p = smem_desc_k128(sbase + L::p + ps.stage * kTile);
-          const uint64_t desc_v = smem_desc_k128(sbase + L::v + vs.stage * kTile);
+          const uint64_t desc_p = smem_desc_kmajor<CTA_K>(sbase + L::p + ps.stage * L::kPTile);
+          const uint64_t desc_v = smem_desc_k128(sbase + L::v + vs.stage * L::kVStage);
           // a 64-key tile is the first or second half (64 bytes per row) of its 128-key V slab
           const uint32_t v_k0 = CTA_K == 64 ? 4u * (seq.tile(it) & 1) : 0u;
 #pragma unroll
           for (int kk = 0; kk < CTA_K / 32; ++kk)
-            mma_i8(tmem + 128 * ob.stage, desc_p + 2 * kk, desc_v + v_k0 + 2 * kk,
+            mma_i8(tmem + L::kBufferCols * ob.stage, desc_p + 2 * kk, desc_v + v_k0 + 2 * kk,
                    idesc_pv, kk > 0);
           mma_commit(bar(Bars::OFULL + ob.stage));
           mma_commit(bar(Bars::VEMPTY + vs.stage));
@@ -814,6 +835,8 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
     if constexpr (KEYBITS)
       key_row = static_cast<const unsigned char*>(a.mask) + int64_t(batch) * a.mask_stride_b +
                 int64_t(head) * a.mask_stride_h;
+    // 16-byte pieces of a P row are permuted by the row as the MMA's operand swizzle prescribes
+    const int swz = CTA_K == 64 ? (row_in >> 1) & 3 : row_in & 7;
     const PackMultipliers pack_mul{a.pack_by256, a.pack_by65536};
     const bool row_ok = row < a.q_len;
     const float scale2 = a.sm_scale * kLog2e;
@@ -865,8 +888,8 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       for (int g = 0; g < 4; ++g) ks_next[g] = __ldg(k_scale + first_tile * 4 + g);
     }
     for (int it = b; it < seq.n_iter && ok; it += kSoftmaxGroups) {
-      const int sb = it % kBuffers, u = it / kBuffers;
-      const uint32_t tmem_row = tmem_lane + 128 * sb;
+      const int sb = it % L::kBuffers, u = it / L::kBuffers;
+      const uint32_t tmem_row = tmem_lane + L::kBufferCols * sb;
       const int tile = seq.tile(it);
       const bool last = seq.last_rules(it, tile);
       float sc[4];
@@ -882,7 +905,7 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       const int slot = it % L::kSlots;
       float2* stat = stats + slot * 128 + row_in;
       uint16_t* my_sums = sums + (slot * 128 + row_in) * (CTA_K / 4);
-      unsigned char* p_row = smem + L::p + slot * kTile + row_in * 128;
+      unsigned char* p_row = smem + L::p + slot * L::kPTile + row_in * CTA_K;
       // KEYBITS: lane l looks at key l of every 32-key chunk, ahead of the wait for the scores
       uint32_t key_bytes[CTA_K / 32] = {};
       if constexpr (KEYBITS) {
@@ -905,7 +928,7 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       // A last tile without tail keys differs from the others only in where its maxima start;
       // with tail keys (their scores are zero-filled, not masked) it takes the general path.
       if (WHOLE || (kHasInt && int_scores && (!last || a.k_len % CTA_K == 0)))
-        softmax_tile_int<CAPTURE, CTA_K, kScoresInt>(tmem_row, sc, p_row, row_in & 7, stat,
+        softmax_tile_int<CAPTURE, CTA_K, kScoresInt>(tmem_row, sc, p_row, swz, stat,
                                                      my_sums, pack_mul, last ? -50000 : INT_MIN);
       else if (KEYBITS) {
         if constexpr (KEYBITS) {
@@ -919,14 +942,14 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
             all &= keep[c];
           }
           if (all == 0xffffffffu)
-            softmax_tile_int<CAPTURE, CTA_K, kScoresScaled>(tmem_row, sc, p_row, row_in & 7, stat,
+            softmax_tile_int<CAPTURE, CTA_K, kScoresScaled>(tmem_row, sc, p_row, swz, stat,
                                                             my_sums, pack_mul);
           else
             softmax_tile_int<CAPTURE, CTA_K, kScoresScaled, true, true>(
-                tmem_row, sc, p_row, row_in & 7, stat, my_sums, pack_mul, INT_MIN, keep);
+                tmem_row, sc, p_row, swz, stat, my_sums, pack_mul, INT_MIN, keep);
         }
       } else if (kHasScaled && below_diagonal && !last)
-        softmax_tile_int<CAPTURE, CTA_K, kScoresScaled>(tmem_row, sc, p_row, row_in & 7, stat,
+        softmax_tile_int<CAPTURE, CTA_K, kScoresScaled>(tmem_row, sc, p_row, swz, stat,
                                                         my_sums, pack_mul);
       else if (BOOLROWS && !last) {
         // boolean per-query mask, tile wholly inside the key range: the row's 64 entries as bits
@@ -936,16 +959,16 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
           uint32_t keep[2];
           mask_row_bits64(mask_bytes, keep);  // rows past the end hold zeros: nothing visible
           softmax_tile_int<CAPTURE, CTA_K, kScoresScaled, true>(
-              tmem_row, sc, p_row, row_in & 7, stat, my_sums, pack_mul, INT_MIN, keep);
+              tmem_row, sc, p_row, swz, stat, my_sums, pack_mul, INT_MIN, keep);
         }
       } else if (kHasMasked && (!kHasUnmasked || a.mask != nullptr))
         softmax_tile_general<CAPTURE, CTA_K, true, KEYMASK>(a, batch, head, row_ok, tmem_row, sc,
-                                                            p_row, row_in & 7, stat, my_sums,
+                                                            p_row, swz, stat, my_sums,
                                                             int_scores, last, row, tile * CTA_K,
                                                             mask_stage);
       else if constexpr (kHasUnmasked)
         softmax_tile_general<CAPTURE, CTA_K, false>(a, batch, head, row_ok, tmem_row, sc, p_row,
-                                                    row_in & 7, stat, my_sums, int_scores, last,
+                                                    swz, stat, my_sums, int_scores, last,
                                                     row, tile * CTA_K, mask_stage);
       // every score of the tile has been read (the loads were waited for) and the probabilities
       // are in shared memory: P.V may now overwrite the buffer
@@ -1074,39 +1097,26 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
     // d = d * f + sum * 2^(tile_m - m_o) and O = O * f + PV * 2^(tile_m - m_o) share weight and
     // (rare) rescale factor f, and their quotient needs no correction at the end.
     float m_o = -INFINITY;  // maximum the dense path's denominator and output rows are scaled to
-    for (int it = 0; it < seq.n_iter && ok; ++it) {
-      const int ob = it & (kBuffers - 1);
-      const int slot = it % L::kSlots;
-      const uint32_t tmem_o = tmem + 128 * ob;
-      float o_scale = 1.0f, w = 0.0f;
-      if constexpr (CAPTURE) {
-        // the statistics warp has replaced the tile's (maximum, sum) by its weights
-        ok = mbar_wait2(bar(Bars::OFULL + ob), (it / kBuffers) & 1, bar(Bars::WFULL + slot),
-                        (it / L::kSlots) & 1, gave_up, 401);
-        if (!ok) break;
-        tc_fence_after();
-        const float2 wf = stats[slot * 128 + row_in];
-        w = wf.x;
-        o_scale = wf.y;
-        mbar_arrive_warp(bar(Bars::SLOTFREE + slot));
-      } else {
-        ok = mbar_wait(bar(Bars::OFULL + ob), (it / kBuffers) & 1, gave_up, 401);
-        if (!ok) break;
-        tc_fence_after();
-        const float2 stat = stats[slot * 128 + row_in];
-        mbar_arrive_warp(bar(Bars::SLOTFREE + slot));
-        st.m = fmaxf(st.m, stat.x);
-        if (st.m > m_o + 8.0f) {
-          o_scale = ex2_approx(m_o - st.m);
-          m_o = st.m;
-        }
-        w = ex2_approx(stat.x - m_o);
-        st.d[0] = fmaf(static_cast<float>(__float_as_uint(stat.y)), w, st.d[0] * o_scale);
+    // Statistics of one tile without capture: the weight of its accumulator and the factor of what
+    // has been folded so far.
+    auto advance = [&](float2 stat, float& w, float& o_scale) {
+      o_scale = 1.0f;
+      st.m = fmaxf(st.m, stat.x);
+      if (st.m > m_o + 8.0f) {
+        o_scale = ex2_approx(m_o - st.m);
+        m_o = st.m;
       }
+      w = ex2_approx(stat.x - m_o);
+      st.d[0] = fmaf(static_cast<float>(__float_as_uint(stat.y)), w, st.d[0] * o_scale);
+    };
+    // O = O * o_scale + float(P.V) * w; the buffer goes back as soon as its last columns are here.
+    auto fold = [&](int it, float w, float o_scale) {
+      const int ob = it % L::kBuffers;
+      const uint32_t tmem_o = tmem + L::kBufferCols * ob + lane_base;
       const bool rescale = __any_sync(0xffffffffu, o_scale != 1.0f);
       const uint64_t w2 = pack_f32x2(w, w), s2 = pack_f32x2(o_scale, o_scale);
       uint32_t acc[16];
-      tmem_load16(tmem_o + lane_base, acc);
+      tmem_load16(tmem_o, acc);
 #pragma unroll
       for (int c = 0; c < kOut / 16; ++c) {
         tmem_load_wait();
@@ -1117,7 +1127,7 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
           f2[i] = pack_f32x2(static_cast<float>(int(acc[2 * i])),
                              static_cast<float>(int(acc[2 * i + 1])));
         if (c < kOut / 16 - 1) {
-          tmem_load16(tmem_o + lane_base + 16 * (c + 1), acc);
+          tmem_load16(tmem_o + 16 * (c + 1), acc);
         } else {
           tc_fence_before();
           mbar_arrive_warp(bar(Bars::BUFFREE + ob));  // Q.K^T of tile it + 4 may take the buffer
@@ -1128,6 +1138,47 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i) O2[8 * c + i] = fma_f32x2(f2[i], w2, O2[8 * c + i]);
+      }
+    };
+    // 64-key tiles are taken two at a time (P.V completes in order, so the second tile's accumulator
+    // stands for both): wait, hand-over and loop cost as much as the fold of such a tile.
+    constexpr int kStep = !CAPTURE && CTA_K == 64 ? 2 : 1;
+    for (int it = 0; it < seq.n_iter && ok; it += kStep) {
+      const int slot = it % L::kSlots;
+      if constexpr (CAPTURE) {
+        // the statistics warp has replaced the tile's (maximum, sum) by its weights
+        ok = mbar_wait2(bar(Bars::OFULL + it % L::kBuffers), (it / L::kBuffers) & 1,
+                        bar(Bars::WFULL + slot), (it / L::kSlots) & 1, gave_up, 401);
+        if (!ok) break;
+        tc_fence_after();
+        const float2 wf = stats[slot * 128 + row_in];
+        mbar_arrive_warp(bar(Bars::SLOTFREE + slot));
+        fold(it, wf.x, wf.y);
+      } else if constexpr (kStep == 1) {
+        ok = mbar_wait(bar(Bars::OFULL + it % L::kBuffers), (it / L::kBuffers) & 1, gave_up, 401);
+        if (!ok) break;
+        tc_fence_after();
+        const float2 stat = stats[slot * 128 + row_in];
+        mbar_arrive_warp(bar(Bars::SLOTFREE + slot));
+        float w, o_scale;
+        advance(stat, w, o_scale);
+        fold(it, w, o_scale);
+      } else {
+        const int last = min(it + 1, seq.n_iter - 1), last_slot = last % L::kSlots;
+        ok = mbar_wait(bar(Bars::OFULL + last % L::kBuffers), (last / L::kBuffers) & 1, gave_up, 401);
+        if (!ok) break;
+        tc_fence_after();
+        const float2 first_stat = stats[slot * 128 + row_in];
+        const float2 last_stat = stats[last_slot * 128 + row_in];
+        mbar_arrive_warp(bar(Bars::SLOTFREE + slot));
+        float w, o_scale, w_last = 0.0f, o_scale_last = 1.0f;
+        advance(first_stat, w, o_scale);
+        if (last > it) {
+          mbar_arrive_warp(bar(Bars::SLOTFREE + last_slot));
+          advance(last_stat, w_last, o_scale_last);
+        }
+        fold(it, w, o_scale);
+        if (last > it) fold(last, w_last, o_scale_last);
       }
     }
     float O[kOut];
@@ -1236,10 +1287,10 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
         // five dependent shuffles per tile.
         constexpr int kChunkTiles = 32;
         constexpr uint32_t kChunkBytes = kChunkTiles * 128 * 8;
-        static_assert(L::p - L::k >= 2 * int(kChunkBytes) && L::k % 16 == 0,
-                      "the K and V rings hold two chunks of pairs");
-        static_assert(L::kSlots * kTile >= 4 * 32 * 33 * 4, "the P ring holds the four sum blocks");
-        float* stage = reinterpret_cast<float*>(smem + L::p) + w * (32 * 33);
+        constexpr int kSumBlocks = L::p > L::k + 2 * int(kChunkBytes) ? L::p : L::k + 2 * int(kChunkBytes);
+        static_assert(L::k % 16 == 0 && kSumBlocks + 4 * 32 * 33 * 4 <= L::stats,
+                      "the K, V and P rings hold two chunks of pairs and the four sum blocks");
+        float* stage = reinterpret_cast<float*>(smem + kSumBlocks) + w * (32 * 33);
         const uint2* slot_pairs = pairs - row_in;
         const int n_chunks = (n_k + kChunkTiles - 1) / kChunkTiles;
         auto fetch = [&](int c) {
