@@ -4,6 +4,24 @@
 
 namespace risa_b200 {
 
+// Division of a non-negative int by a constant of the launch: n / d = (n * mul) >> shift for all
+// n < 2^31 (mul = floor(2^(31 + l) / d) + 1 with l = ceil(log2 d)).
+struct FastDivisor {
+  uint32_t mul, shift, divisor;
+#ifdef __CUDACC__
+  __device__ __forceinline__ int divide(int n, int& rest) const {
+    const int q = int((uint64_t(uint32_t(n)) * mul) >> shift);
+    rest = n - q * int(divisor);
+    return q;
+  }
+#endif
+};
+inline FastDivisor fast_divisor(uint32_t d) {
+  uint32_t l = 0;
+  while ((uint64_t(1) << l) < d) ++l;
+  return {uint32_t((uint64_t(1) << (31 + l)) / d + 1), 31 + l, d};
+}
+
 struct AttentionArgs {
   const int8_t* q;
   const int8_t* k;
@@ -47,6 +65,11 @@ struct AttentionArgs {
   // 2^8 and 2^16 as run-time values for the multiply-add packing of probability codes
   // (softmax_row.cuh, MAD_PACK)
   uint32_t pack_by256, pack_by65536;
+  // Resident CTAs of the tensor-core kernel: how many units there are to take, and what a unit number
+  // is taken apart with (units of a chunk of heads, heads of a chunk, heads x output halves; query
+  // heads per KV head).
+  int units;
+  FastDivisor by_chunk_units, by_chunk, by_heads, by_group;
 };
 
 // One part of AttentionArgs::tail_scratch: 128 rows x (128 channels, maximum, denominator).

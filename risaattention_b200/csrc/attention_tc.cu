@@ -78,20 +78,21 @@ constexpr unsigned int kSelfTestSite = 900;  // site number reported by the boun
 // for with shallower rings.  Kernels with 64-key tiles (per-query masks, short sequences,
 // head_dim 64) have smaller K stages and spend the difference on a per-warp staging area through
 // which mask values are loaded with coalesced accesses and handed to the row-owning threads.
-template <int D, int CTA_K>
+template <int D, int CTA_K, int MODE>
 struct SmemLayout {
   static constexpr int kOut = D == 256 ? 128 : D;          // output channels per CTA
   static constexpr int kHalves = D == 256 ? 2 : 1;         // CTAs per (query block, head)
   static constexpr int kPanels = D == 256 ? 2 : 1;         // column panels of a Q / K tile
   static constexpr int kPanelBytes = D == 64 ? 64 : 128;   // bytes per row of a panel
   static constexpr int kKSt = D == 256 ? 2 : kKStages;     // K ring depth
-  static constexpr int kVSt = D == 256 ? 2 : D == 64 ? 6 : CTA_K == 64 ? 4 : 3;  // V ring depth
+  static constexpr int kVSt = D == 256 ? 2 : D == 64 ? 6 : 3;  // V ring depth
   // Tensor memory: accumulator buffers as wide as the wider of the scores and the output, so 64-key
   // tiles at head_dim 64 have eight of 64 columns, everything else four of 128.
   static constexpr int kBuffers = D == 64 ? 8 : 4;
   static constexpr int kBufferCols = 512 / kBuffers;
   static constexpr int kSlots = D == 256 ? 3 : kBuffers;   // P tiles and per-row statistics
   static constexpr int kQBytes = kPanels * 128 * kPanelBytes;  // the Q tile
+  static constexpr int kQStages = MODE == kDense && D != 256 ? 2 : 1;  // Q tiles held at once
   static constexpr int kKPanel = CTA_K * kPanelBytes;      // one column panel of a K stage
   static constexpr int kVStage = kOut * 128;               // one V stage
   static constexpr int kPTile = 128 * CTA_K;               // one P tile: rows of CTA_K bytes
@@ -100,25 +101,35 @@ struct SmemLayout {
   static constexpr int kMaskStageBytes =
       CTA_K == 64 ? kSoftmaxGroups * 4 * kMaskStageWords * 4 : 0;  // one area per softmax warp
   static constexpr int q = 0;
-  static constexpr int k = q + kQBytes;
+  static constexpr int k = q + kQStages * kQBytes;
   static constexpr int v = k + kKSt * kKStage;
   static constexpr int p = v + kVSt * kVStage;
   static constexpr int stats = p + kSlots * kPTile;        // float2 [slots][128]: tile max, U8 sum
   static constexpr int sums = stats + kSlots * 128 * 8;    // uint16 [slots][128][CTA_K / 4] (capture)
-  static constexpr int sums_bytes = (kSlots < 4 ? 4 : kSlots) * 128 * (CTA_K / 2);
+  static constexpr int sums_bytes =
+      MODE == kDense ? 0 : (kSlots < 4 ? 4 : kSlots) * 128 * (CTA_K / 2);
   static constexpr int mask_stage = sums + sums_bytes;
   static constexpr int rowstate = mask_stage + kMaskStageBytes;  // float [5][128]: m, d[4] (capture)
   static constexpr int v_affine = rowstate + 5 * 128 * 4;  // float [2][128]: V scales, V centres
-  static constexpr int bars = v_affine + 2 * 128 * 4;      // 8-byte mbarriers
-  static constexpr int n_bars = 1 + 2 * kKStages + 2 * kVStages + 6 * kMaxBuffers + 2;
+  // Output rows on their way out: per warp 32 rows of 64 channels (128 bytes, rows 144 bytes apart).
+  // Capture and selection write their rows when the K / V rings are idle and stage them there.
+  static constexpr int kOutPitch = 9;                      // 16-byte pieces
+  static constexpr int out_stage = MODE == kDense ? v_affine + 2 * 128 * 4 : k;
+  static constexpr int bars = v_affine + 2 * 128 * 4 +
+                              (MODE == kDense ? 4 * 32 * kOutPitch * 16 : 0);  // 8-byte mbarriers
+  static constexpr int n_bars = 1 + 2 * kKStages + 2 * kVStages + 6 * kMaxBuffers + 2 + 3;
   static constexpr int tmem_slot = bars + n_bars * 8;
   static constexpr int gave_up = tmem_slot + 8;            // site of the first expired wait, or 0
   static constexpr int total = tmem_slot + 16;
   static constexpr size_t bytes = total + 1024;            // room to align the base to 1024
 };
-static_assert(SmemLayout<256, 128>::bytes <= 232448 && SmemLayout<128, 128>::bytes <= 232448 &&
-                  SmemLayout<256, 64>::bytes <= 232448 && SmemLayout<128, 64>::bytes <= 232448 &&
-                  SmemLayout<64, 64>::bytes <= 232448,
+template <int MODE>
+constexpr bool layouts_fit() {
+  return SmemLayout<256, 128, MODE>::bytes <= 232448 && SmemLayout<128, 128, MODE>::bytes <= 232448 &&
+         SmemLayout<256, 64, MODE>::bytes <= 232448 && SmemLayout<128, 64, MODE>::bytes <= 232448 &&
+         SmemLayout<64, 64, MODE>::bytes <= 232448;
+}
+static_assert(layouts_fit<kDense>() && layouts_fit<kCapture>() && layouts_fit<kSelect>(),
               "shared memory per CTA");
 
 struct TileSeq {
@@ -168,7 +179,7 @@ __device__ __forceinline__ TileSeq tile_sequence(const AttentionArgs& a, int64_t
 
 struct Bars {
   uint32_t base;
-  static constexpr int QFULL = 0, KFULL = 1, KEMPTY = KFULL + kKStages, VFULL = KEMPTY + kKStages,
+  static constexpr int QFULL = 0 /* two */, QEMPTY = 2 /* two */, KFULL = 4, KEMPTY = KFULL + kKStages, VFULL = KEMPTY + kKStages,
                        VEMPTY = VFULL + kVStages, SFULL = VEMPTY + kVStages,
                        BUFFREE = SFULL + kMaxBuffers, PFULL = BUFFREE + kMaxBuffers,
                        SLOTFREE = PFULL + kMaxBuffers, OFULL = SLOTFREE + kMaxBuffers,
@@ -591,11 +602,19 @@ __device__ __forceinline__ void softmax_tile_general(const AttentionArgs& a, int
 // as 16-byte pieces (chosen on the host, launch_tc): their tiles take the bit form of the fast path.
 // It is a kernel of its own so that the code of every other call stays exactly as it is -- the
 // register allocation of the tile loop reacts to any path that is compiled into it.
+// PERSIST (dense launches): the CTAs stay and take one (query block, head) unit after the other, and
+// every ring and barrier runs on across units.  A CTA of its own per unit costs about 6 us besides its
+// tiles (launch, barrier and tensor-memory set-up, first loads, a pipeline that fills and drains, the
+// epilogue); staying, the next unit's loads, products and softmax run under the previous unit's last
+// folds and output rows.  Attention alone, before -> after: causal 4096 at head_dim 64 (32 heads) 176
+// -> 137 us, 8192 keys at head_dim 128 426 -> 405, 2048 keys 40.4 -> 37.6, 480 heads of 333 x 333 94
+// -> 75.  Capture and selection use the idle rings after their last tile and keep a CTA per unit.
 template <int MODE, int CTA_K, int D, int VARIANT = 0>
 __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, const AttentionArgs a) {
   constexpr bool CAPTURE = MODE != kDense;  // exact per-tile statistics and denominators
+  constexpr bool PERSIST = !CAPTURE;
   // Which softmax paths an instantiation holds (the host picks the instantiation, launch_tc):
   // 0 every path; 1 boolean per-query masks read as bits; 2 no mask, not causal, positive scale;
   // 3 causal without mask, positive scale; 4 any other per-query mask; 5 masks broadcast over the
@@ -609,7 +628,7 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
   constexpr bool kHasInt = VARIANT == 0 || PLAIN, kHasScaled = VARIANT == 0 || CAUSAL,
                  kHasMasked = VARIANT == 0 || BOOLROWS || MASKED || KEYMASK,
                  kHasUnmasked = VARIANT == 0 || VARIANT == 2 || CAUSAL;
-  using L = SmemLayout<D, CTA_K>;
+  using L = SmemLayout<D, CTA_K, MODE>;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -620,36 +639,53 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
   const int lane = threadIdx.x & 31;
   const int wg = warp >> 2;
   const int n_k = (a.k_len + CTA_K - 1) / CTA_K, n_q = (a.q_len + 127) / 128;
-  // Launch order is query block fastest, then (head, half), then batch.  With a split tail the grid
-  // is one-dimensional: CTAs before tail_begin are whole (query block, head) units, the rest come
-  // in groups of tail_splits parts of one unit each.
+  // Units are ordered query block fastest, then (head, half), then batch.  With a split tail, units
+  // before tail_begin are whole (query block, head) pairs, the rest come in groups of tail_splits
+  // parts of one pair each.
   int bx = blockIdx.x, by = blockIdx.y, batch = blockIdx.z, part = 0, parts = 1, tail_unit = -1;
-  if (MODE == kDense && a.tail_splits > 1) {
-    int unit = blockIdx.x;
-    if (unit >= a.tail_begin) {
-      tail_unit = (unit - a.tail_begin) / a.tail_splits;
-      part = (unit - a.tail_begin) % a.tail_splits;
-      parts = a.tail_splits;
-      unit = a.tail_begin + tail_unit;
+  const bool longest_first = CAUSAL || (!PLAIN && a.is_causal);
+  int unit = blockIdx.x;  // unit in hand (PERSIST)
+  int head, half;
+  int64_t bh, kvh;
+  // Causal units visit bx + 1 query blocks' worth of key tiles: the longest ones come first, so that
+  // the short ones fill the end of the launch instead of the long ones stretching it.  Resident CTAs
+  // take every gridDim.x-th unit, every other round in reverse, which evens falling lengths out; their
+  // units come in chunks of a few heads, the same query block of all heads of a chunk together
+  // (chunk_heads(); one head to a chunk where all units are equally long).
+  auto place = [&] {
+    if constexpr (PERSIST) {
+      int pair = unit;
+      if (PLAIN || VARIANT == 0) {  // the calls whose last wave may be split
+        parts = 1;
+        if (unit >= a.tail_begin) {
+          tail_unit = (unit - a.tail_begin) / a.tail_splits;
+          part = (unit - a.tail_begin) % a.tail_splits;
+          parts = a.tail_splits;
+          pair = a.tail_begin + tail_unit;
+        }
+      }
+      int in_chunk, row;
+      const int chunk = a.by_chunk_units.divide(pair, in_chunk);
+      bx = a.by_chunk.divide(in_chunk, row);
+      batch = a.by_heads.divide(chunk * int(a.by_chunk.divisor) + row, by);
     }
-    const int rows_y = a.q_heads * L::kHalves;
-    bx = unit % n_q;
-    by = (unit / n_q) % rows_y;
-    batch = unit / (n_q * rows_y);
-  }
-  // Causal CTAs visit bx + 1 query blocks' worth of key tiles: the longest ones are launched first,
-  // so that the short ones fill the end of the launch instead of the long ones stretching it.
-  if (CAUSAL || (!PLAIN && a.is_causal)) bx = n_q - 1 - bx;
-  const int head = by / L::kHalves, half = by % L::kHalves;
-  const int kv_head = head / (a.q_heads / a.kv_heads);
-  const int64_t bh = int64_t(batch) * a.q_heads + head;
-  const int64_t kvh = int64_t(batch) * a.kv_heads + kv_head;
+    if (longest_first) bx = n_q - 1 - bx;
+    head = by / L::kHalves;
+    half = by % L::kHalves;
+    bh = int64_t(batch) * a.q_heads + head;
+    int in_group;
+    kvh = int64_t(batch) * a.kv_heads + a.by_group.divide(head, in_group);
+  };
+  place();
   const uint32_t gave_up = sbase + L::gave_up;  // set by the first wait of this CTA that expires
   Bars bar{sbase + L::bars};
 
   if (threadIdx.x == 0) {
     *reinterpret_cast<volatile uint32_t*>(smem + L::gave_up) = 0u;
-    mbar_init(bar(Bars::QFULL), 1);
+    for (int s = 0; s < L::kQStages; ++s) {
+      mbar_init(bar(Bars::QFULL + s), 1);
+      mbar_init(bar(Bars::QEMPTY + s), 1);
+    }
     for (int s = 0; s < kKStages; ++s) {
       mbar_init(bar(Bars::KFULL + s), 1);
       mbar_init(bar(Bars::KEMPTY + s), 1);
@@ -681,108 +717,156 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
   // everything above needs no result of the kernels before this one; everything below does
   chain_wait();
 
-  const TileSeq seq = tile_sequence<CTA_K>(a, bh, bx, n_q, n_k, CAPTURE, part, parts);
+  TileSeq seq = tile_sequence<CTA_K>(a, bh, bx, n_q, n_k, CAPTURE, part, parts);
+  // Steps to the CTA's next unit; every role walks the same units on its own.  `round` units and
+  // `base` tiles lie behind; tile it of the unit in hand is tile base + it of the CTA's rings.
+  int round = 0, base = 0;
+  auto next_unit = [&] {
+    if constexpr (!PERSIST) return false;
+    base += seq.n_iter;
+    ++round;
+    const int turn = (round & 1) != 0 ? int(gridDim.x) - 1 - int(blockIdx.x) : int(blockIdx.x);
+    unit = round * int(gridDim.x) + turn;
+    if (unit >= a.units) return false;
+    place();
+    seq = tile_sequence<CTA_K>(a, bh, bx, n_q, n_k, CAPTURE, part, parts);
+    return true;
+  };
   float2* stats = reinterpret_cast<float2*>(smem + L::stats);
   uint16_t* sums = reinterpret_cast<uint16_t*>(smem + L::sums);
 
   if (wg == 4) {
     regs_dec<kRegsIssue>();
-    const int n_iter = __shfl_sync(0xffffffffu, seq.n_iter, 0);
     // Two producers, one for Q and K and one for V: K is consumed as soon as an accumulator buffer is
     // free, V only after the softmax, so one warp that waited for both would hold K back.  Like the
     // MMA warps they walk their loops converged and elect a lane for the copies.
+    auto uniform = [](int v) { return __shfl_sync(0xffffffffu, v, 0); };
     if (warp == kIssueWarp) {
       // ---------------------------------------------------------------- producer: Q, K
       if (elect_one()) {
         tma_prefetch_descriptor(&map_q);
         tma_prefetch_descriptor(&map_k);
-        mbar_expect_tx(bar(Bars::QFULL), 128 * D);
-#pragma unroll
-        for (int panel = 0; panel < L::kPanels; ++panel)
-          tma_load_3d(sbase + L::q + panel * kTile, &map_q, bar(Bars::QFULL), 128 * panel, bx * 128,
-                      int(bh));
       }
       RingPos<L::kKSt> ks;
-      int it = 0;
-      for (; it < n_iter; ++it) {
-        const bool ok = mbar_wait<true>(bar(Bars::KEMPTY + ks.stage), ks.phase ^ 1, gave_up, 101);
+      RingPos<L::kQStages> qs;
+      int q_loads = 0, k_loads = 0;
+      bool ok = true;
+      do {
+        const int n_iter = uniform(seq.n_iter), row_q = uniform(bx * 128), slab_q = uniform(int(bh)),
+                  slab_k = uniform(int(kvh));
+        if (PERSIST && q_loads >= L::kQStages)
+          ok = mbar_wait<true>(bar(Bars::QEMPTY + qs.stage), qs.phase ^ 1, gave_up, 103);
         if (!__all_sync(0xffffffffu, ok)) break;
-        const int row0 = seq.tile(it) * CTA_K;
         if (elect_one()) {
-          mbar_expect_tx(bar(Bars::KFULL + ks.stage), CTA_K * D);
+          mbar_expect_tx(bar(Bars::QFULL + qs.stage), 128 * D);
 #pragma unroll
           for (int panel = 0; panel < L::kPanels; ++panel)
-            tma_load_3d(sbase + L::k + ks.stage * L::kKStage + panel * L::kKPanel, &map_k,
-                        bar(Bars::KFULL + ks.stage), 128 * panel, row0, int(kvh));
+            tma_load_3d(sbase + L::q + qs.stage * L::kQBytes + panel * kTile, &map_q,
+                        bar(Bars::QFULL + qs.stage), 128 * panel, row_q, slab_q);
         }
         __syncwarp();
-        ks.next();
-      }
-      if (it < n_iter) {
+        ++q_loads;
+        qs.next();
+        for (int it = 0; it < n_iter; ++it) {
+          ok = mbar_wait<true>(bar(Bars::KEMPTY + ks.stage), ks.phase ^ 1, gave_up, 101);
+          if (!__all_sync(0xffffffffu, ok)) break;
+          const int row0 = seq.tile(it) * CTA_K;
+          if (elect_one()) {
+            mbar_expect_tx(bar(Bars::KFULL + ks.stage), CTA_K * D);
+#pragma unroll
+            for (int panel = 0; panel < L::kPanels; ++panel)
+              tma_load_3d(sbase + L::k + ks.stage * L::kKStage + panel * L::kKPanel, &map_k,
+                          bar(Bars::KFULL + ks.stage), 128 * panel, row0, slab_k);
+          }
+          __syncwarp();
+          ++k_loads;
+          ks.next();
+        }
+        if (!__all_sync(0xffffffffu, ok)) break;
+      } while (next_unit());
+      if (!__all_sync(0xffffffffu, ok)) {
         // drain: every issued load must land before shared memory can be released
-        mbar_drain(bar(Bars::QFULL), 0);
-        for (int j = max(0, it - L::kKSt); j < it; ++j)
+        for (int j = max(0, q_loads - L::kQStages); j < q_loads; ++j)
+          mbar_drain(bar(Bars::QFULL + j % L::kQStages), (j / L::kQStages) & 1);
+        for (int j = max(0, k_loads - L::kKSt); j < k_loads; ++j)
           mbar_drain(bar(Bars::KFULL + j % L::kKSt), (j / L::kKSt) & 1);
       }
     } else if (warp == kIssueWarp + 3) {
       // ---------------------------------------------------------------- producer: V
       if (elect_one()) tma_prefetch_descriptor(&map_v);
       RingPos<L::kVSt> vs;
-      int it = 0;
-      for (; it < n_iter; ++it) {
-        const bool ok = mbar_wait<true>(bar(Bars::VEMPTY + vs.stage), vs.phase ^ 1, gave_up, 102);
-        if (!__all_sync(0xffffffffu, ok)) break;
-        // V always arrives as the 128-key slab that holds the tile (64-key tiles use half of it):
-        // rows stay 128 bytes wide, so one swizzle mode and one descriptor form serve both widths
-        const int key0 = (seq.tile(it) * CTA_K) & ~127;
-        if (elect_one()) {
-          mbar_expect_tx(bar(Bars::VFULL + vs.stage), L::kVStage);
-          tma_load_3d(sbase + L::v + vs.stage * L::kVStage, &map_v, bar(Bars::VFULL + vs.stage),
-                      key0, L::kOut * half, int(kvh));
+      int v_loads = 0;
+      bool ok = true;
+      do {
+        const int n_iter = uniform(seq.n_iter), row_v = uniform(L::kOut * half),
+                  slab_v = uniform(int(kvh));
+        for (int it = 0; it < n_iter; ++it) {
+          ok = mbar_wait<true>(bar(Bars::VEMPTY + vs.stage), vs.phase ^ 1, gave_up, 102);
+          if (!__all_sync(0xffffffffu, ok)) break;
+          // V always arrives as the 128-key slab that holds the tile (64-key tiles use half of it):
+          // rows stay 128 bytes wide, so one swizzle mode and one descriptor form serve both widths
+          const int key0 = (seq.tile(it) * CTA_K) & ~127;
+          if (elect_one()) {
+            mbar_expect_tx(bar(Bars::VFULL + vs.stage), L::kVStage);
+            tma_load_3d(sbase + L::v + vs.stage * L::kVStage, &map_v, bar(Bars::VFULL + vs.stage),
+                        key0, row_v, slab_v);
+          }
+          __syncwarp();
+          ++v_loads;
+          vs.next();
         }
-        __syncwarp();
-        vs.next();
-      }
-      if (it < n_iter) {
-        for (int j = max(0, it - L::kVSt); j < it; ++j)
+        if (!__all_sync(0xffffffffu, ok)) break;
+      } while (next_unit());
+      if (!__all_sync(0xffffffffu, ok)) {
+        for (int j = max(0, v_loads - L::kVSt); j < v_loads; ++j)
           mbar_drain(bar(Bars::VFULL + j % L::kVSt), (j / L::kVSt) & 1);
       }
     } else if (warp == kIssueWarp + 1) {
       // ---------------------------------------------------------------- MMA issue: S = Q.K^T
-      // Tile it goes to buffer it % 4 as soon as the correction group has read that buffer's
-      // previous tile (it - 4) out.  Issuing the two GEMMs from two warps halves the per-tile barrier round trips on
-      // each.  The whole warp walks the loop and one lane is elected for the MMAs: with control flow
-      // that is uniform over the warp the descriptors and barrier addresses stay in uniform
-      // registers, and this warp, which gets few issue slots beside the softmax warps of its
+      // A tile goes to its accumulator buffer as soon as the correction group has read that buffer's
+      // previous tile out.  Issuing the two GEMMs from two warps halves the per-tile barrier round
+      // trips on each.  The whole warp walks the loop and one lane is elected for the MMAs: with
+      // control flow that is uniform over the warp the descriptors and barrier addresses stay in
+      // uniform registers, and this warp, which gets few issue slots beside the softmax warps of its
       // scheduler, has a short instruction stream (with one thread per loop the P.V issue alone took
       // 800 to 1300 cycles of a tile's 1700).
       constexpr uint32_t idesc_qk = idesc_i8(true, true, CTA_K);
       RingPos<L::kKSt> ks;
       RingPos<L::kBuffers> sb;
-      bool ok = mbar_wait<true>(bar(Bars::QFULL), 0, gave_up, 201);
-      for (int it = 0; it < n_iter; ++it) {
-        ok = ok && mbar_wait2<true>(bar(Bars::KFULL + ks.stage), ks.phase,
-                                    bar(Bars::BUFFREE + sb.stage), sb.phase ^ 1, gave_up, 202);
-        if (!__all_sync(0xffffffffu, ok)) break;
-        tc_fence_after();
-        if (elect_one()) {
+      RingPos<L::kQStages> qs;
+      bool ok = true;
+      do {
+        const int n_iter = uniform(seq.n_iter);
+        ok = mbar_wait<true>(bar(Bars::QFULL + qs.stage), qs.phase, gave_up, 201);
+        const uint32_t q_tile = sbase + L::q + qs.stage * L::kQBytes;
+        for (int it = 0; it < n_iter; ++it) {
+          ok = ok && mbar_wait2<true>(bar(Bars::KFULL + ks.stage), ks.phase,
+                                      bar(Bars::BUFFREE + sb.stage), sb.phase ^ 1, gave_up, 202);
+          if (!__all_sync(0xffffffffu, ok)) break;
+          tc_fence_after();
+          if (elect_one()) {
 #pragma unroll
-          for (int panel = 0; panel < L::kPanels; ++panel) {
-            const uint64_t desc_q = smem_desc_kmajor<L::kPanelBytes>(sbase + L::q + panel * kTile);
-            const uint64_t desc_k = smem_desc_kmajor<L::kPanelBytes>(
-                sbase + L::k + ks.stage * L::kKStage + panel * L::kKPanel);
+            for (int panel = 0; panel < L::kPanels; ++panel) {
+              const uint64_t desc_q = smem_desc_kmajor<L::kPanelBytes>(q_tile + panel * kTile);
+              const uint64_t desc_k = smem_desc_kmajor<L::kPanelBytes>(
+                  sbase + L::k + ks.stage * L::kKStage + panel * L::kKPanel);
 #pragma unroll
-            for (int kk = 0; kk < L::kPanelBytes / 32; ++kk)
-              mma_i8(tmem + L::kBufferCols * sb.stage, desc_q + 2 * kk, desc_k + 2 * kk, idesc_qk,
-                     (panel | kk) > 0);
+              for (int kk = 0; kk < L::kPanelBytes / 32; ++kk)
+                mma_i8(tmem + L::kBufferCols * sb.stage, desc_q + 2 * kk, desc_k + 2 * kk, idesc_qk,
+                       (panel | kk) > 0);
+            }
+            mma_commit(bar(Bars::SFULL + sb.stage));
+            mma_commit(bar(Bars::KEMPTY + ks.stage));
           }
-          mma_commit(bar(Bars::SFULL + sb.stage));
-          mma_commit(bar(Bars::KEMPTY + ks.stage));
+          __syncwarp();
+          ks.next();
+          sb.next();
         }
+        if (!__all_sync(0xffffffffu, ok)) break;
+        if (PERSIST && elect_one()) mma_commit(bar(Bars::QEMPTY + qs.stage));
         __syncwarp();
-        ks.next();
-        sb.next();
-      }
+        qs.next();
+      } while (next_unit());
     } else if (warp == kIssueWarp + 2) {
       // ---------------------------------------------------------------- MMA issue: P.V
       constexpr uint32_t idesc_pv = idesc_i8(false, true, L::kOut);
@@ -790,28 +874,32 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       RingPos<L::kSlots> ps;
       RingPos<L::kBuffers> ob;
       bool ok = true;
-      for (int it = 0; it < n_iter; ++it) {
-        ok = mbar_wait2<true>(bar(Bars::VFULL + vs.stage), vs.phase, bar(Bars::PFULL + ps.stage),
-                              ps.phase, gave_up, 204);
-        if (!__all_sync(0xffffffffu, ok)) break;
-        tc_fence_after();
-        if (elect_one()) {
-          const uint64_t desc_p = smem_desc_kmajor<CTA_K>(sbase + L::p + ps.stage * L::kPTile);
-          const uint64_t desc_v = smem_desc_k128(sbase + L::v + vs.stage * L::kVStage);
-          // a 64-key tile is the first or second half (64 bytes per row) of its 128-key V slab
-          const uint32_t v_k0 = CTA_K == 64 ? 4u * (seq.tile(it) & 1) : 0u;
+      do {
+        const int n_iter = uniform(seq.n_iter);
+        for (int it = 0; it < n_iter; ++it) {
+          ok = mbar_wait2<true>(bar(Bars::VFULL + vs.stage), vs.phase, bar(Bars::PFULL + ps.stage),
+                                ps.phase, gave_up, 204);
+          if (!__all_sync(0xffffffffu, ok)) break;
+          tc_fence_after();
+          if (elect_one()) {
+            const uint64_t desc_p = smem_desc_kmajor<CTA_K>(sbase + L::p + ps.stage * L::kPTile);
+            const uint64_t desc_v = smem_desc_k128(sbase + L::v + vs.stage * L::kVStage);
+            // a 64-key tile is the first or second half (64 bytes per row) of its 128-key V slab
+            const uint32_t v_k0 = CTA_K == 64 ? 4u * (seq.tile(it) & 1) : 0u;
 #pragma unroll
-          for (int kk = 0; kk < CTA_K / 32; ++kk)
-            mma_i8(tmem + L::kBufferCols * ob.stage, desc_p + 2 * kk, desc_v + v_k0 + 2 * kk,
-                   idesc_pv, kk > 0);
-          mma_commit(bar(Bars::OFULL + ob.stage));
-          mma_commit(bar(Bars::VEMPTY + vs.stage));
+            for (int kk = 0; kk < CTA_K / 32; ++kk)
+              mma_i8(tmem + L::kBufferCols * ob.stage, desc_p + 2 * kk, desc_v + v_k0 + 2 * kk,
+                     idesc_pv, kk > 0);
+            mma_commit(bar(Bars::OFULL + ob.stage));
+            mma_commit(bar(Bars::VEMPTY + vs.stage));
+          }
+          __syncwarp();
+          vs.next();
+          ps.next();
+          ob.next();
         }
-        __syncwarp();
-        vs.next();
-        ps.next();
-        ob.next();
-      }
+        if (!__all_sync(0xffffffffu, ok)) break;
+      } while (next_unit());
     }
   } else if (wg < kSoftmaxGroups) {
     // ------------------------------------------------------------------ softmax of tiles it = wg, wg+3, ...
@@ -819,7 +907,9 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
     // grows would over-subscribe the pool (see the static_assert above)
     if constexpr (kRegsSoftmax > kRegsLaunch) regs_inc<kRegsSoftmax>();
     else if constexpr (kRegsSoftmax < kRegsLaunch) regs_dec<kRegsSoftmax>();
-    const int b = wg;                      // first tile of this group
+    int b = wg;                            // first tile of this group in the unit in hand
+    bool ok = true;
+    do {
     const int row_in = threadIdx.x & 127;  // tensor-memory lane
     const int row = bx * 128 + row_in;
     const uint32_t tmem_lane = tmem + (uint32_t((warp & 3) * 32) << 16);
@@ -847,7 +937,6 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
     uint32_t* mask_stage = nullptr;  // this warp's staging area for per-query mask blocks
     if constexpr (L::kMaskStageBytes > 0)
       mask_stage = reinterpret_cast<uint32_t*>(smem + L::mask_stage) + warp * L::kMaskStageWords;
-    bool ok = true;
     float* rowstate = reinterpret_cast<float*>(smem + L::rowstate);
     CaptureLayout cap;
     if constexpr (MODE == kCapture) cap = capture_layout(a, n_q, n_k);
@@ -887,8 +976,9 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
 #pragma unroll
       for (int g = 0; g < 4; ++g) ks_next[g] = __ldg(k_scale + first_tile * 4 + g);
     }
-    for (int it = b; it < seq.n_iter && ok; it += kSoftmaxGroups) {
-      const int sb = it % L::kBuffers, u = it / L::kBuffers;
+    int it = b;
+    for (; it < seq.n_iter && ok; it += kSoftmaxGroups) {
+      const int ring = base + it, sb = ring % L::kBuffers, u = ring / L::kBuffers;
       const uint32_t tmem_row = tmem_lane + L::kBufferCols * sb;
       const int tile = seq.tile(it);
       const bool last = seq.last_rules(it, tile);
@@ -902,7 +992,7 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       }
       // The P slot is free once the P.V that read it is done, the statistics slot once the
       // correction group has read the tile four back; S is ready when the MMA warp says so.
-      const int slot = it % L::kSlots;
+      const int slot = ring % L::kSlots;
       float2* stat = stats + slot * 128 + row_in;
       uint16_t* my_sums = sums + (slot * 128 + row_in) * (CTA_K / 4);
       unsigned char* p_row = smem + L::p + slot * L::kPTile + row_in * CTA_K;
@@ -919,8 +1009,8 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       if constexpr (BOOLROWS) {
         if (!last && row_ok) mask_row_load64(bool_row + tile * CTA_K, mask_bytes);
       }
-      ok = mbar_wait2(bar(Bars::SLOTFREE + slot), ((it / L::kSlots) & 1) ^ 1, bar(Bars::SFULL + sb),
-                      u & 1, gave_up, 301);
+      ok = mbar_wait2(bar(Bars::SLOTFREE + slot), ((ring / L::kSlots) & 1) ^ 1,
+                      bar(Bars::SFULL + sb), u & 1, gave_up, 301);
       if (!ok) break;
       tc_fence_after();
       // causal: tiles that end at or before the CTA's first query are fully visible
@@ -1062,10 +1152,14 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
         mbar_arrive(bar(Bars::WFULL + slot));
       }
     }
+    b = it - seq.n_iter;
+    } while (ok && next_unit());
   } else {
     // ------------------------------------------------------------------ correction + epilogue
     regs_inc<kRegsCorrection>();
     const int row_in = threadIdx.x & 127;
+    bool ok = true;  // false: a wait expired; this and all later units of the CTA are marked with NaN
+    do {
     const int row = bx * 128 + row_in;
     const bool row_ok = row < a.q_len;
     const uint32_t lane_base = uint32_t((warp & 3) * 32) << 16;
@@ -1076,11 +1170,11 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
     uint64_t O2[kOut / 2];
 #pragma unroll
     for (int i = 0; i < kOut / 2; ++i) O2[i] = 0ull;
-    bool ok = true;
     // The epilogue multiplies every output channel by its V scale and adds its V centre; the two
     // vectors are the same for all rows, so they are brought into shared memory now (their global
     // load latency passes during the first tiles instead of in front of every store).
     float* v_affine = reinterpret_cast<float*>(smem + L::v_affine);
+    if (PERSIST && round > 0) asm volatile("bar.sync 3, 128;" ::: "memory");  // previous unit's are read
     if (row_in < kOut) {
       v_affine[row_in] = __ldg(a.v_scale + kvh * D + kOut * half + row_in);
       v_affine[128 + row_in] = __ldg(a.v_center + kvh * D + kOut * half + row_in);
@@ -1103,15 +1197,16 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       o_scale = 1.0f;
       st.m = fmaxf(st.m, stat.x);
       if (st.m > m_o + 8.0f) {
-        o_scale = ex2_approx(m_o - st.m);
+        // (nothing has been folded before the first tile: no pass over 128 zeros)
+        if (m_o != -INFINITY) o_scale = ex2_approx(m_o - st.m);
         m_o = st.m;
       }
       w = ex2_approx(stat.x - m_o);
       st.d[0] = fmaf(static_cast<float>(__float_as_uint(stat.y)), w, st.d[0] * o_scale);
     };
     // O = O * o_scale + float(P.V) * w; the buffer goes back as soon as its last columns are here.
-    auto fold = [&](int it, float w, float o_scale) {
-      const int ob = it % L::kBuffers;
+    auto fold = [&](int ring, float w, float o_scale) {
+      const int ob = ring % L::kBuffers;
       const uint32_t tmem_o = tmem + L::kBufferCols * ob + lane_base;
       const bool rescale = __any_sync(0xffffffffu, o_scale != 1.0f);
       const uint64_t w2 = pack_f32x2(w, w), s2 = pack_f32x2(o_scale, o_scale);
@@ -1144,27 +1239,28 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
     // stands for both): wait, hand-over and loop cost as much as the fold of such a tile.
     constexpr int kStep = !CAPTURE && CTA_K == 64 ? 2 : 1;
     for (int it = 0; it < seq.n_iter && ok; it += kStep) {
-      const int slot = it % L::kSlots;
+      const int ring = base + it, slot = ring % L::kSlots;
       if constexpr (CAPTURE) {
         // the statistics warp has replaced the tile's (maximum, sum) by its weights
-        ok = mbar_wait2(bar(Bars::OFULL + it % L::kBuffers), (it / L::kBuffers) & 1,
-                        bar(Bars::WFULL + slot), (it / L::kSlots) & 1, gave_up, 401);
+        ok = mbar_wait2(bar(Bars::OFULL + ring % L::kBuffers), (ring / L::kBuffers) & 1,
+                        bar(Bars::WFULL + slot), (ring / L::kSlots) & 1, gave_up, 401);
         if (!ok) break;
         tc_fence_after();
         const float2 wf = stats[slot * 128 + row_in];
         mbar_arrive_warp(bar(Bars::SLOTFREE + slot));
-        fold(it, wf.x, wf.y);
+        fold(ring, wf.x, wf.y);
       } else if constexpr (kStep == 1) {
-        ok = mbar_wait(bar(Bars::OFULL + it % L::kBuffers), (it / L::kBuffers) & 1, gave_up, 401);
+        ok = mbar_wait(bar(Bars::OFULL + ring % L::kBuffers), (ring / L::kBuffers) & 1, gave_up, 401);
         if (!ok) break;
         tc_fence_after();
         const float2 stat = stats[slot * 128 + row_in];
         mbar_arrive_warp(bar(Bars::SLOTFREE + slot));
         float w, o_scale;
         advance(stat, w, o_scale);
-        fold(it, w, o_scale);
+        fold(ring, w, o_scale);
       } else {
-        const int last = min(it + 1, seq.n_iter - 1), last_slot = last % L::kSlots;
+        const bool two = it + 1 < seq.n_iter;
+        const int last = two ? ring + 1 : ring, last_slot = last % L::kSlots;
         ok = mbar_wait(bar(Bars::OFULL + last % L::kBuffers), (last / L::kBuffers) & 1, gave_up, 401);
         if (!ok) break;
         tc_fence_after();
@@ -1173,17 +1269,14 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
         mbar_arrive_warp(bar(Bars::SLOTFREE + slot));
         float w, o_scale, w_last = 0.0f, o_scale_last = 1.0f;
         advance(first_stat, w, o_scale);
-        if (last > it) {
+        if (two) {
           mbar_arrive_warp(bar(Bars::SLOTFREE + last_slot));
           advance(last_stat, w_last, o_scale_last);
         }
-        fold(it, w, o_scale);
-        if (last > it) fold(last, w_last, o_scale_last);
+        fold(ring, w, o_scale);
+        if (two) fold(last, w_last, o_scale_last);
       }
     }
-    float O[kOut];
-#pragma unroll
-    for (int i = 0; i < kOut / 2; ++i) unpack_f32x2(O2[i], O[2 * i], O[2 * i + 1]);
     int claimed = -1;
     uint2* pairs = nullptr;
     if constexpr (CAPTURE) {
@@ -1210,50 +1303,81 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       float* mine = a.tail_scratch + (size_t(tail_unit) * parts + part) * (130 * 128) + row_in;
       const float poison = ok ? 0.0f : __int_as_float(0x7fffffff);
 #pragma unroll
-      for (int ch = 0; ch < kOut; ++ch) mine[ch * 128] = O[ch] + poison;
+      for (int ch = 0; ch < kOut; ch += 2) {
+        float o0, o1;
+        unpack_f32x2(O2[ch / 2], o0, o1);
+        mine[ch * 128] = o0 + poison;
+        mine[(ch + 1) * 128] = o1 + poison;
+      }
       mine[128 * 128] = m_o;
       mine[129 * 128] = denom + poison;
-    } else if (ok && row_ok) {
-      if (MODE == kCapture && half == 0) {
+    } else if (__all_sync(0xffffffffu, ok)) {
+      if (MODE == kCapture && half == 0 && row_ok) {
         const CaptureLayout cap = capture_layout(a, n_q, n_k);
         cap.state[grow * 2] = st.m;
         cap.state[grow * 2 + 1] = denom;
       }
       // dense path: denominator and rows share the stale maximum's units, the quotient is exact
       const float inv = rcp_approx(denom);
+      const uint64_t inv2 = pack_f32x2(inv, inv);
       const bool zero = !PLAIN && (a.is_causal || a.mask != nullptr) && !(denom > 0.0f);
       const float* vs = v_affine;
       const float* vc = v_affine + 128;
-      char* o_row = static_cast<char*>(a.o) + 2 * kOut * half +
-                    2 * (batch * a.o_stride_b + head * a.o_stride_h + int64_t(row) * a.o_stride_n);
+      // A thread holds a row; stored from here a warp's 16-byte pieces would land in 32 rows each, so
+      // 64 channels at a time go through a staging block of the warp and leave as whole 128-byte runs
+      // (five thousand cycles of an epilogue became two thousand).
+      char* o_block = static_cast<char*>(a.o) + 2 * kOut * half +
+                      2 * (batch * a.o_stride_b + head * a.o_stride_h +
+                           int64_t(row - lane) * a.o_stride_n);
+      uint4* staged = reinterpret_cast<uint4*>(smem + L::out_stage) + (warp & 3) * 32 * L::kOutPitch;
 #pragma unroll
-      for (int ch = 0; ch < kOut; ch += 8) {
-        // eight channels' scales and centres as four 16-byte shared-memory loads (the same
-        // addresses in every thread: one broadcast each)
-        float scale8[8], centre8[8];
-        *reinterpret_cast<float4*>(scale8) = *reinterpret_cast<const float4*>(vs + ch);
-        *reinterpret_cast<float4*>(scale8 + 4) = *reinterpret_cast<const float4*>(vs + ch + 4);
-        *reinterpret_cast<float4*>(centre8) = *reinterpret_cast<const float4*>(vc + ch);
-        *reinterpret_cast<float4*>(centre8 + 4) = *reinterpret_cast<const float4*>(vc + ch + 4);
-        uint32_t packed[4];
+      for (int c0 = 0; c0 < kOut; c0 += 64) {
+        // the element type is the same for the whole launch: one branch per 64 channels
+        auto finish = [&](auto to_half) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          float r0 = fmaf(O[ch + 2 * i] * inv, scale8[2 * i], centre8[2 * i]);
-          float r1 = fmaf(O[ch + 2 * i + 1] * inv, scale8[2 * i + 1], centre8[2 * i + 1]);
-          if (zero) r0 = r1 = 0.0f;
-          if (a.out_dtype_code == 1) {
-            const __half2 h = __floats2half2_rn(r0, r1);
-            packed[i] = *reinterpret_cast<const uint32_t*>(&h);
-          } else {
-            const __nv_bfloat162 h = __floats2bfloat162_rn(r0, r1);
-            packed[i] = *reinterpret_cast<const uint32_t*>(&h);
+          for (int ch = c0; ch < c0 + 64; ch += 8) {
+            // eight channels' scales and centres as four 16-byte shared-memory loads (the same
+            // addresses in every thread: one broadcast each), the arithmetic in packed pairs
+            ulonglong2 scales[2], centres[2];
+            scales[0] = *reinterpret_cast<const ulonglong2*>(vs + ch);
+            scales[1] = *reinterpret_cast<const ulonglong2*>(vs + ch + 4);
+            centres[0] = *reinterpret_cast<const ulonglong2*>(vc + ch);
+            centres[1] = *reinterpret_cast<const ulonglong2*>(vc + ch + 4);
+            uint32_t packed[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const uint64_t scaled = mul_f32x2(O2[(ch >> 1) + i], inv2);
+              const uint64_t r = fma_f32x2(scaled, i & 1 ? scales[i >> 1].y : scales[i >> 1].x,
+                                           i & 1 ? centres[i >> 1].y : centres[i >> 1].x);
+              float r0, r1;
+              unpack_f32x2(r, r0, r1);
+              if constexpr (decltype(to_half)::value) {
+                const __half2 h = __floats2half2_rn(r0, r1);
+                packed[i] = *reinterpret_cast<const uint32_t*>(&h);
+              } else {
+                const __nv_bfloat162 h = __floats2bfloat162_rn(r0, r1);
+                packed[i] = *reinterpret_cast<const uint32_t*>(&h);
+              }
+              if (!PLAIN) packed[i] = zero ? 0u : packed[i];
+            }
+            staged[lane * L::kOutPitch + (ch - c0) / 8] =
+                make_uint4(packed[0], packed[1], packed[2], packed[3]);
           }
+        };
+        if (a.out_dtype_code == 1) finish(std::true_type{});
+        else finish(std::false_type{});
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int r = 4 * i + lane / 8;
+          const uint4 piece = staged[r * L::kOutPitch + lane % 8];
+          if (row - lane + r < a.q_len)
+            *reinterpret_cast<uint4*>(o_block + 2 * r * a.o_stride_n + 2 * c0 + 16 * (lane % 8)) = piece;
         }
-        *reinterpret_cast<uint4*>(o_row + 2 * ch) =
-            make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        __syncwarp();
       }
       // the LSE wants the denominator's own reference point: the stale maximum without capture
-      if (a.lse && half == 0) a.lse[grow] = row_lse(denom, CAPTURE ? st.m : m_o);
+      if (a.lse && half == 0 && row_ok) a.lse[grow] = row_lse(denom, CAPTURE ? st.m : m_o);
     } else if (row_ok) {
       // a wait of this CTA expired: mark the rows it owns, so that a failed launch cannot be taken
       // for a result (NaN in both 16-bit output formats, NaN LSE)
@@ -1273,6 +1397,7 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
         // warp, then the four warp sums as (w0 + w2) + (w1 + w3)), because the masses feed an
         // exact selection.  The rings are idle by now: the capture sums' area is reused.
         const int n4 = (n_k + 3) & ~3;
+        asm volatile("bar.sync 1, 128;" ::: "memory");  // the output rows have left the K / V rings
         float* s_mass = reinterpret_cast<float*>(smem + L::sums);  // [n4], padded with -inf
         float* s_sorted = s_mass + n4;                             // [n_k] descending
         float* s_warp = s_sorted + n_k;                            // [4][n_k], then the ranks
@@ -1416,6 +1541,7 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
         }
       }
     }
+    } while (next_unit());
   }
 
   tc_fence_before();
@@ -1601,6 +1727,29 @@ bool reads_mask_keys_as_bits(const AttentionArgs& a) {
          !a.is_causal && a.block_mass == nullptr && a.select_scratch == nullptr;
 }
 
+// How many heads (output halves and batch entries counted) a causal launch interleaves to go through
+// its units longest first: as many as keep their K and V codes in a third of L2 -- all of them, for
+// an even end, in short calls -- and a divisor of their number.  4 x 24 heads of 16128 keys in one
+// chunk read K and V from DRAM instead of L2: 8.15 ms against 7.65.
+int chunk_heads(const AttentionArgs& a, int halves) {
+  const int64_t rows = int64_t(a.q_heads) * halves * a.batch;
+  if (!a.is_causal) return 1;
+  const int64_t bytes = int64_t(2) * a.batch * a.kv_heads * a.k_len * a.head_dim;
+  int64_t chunk = rows * (int64_t(42) << 20) / std::max<int64_t>(bytes, 1);
+  chunk = std::max<int64_t>(1, std::min(chunk, rows));
+  while (rows % chunk != 0) --chunk;
+  return int(chunk);
+}
+
+int sms_of_device(int device) {
+  static thread_local int sms = 0, sms_device = -1;
+  if (sms_device != device) {
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    sms_device = device;
+  }
+  return sms;
+}
+
 template <int MODE, int CTA_K, int D, int VARIANT = 0>
 int launch_tc(const AttentionArgs& a, const CUtensorMap& map_q, const CUtensorMap& map_k,
               const CUtensorMap& map_v, cudaStream_t stream) {
@@ -1610,10 +1759,10 @@ int launch_tc(const AttentionArgs& a, const CUtensorMap& map_q, const CUtensorMa
   cudaGetDevice(&device);
   if (configured != device) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(SmemLayout<D, CTA_K>::bytes));
+                                         int(SmemLayout<D, CTA_K, MODE>::bytes));
     if (e != cudaSuccess)
       return fail(RISA_B200_CUDA, "attention: cannot reserve %zu bytes of shared memory: %s",
-                  SmemLayout<D, CTA_K>::bytes, cudaGetErrorString(e));
+                  SmemLayout<D, CTA_K, MODE>::bytes, cudaGetErrorString(e));
     // setmaxnreg hands out the registers the CTA is launched with; if the compiler ever gave this
     // kernel fewer than the roles ask for, the increase could never be granted (it blocks, beyond
     // the reach of the bounded waits), so such a build must not run
@@ -1628,32 +1777,30 @@ int launch_tc(const AttentionArgs& a, const CUtensorMap& map_q, const CUtensorMa
                   "need a pool of %d", attr.numRegs, kPool / kThreads);
     configured = device;
   }
-  const dim3 grid((a.q_len + 127) / 128, a.q_heads * SmemLayout<D, CTA_K>::kHalves, a.batch);
+  const dim3 grid((a.q_len + 127) / 128, a.q_heads * SmemLayout<D, CTA_K, MODE>::kHalves, a.batch);
   if constexpr (MODE == kDense) {
-    static thread_local int sms = 0, sms_device = -1;
-    if (sms_device != device) {
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-      sms_device = device;
-    }
-    const int ctas = int(grid.x * grid.y * grid.z), n_k = (a.k_len + CTA_K - 1) / CTA_K;
-    const int parts = tail_split_factor(a, ctas, n_k, sms);
+    // resident CTAs, one per SM, over all units; the rest of the last round may be split into parts
+    const int sms = sms_of_device(device), n_k = (a.k_len + CTA_K - 1) / CTA_K;
+    const int ctas = int(grid.x * grid.y * grid.z), parts = tail_split_factor(a, ctas, n_k, sms);
+    AttentionArgs all = a;
+    all.tail_begin = all.units = ctas;
+    all.tail_splits = 0;
+    const int rest = parts > 0 ? ctas % sms : 0;
     if (parts > 0) {
-      AttentionArgs split = a;
-      const int rest = ctas % sms;
-      split.tail_begin = ctas - rest;
-      split.tail_splits = parts;
-      launch_chained(kernel, dim3(split.tail_begin + rest * parts), dim3(kThreads),
-                     SmemLayout<D, CTA_K>::bytes, stream, map_q, map_k, map_v, split);
-      launch_chained(tail_merge_kernel, dim3(rest, SmemLayout<D, CTA_K>::kOut / kMergeChannels),
-                     dim3(128), 0, stream, split,
-                     SmemLayout<D, CTA_K>::kHalves, SmemLayout<D, CTA_K>::kOut);
-      return check_launch("attention (tensor-core kernel, split tail)");
+      all.tail_begin = ctas - rest;
+      all.tail_splits = parts;
+      all.units = all.tail_begin + rest * parts;
     }
+    launch_chained(kernel, dim3(std::min(all.units, sms)), dim3(kThreads),
+                   SmemLayout<D, CTA_K, MODE>::bytes, stream, map_q, map_k, map_v, all);
+    if (parts > 0)
+      launch_chained(tail_merge_kernel, dim3(rest, SmemLayout<D, CTA_K, MODE>::kOut / kMergeChannels),
+                     dim3(128), 0, stream, all, SmemLayout<D, CTA_K, MODE>::kHalves,
+                     SmemLayout<D, CTA_K, MODE>::kOut);
+  } else {
+    launch_chained(kernel, grid, dim3(kThreads), SmemLayout<D, CTA_K, MODE>::bytes, stream, map_q,
+                   map_k, map_v, a);
   }
-  AttentionArgs whole = a;
-  whole.tail_splits = 0;
-  launch_chained(kernel, grid, dim3(kThreads), SmemLayout<D, CTA_K>::bytes, stream, map_q, map_k, map_v,
-                 whole);
   return check_launch("attention (tensor-core kernel)");
 }
 
@@ -1674,7 +1821,8 @@ bool attention_tc_supported(const AttentionArgs& a) {
          a.o_stride_h % 8 == 0 && a.o_stride_n % 8 == 0;
 }
 
-int attention_tc(const AttentionArgs& a, cudaStream_t stream, bool every_path) {
+int attention_tc(const AttentionArgs& args, cudaStream_t stream, bool every_path) {
+  AttentionArgs a = args;
   const int n_k = (a.k_len + a.cta_k - 1) / a.cta_k;
   const uint32_t d = uint32_t(a.head_dim);
   CUtensorMap map_q, map_k, map_v;
@@ -1687,6 +1835,11 @@ int attention_tc(const AttentionArgs& a, cudaStream_t stream, bool every_path) {
                 v_rows))
     return fail(RISA_B200_CUDA, "attention: tensor map creation failed");
   const int mode = a.select_scratch ? kSelect : a.block_mass ? kCapture : kDense;
+  const int chunk = chunk_heads(a, d == 256 ? 2 : 1);
+  a.by_chunk_units = fast_divisor(uint32_t(chunk) * uint32_t((a.q_len + 127) / 128));
+  a.by_chunk = fast_divisor(uint32_t(chunk));
+  a.by_heads = fast_divisor(uint32_t(a.q_heads * (d == 256 ? 2 : 1)));
+  a.by_group = fast_divisor(uint32_t(a.q_heads / a.kv_heads));
   auto launch = [&](auto cta_k, auto head_dim) {
     constexpr int K = decltype(cta_k)::value, HD = decltype(head_dim)::value;
     // calls without mask or causal rule and with a positive scale: the instantiations that hold
