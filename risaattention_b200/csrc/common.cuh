@@ -33,6 +33,17 @@ inline int check_launch(const char* what) {
     if (!(cond)) return ::risa_b200::fail(RISA_B200_INVALID, __VA_ARGS__); \
   } while (0)
 
+// Quantisation of inputs whose head dim in_dim is narrower than the kernel's (prep_qk.cu).
+int quantize_qkv_narrow(
+    const void* q, void* q_codes, float* q_scale, const void* k, void* k_codes, float* k_scale,
+    const void* v, void* v_codes, float* v_scale, float* v_center, int batch, int q_heads,
+    int q_len, int kv_heads, int k_len, int head_dim, int in_dim, int cta_k, int padded_len,
+    int64_t q_stride_b, int64_t q_stride_h, int64_t q_stride_n, int64_t k_stride_b,
+    int64_t k_stride_h, int64_t k_stride_n, int64_t v_stride_b, int64_t v_stride_h,
+    int64_t v_stride_n, int dtype_code, int midpoint_affine, int32_t* anchors,
+    const int32_t* q_perm, const int32_t* kv_perm, void* workspace, size_t workspace_bytes,
+    void* stream_ptr);
+
 // ---- device helpers ----------------------------------------------------------------------
 #ifdef __CUDACC__
 template <typename T> struct Load4;

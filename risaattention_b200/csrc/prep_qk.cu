@@ -73,10 +73,13 @@ __device__ __forceinline__ void rotate16(float* v, int chunk) {
   for (int i = 0; i < 16; ++i) v[i] *= kNorm;
 }
 
+// Sixteen channels of a row, of which the input has `have` (a multiple of 4 or more than 16); the
+// channels it lacks are left as they are.
 template <typename T>
-__device__ __forceinline__ void load16(const T* p, float* v) {
+__device__ __forceinline__ void load16(const T* p, float* v, int have) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) Load4<T>::load(p + 4 * i, v + 4 * i);
+  for (int i = 0; i < 4; ++i)
+    if (have > 4 * i) Load4<T>::load(p + 4 * i, v + 4 * i);
 }
 
 __device__ __forceinline__ float absmax16(const float* v) {
@@ -106,6 +109,7 @@ struct QJob {
   int q_len, q_heads, batch, blocks, scales_per_head;
   int64_t stride_b, stride_h, stride_n;
   const int32_t* perm;
+  int in_dim;  // channels the input has; the head's channels from here on are zeros
 };
 
 template <typename T, int D, int ROT>
@@ -134,40 +138,52 @@ __device__ __forceinline__ void quantize_q_block(const QJob& job, int blk, int h
   const int j = (lane % GLANES) / LPR;      // row inside the group
   const int chunk = lane % LPR;             // 16-channel chunk inside the row
 
-  // Passes are independent (a scale group lives inside one pass); they are taken kBatch at a time so
-  // that a thread holds kBatch * 16 values instead of all of them: fewer registers, more resident
-  // CTAs whose load and arithmetic phases overlap one another.
-  constexpr int kBatch = 2;
+  // Passes are independent (a scale group lives inside one pass).  The rows of up to four of them are
+  // loaded at once, as they are in memory (eight registers per 16-bit row chunk), and rotated one
+  // after the other: all of a CTA's load latency passes at once, with no more than one converted row
+  // in registers and four CTAs per SM.
+  constexpr int kBatch = sizeof(T) == 2 && PASSES % 4 == 0 ? 4 : 2;
   static_assert(PASSES % kBatch == 0, "pass batching");
+  const int have = job.in_dim - chunk * 16;
 #pragma unroll 1
   for (int p0 = 0; p0 < PASSES; p0 += kBatch) {
-    float v[kBatch][16];
-    int rows[kBatch];
+    Raw4<T> raw[kBatch][4];
+    const int group0 = (warp * PASSES + p0) * GPP + slot;  // 0..GROUPS-1 == tile*8 + o
+    auto row_of = [&](int p) {
+      const int group = group0 + p * GPP;
+      return blk * 128 + (group >> 3) * TILE_ROWS + (group & 7) + 8 * j;
+    };
 #pragma unroll
     for (int p = 0; p < kBatch; ++p) {
-      const int group = (warp * PASSES + p0 + p) * GPP + slot;  // 0..GROUPS-1 == tile*8 + o
-      const int row = blk * 128 + (group >> 3) * TILE_ROWS + (group & 7) + 8 * j;
-      rows[p] = row;
-#pragma unroll
-      for (int i = 0; i < 16; ++i) v[p][i] = 0.f;
+      const int row = row_of(p);
       if (row < q_len) {
         const int64_t src = row_map ? __ldg(row_map + row) : row;
-        load16(in + src * stride_n + chunk * 16, v[p]);
+        const T* from = in + src * stride_n + chunk * 16;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (have > 4 * i) raw[p][i].load(from + 4 * i);
       }
     }
 #pragma unroll
     for (int p = 0; p < kBatch; ++p) {
-      rotate16<ROT>(v[p], D == 256 ? (chunk & 7) : chunk);
-      float mx = absmax16(v[p]);
+      const int row = row_of(p);
+      float v[16];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float x[4];
+        raw[p][i].get(x);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) v[4 * i + c] = row < q_len && have > 4 * i ? x[c] : 0.0f;
+      }
+      rotate16<ROT>(v, D == 256 ? (chunk & 7) : chunk);
+      float mx = absmax16(v);
 #pragma unroll
       for (int off = GLANES / 2; off > 0; off >>= 1)
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
       const float sc = mx / 127.f + 1e-7f;
       const float inv = 1.f / sc;
-      const int group = (warp * PASSES + p0 + p) * GPP + slot;
-      if ((lane % GLANES) == 0) sc_out[group] = sc;
-      if (rows[p] < q_len)
-        store16_codes(out + static_cast<int64_t>(rows[p]) * D + chunk * 16, v[p], inv);
+      if ((lane % GLANES) == 0) sc_out[group0 + p * GPP] = sc;
+      if (row < q_len) store16_codes(out + static_cast<int64_t>(row) * D + chunk * 16, v, inv);
     }
   }
 }
@@ -184,7 +200,15 @@ __global__ __launch_bounds__(256) void quantize_q_kernel(const QJob job) {
 // Warp (w, s) takes a contiguous share of group w's rows; groups spanning several warps combine
 // their maxima through shared memory.
 // ------------------------------------------------------------------------------------------
-constexpr int k_threads(int d, int cta_k) { return d * cta_k / 64 < 128 ? 128 : d * cta_k / 64; }
+// A thread group takes a key tile, or two of the four scale groups of a tile of 128 keys of 256
+// channels: 32 values per thread, so that 64 registers do and two CTAs of the launch that also packs V
+// fit an SM.  (With 64 values per thread and one CTA: 8 heads of 16384 keys of 256 channels 145 us, V
+// included; 4 heads of 32768 keys of 128 channels with byte stores for V 83 us, now 55.)
+constexpr int k_items_per_tile(int d, int cta_k) { return d * cta_k > 32 * 512 ? 2 : 1; }
+constexpr int k_threads(int d, int cta_k) {
+  const int n = d * cta_k / 32 / k_items_per_tile(d, cta_k);
+  return n < 128 ? 128 : n;
+}
 
 struct KJob {
   const void* k;
@@ -194,13 +218,14 @@ struct KJob {
   int k_len, kv_heads, batch, tiles;
   int64_t stride_b, stride_h, stride_n;
   const int32_t* perm;
+  int in_dim;  // channels the input has; the head's channels from here on are zeros
 };
 
-// One key tile by k_threads(D, CTA_K) consecutive threads.  `sub` is the index of that thread group
+// One item (key tile or half of its scale groups) by k_threads(D, CTA_K) consecutive threads.  `sub` is the index of that thread group
 // inside the CTA (0 when the CTA is exactly one group) and `tid` the thread's index inside the
 // group; groups of a CTA meet only at their own named barrier.
 template <typename T, int D, int CTA_K, int ROT>
-__device__ __forceinline__ void quantize_k_tile(const KJob& job, int tile, int h, int b, int sub,
+__device__ __forceinline__ void quantize_k_tile(const KJob& job, int item, int h, int b, int sub,
                                                 int tid) {
   const T* __restrict__ k = static_cast<const T*>(job.k);
   int8_t* __restrict__ codes = job.codes;
@@ -210,8 +235,9 @@ __device__ __forceinline__ void quantize_k_tile(const KJob& job, int tile, int h
   const int32_t* __restrict__ perm = job.perm;
   constexpr int LPR = D / 16;
   constexpr int RPP = 32 / LPR;                 // rows per warp pass
-  constexpr int THREADS = k_threads(D, CTA_K);  // at most 64 values per lane
-  constexpr int NW = THREADS / 128;             // warps per scale group (>= 1 except D64)
+  constexpr int THREADS = k_threads(D, CTA_K);
+  constexpr int ITEMS = k_items_per_tile(D, CTA_K), GROUPS = 4 / ITEMS;  // scale groups of an item
+  constexpr int NW = THREADS / (32 * GROUPS);   // warps per scale group
   constexpr int WPG = NW < 1 ? 1 : NW;
   constexpr int GROUP_ROWS = CTA_K / 4;
   constexpr int RW = GROUP_ROWS / WPG;          // rows per warp
@@ -219,7 +245,7 @@ __device__ __forceinline__ void quantize_k_tile(const KJob& job, int tile, int h
   static_assert(PASSES >= 1 && PASSES * RPP == RW, "tile geometry");
   __shared__ float warp_max[512 / THREADS][4][WPG];
   const int lane = tid & 31, warp = tid >> 5;
-  const int w = warp % 4, s = warp / 4;
+  const int w = item % ITEMS * GROUPS + warp % GROUPS, s = warp / GROUPS, tile = item / ITEMS;
   const T* in = k + b * stride_b + h * stride_h;
   const int64_t bh = static_cast<int64_t>(b) * kv_heads + h;
   int8_t* out = codes + bh * k_len * D;
@@ -232,7 +258,7 @@ __device__ __forceinline__ void quantize_k_tile(const KJob& job, int tile, int h
   const int anchor = __ldg(job.anchors + bh);
   if (anchor >= 0) {
     const int64_t src = row_map ? __ldg(row_map + anchor) : anchor;
-    load16(in + src * stride_n + chunk * 16, bias);
+    load16(in + src * stride_n + chunk * 16, bias, job.in_dim - chunk * 16);
   }
 
   float v[PASSES][16];
@@ -247,7 +273,7 @@ __device__ __forceinline__ void quantize_k_tile(const KJob& job, int tile, int h
     for (int c = 0; c < 16; ++c) v[p][c] = 0.f;
     if (row < k_len) {
       const int64_t src = row_map ? __ldg(row_map + row) : row;
-      load16(in + src * stride_n + chunk * 16, v[p]);
+      load16(in + src * stride_n + chunk * 16, v[p], job.in_dim - chunk * 16);
 #pragma unroll
       for (int c = 0; c < 16; ++c) v[p][c] -= bias[c];
     }
@@ -274,7 +300,7 @@ __device__ __forceinline__ void quantize_k_tile(const KJob& job, int tile, int h
       store16_codes(out + static_cast<int64_t>(rows[p]) * D + chunk * 16, v[p], inv);
 }
 
-// grid (key tiles, kv heads, batch), k_threads(D, CTA_K) threads.
+// grid (items of a head, kv heads, batch), k_threads(D, CTA_K) threads.
 template <typename T, int D, int CTA_K, int ROT>
 __global__ __launch_bounds__(k_threads(D, CTA_K)) void quantize_k_kernel(const KJob job) {
   chain_wait();
@@ -283,29 +309,30 @@ __global__ __launch_bounds__(k_threads(D, CTA_K)) void quantize_k_kernel(const K
 }
 
 // The two steps that need the results of the first launch -- K quantisation (anchors) and the V
-// code step (ranges) -- as one launch of 512-thread CTAs: CTAs [0, V CTAs) are CTAs of the tiled V
+// code step (ranges) -- as one launch of 512-thread CTAs: CTAs [0, V CTAs) are CTAs of the V
 // code step (they run longest), each of the rest holds 512 / k_threads key tiles, one per thread
 // group.
 template <typename T, int D, int CTA_K, int ROT, bool AFFINE>
-__global__ __launch_bounds__(kTiledThreads) void quantize_k_v_codes_kernel(const KJob k_job,
+__global__ __launch_bounds__(kVThreads, 2) void quantize_k_v_codes_kernel(const KJob k_job,
                                                                             const VCodesJob v_job) {
   chain_wait();
   chain_release();
-  const int v_columns = v_job.slots / kTiledSlots;
-  const int v_blocks = v_columns * (v_job.batch * v_job.kv_heads * v_job.head_dim / kTiledChannels);
+  const int v_blocks = v_job.parts * (v_job.batch * v_job.kv_heads * v_job.head_dim / kVChannels);
   int block = blockIdx.x;
   if (block < v_blocks) {
-    v_codes_tiled_block<T, AFFINE>(v_job, block % v_columns, block / v_columns);
+    v_codes_block<T, AFFINE>(v_job, block % v_job.parts, block / v_job.parts);
     return;
   }
   block -= v_blocks;
   constexpr int THREADS = k_threads(D, CTA_K);
-  constexpr int SUBS = kTiledThreads / THREADS;
+  constexpr int SUBS = kVThreads / THREADS;
   const int sub = threadIdx.x / THREADS, tid = threadIdx.x % THREADS;
-  const int item = block * SUBS + sub;  // (batch, head, tile), tile fastest
-  if (item >= k_job.tiles * k_job.kv_heads * k_job.batch) return;
-  const int tile = item % k_job.tiles, bh = item / k_job.tiles;
-  quantize_k_tile<T, D, CTA_K, ROT>(k_job, tile, bh % k_job.kv_heads, bh / k_job.kv_heads, sub, tid);
+  const int items = k_job.tiles * k_items_per_tile(D, CTA_K);
+  const int item = block * SUBS + sub;  // (batch, head, item of the head), the last fastest
+  if (item >= items * k_job.kv_heads * k_job.batch) return;
+  const int bh = item / items;
+  quantize_k_tile<T, D, CTA_K, ROT>(k_job, item % items, bh % k_job.kv_heads, bh / k_job.kv_heads,
+                                    sub, tid);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -320,6 +347,7 @@ struct AnchorJob {
   int k_len, head_dim, kv_heads, batch;
   int64_t stride_b, stride_h, stride_n;
   const int32_t* perm;
+  int in_dim;  // channels the input has; the head's channels from here on are zeros
 };
 
 // Threads 0..127 of the CTA do the work; a CTA may be larger (every thread takes the barriers).
@@ -341,7 +369,7 @@ __device__ __forceinline__ void detect_anchor_block(const AnchorJob& job, int h,
       const int sample = idx / head_dim, channel = idx - sample * head_dim;
       const int row = sample * (k_len - 1) / (S - 1);
       const int64_t src = row_map ? __ldg(row_map + row) : row;
-      smp[idx] = load_scalar(in + src * job.stride_n + channel);
+      smp[idx] = channel < job.in_dim ? load_scalar(in + src * job.stride_n + channel) : 0.0f;
     }
   }
   __syncthreads();
@@ -491,20 +519,19 @@ template <typename T, int D, int CTA_K, int ROT>
 void launch_k(KJob k_job, const VCodesJob* codes_job, cudaStream_t stream) {
   k_job.tiles = (k_job.k_len + CTA_K - 1) / CTA_K;
   if (codes_job) {
-    constexpr int SUBS = kTiledThreads / k_threads(D, CTA_K);
-    const int k_items = k_job.tiles * k_job.kv_heads * k_job.batch;
-    const int v_blocks = codes_job->slots / kTiledSlots *
-                         (codes_job->batch * codes_job->kv_heads * codes_job->head_dim /
-                          kTiledChannels);
+    constexpr int SUBS = kVThreads / k_threads(D, CTA_K);
+    const int k_items = k_job.tiles * k_items_per_tile(D, CTA_K) * k_job.kv_heads * k_job.batch;
+    const int v_blocks = codes_job->parts * (codes_job->batch * codes_job->kv_heads *
+                                             codes_job->head_dim / kVChannels);
     const dim3 grid(v_blocks + (k_items + SUBS - 1) / SUBS);
     if (codes_job->midpoint_affine)
-      launch_chained(quantize_k_v_codes_kernel<T, D, CTA_K, ROT, true>, grid, dim3(kTiledThreads), 0,
+      launch_chained(quantize_k_v_codes_kernel<T, D, CTA_K, ROT, true>, grid, dim3(kVThreads), 0,
                      stream, k_job, *codes_job);
     else
-      launch_chained(quantize_k_v_codes_kernel<T, D, CTA_K, ROT, false>, grid, dim3(kTiledThreads),
+      launch_chained(quantize_k_v_codes_kernel<T, D, CTA_K, ROT, false>, grid, dim3(kVThreads),
                      0, stream, k_job, *codes_job);
   } else {
-    launch_chained(quantize_k_kernel<T, D, CTA_K, ROT>, dim3(k_job.tiles, k_job.kv_heads, k_job.batch),
+    launch_chained(quantize_k_kernel<T, D, CTA_K, ROT>, dim3(k_job.tiles * k_items_per_tile(D, CTA_K), k_job.kv_heads, k_job.batch),
                    dim3(k_threads(D, CTA_K)), 0, stream, k_job);
   }
 }
@@ -534,7 +561,7 @@ int risa_b200::quantize_qk_with_v_steps(const void* q, void* q_codes, float* q_s
                                       int64_t k_stride_b, int64_t k_stride_h, int64_t k_stride_n,
                                       int dtype_code, int32_t* anchors, const int32_t* q_perm,
                                       const int32_t* k_perm, const VRangeJob* range_job,
-                                      const VCodesJob* codes_job, void* stream_ptr) {
+                                      const VCodesJob* codes_job, void* stream_ptr, int in_dim) {
   RISA_REQUIRE(head_dim == 64 || head_dim == 128 || head_dim == 256,
                "quantize_qk: padded head_dim must be 64, 128, or 256");
   RISA_REQUIRE((cta_k == 64 || cta_k == 128) && !(head_dim == 64 && cta_k != 64),
@@ -571,6 +598,7 @@ int risa_b200::quantize_qk_with_v_steps(const void* q, void* q_codes, float* q_s
   q_job.stride_h = q_stride_h;
   q_job.stride_n = q_stride_n;
   q_job.perm = q_perm;
+  q_job.in_dim = in_dim > 0 ? in_dim : head_dim;
   AnchorJob anchor_job;
   anchor_job.k = k;
   anchor_job.anchors = anchors;
@@ -582,6 +610,7 @@ int risa_b200::quantize_qk_with_v_steps(const void* q, void* q_codes, float* q_s
   anchor_job.stride_h = k_stride_h;
   anchor_job.stride_n = k_stride_n;
   anchor_job.perm = k_perm;
+  anchor_job.in_dim = q_job.in_dim;
   KJob k_job;
   k_job.k = k;
   k_job.codes = static_cast<int8_t*>(k_codes);
@@ -595,6 +624,7 @@ int risa_b200::quantize_qk_with_v_steps(const void* q, void* q_codes, float* q_s
   k_job.stride_h = k_stride_h;
   k_job.stride_n = k_stride_n;
   k_job.perm = k_perm;
+  k_job.in_dim = q_job.in_dim;
 #define RISA_QK(D, ROT) \
   launch_qk<T, D, ROT>(q_job, anchor_job, range_job, k_job, codes_job, cta_k, stream)
   const bool h4_only = k_len <= 256;
@@ -625,8 +655,42 @@ extern "C" int risa_b200_quantize_qk(const void* q, void* q_codes, float* q_scal
 }
 
 // Q, K and V of one call.  Same results as risa_b200_quantize_qk followed by risa_b200_quantize_v;
-// the V range step travels in the first launch (quantize_q_scan_kernel) and, for key lengths and
-// buffers the tiled code step accepts, the V code step in the second (quantize_k_v_codes_kernel).
+// the V range step travels in the first launch (quantize_q_scan_kernel) and, for buffers the register
+// form of the code step accepts, the V code step in the second (quantize_k_v_codes_kernel).
+// in_dim: the head dim of q, k and v where it is smaller than head_dim, a multiple of 4; the codes are
+// those of inputs padded with zeros to head_dim, without a padded copy.
+int risa_b200::quantize_qkv_narrow(
+    const void* q, void* q_codes, float* q_scale, const void* k, void* k_codes, float* k_scale,
+    const void* v, void* v_codes, float* v_scale, float* v_center, int batch, int q_heads,
+    int q_len, int kv_heads, int k_len, int head_dim, int in_dim, int cta_k, int padded_len,
+    int64_t q_stride_b, int64_t q_stride_h, int64_t q_stride_n, int64_t k_stride_b,
+    int64_t k_stride_h, int64_t k_stride_n, int64_t v_stride_b, int64_t v_stride_h,
+    int64_t v_stride_n, int dtype_code, int midpoint_affine, int32_t* anchors,
+    const int32_t* q_perm, const int32_t* kv_perm, void* workspace, size_t workspace_bytes,
+    void* stream_ptr) {
+  RISA_REQUIRE(in_dim > 0 && in_dim <= head_dim && in_dim % 4 == 0 &&
+                   (in_dim == head_dim || head_dim % kVChannels == 0),
+               "quantize_qkv: input head_dim must be a multiple of 4 up to the padded head_dim");
+  VRangeJob range_job;
+  VCodesJob codes_job;
+  int status = v_quantize_jobs(v, v_codes, v_scale, v_center, batch, kv_heads, k_len, head_dim,
+                               padded_len, v_stride_b, v_stride_h, v_stride_n, dtype_code,
+                               midpoint_affine, kv_perm, workspace, workspace_bytes, &range_job,
+                               &codes_job, in_dim);
+  if (status != RISA_B200_OK) return status;
+  const bool codes_fused = codes_job.v != nullptr;
+  RISA_REQUIRE(codes_fused || in_dim == head_dim, "quantize_qkv: V codes must be 16-byte aligned");
+  status = quantize_qk_with_v_steps(q, q_codes, q_scale, k, k_codes, k_scale, batch, q_heads, q_len,
+                                    kv_heads, k_len, head_dim, cta_k, q_stride_b, q_stride_h,
+                                    q_stride_n, k_stride_b, k_stride_h, k_stride_n, dtype_code,
+                                    anchors, q_perm, kv_perm, &range_job,
+                                    codes_fused ? &codes_job : nullptr, stream_ptr, in_dim);
+  if (status != RISA_B200_OK) return status;
+  return quantize_v_after_range(v, v_codes, v_scale, v_center, batch, kv_heads, k_len, head_dim,
+                                padded_len, v_stride_b, v_stride_h, v_stride_n, dtype_code,
+                                midpoint_affine, kv_perm, workspace, codes_fused, stream_ptr);
+}
+
 extern "C" int risa_b200_quantize_qkv(
     const void* q, void* q_codes, float* q_scale, const void* k, void* k_codes, float* k_scale,
     const void* v, void* v_codes, float* v_scale, float* v_center, int batch, int q_heads,
@@ -636,21 +700,10 @@ extern "C" int risa_b200_quantize_qkv(
     int64_t v_stride_n, int dtype_code, int midpoint_affine, int32_t* anchors,
     const int32_t* q_perm, const int32_t* kv_perm, void* workspace, size_t workspace_bytes,
     void* stream_ptr) {
-  VRangeJob range_job;
-  VCodesJob codes_job;
-  int status = v_quantize_jobs(v, v_codes, v_scale, v_center, batch, kv_heads, k_len, head_dim,
-                               padded_len, v_stride_b, v_stride_h, v_stride_n, dtype_code,
-                               midpoint_affine, kv_perm, workspace, workspace_bytes, &range_job,
-                               &codes_job);
-  if (status != RISA_B200_OK) return status;
-  const bool codes_fused = codes_job.v != nullptr;
-  status = quantize_qk_with_v_steps(q, q_codes, q_scale, k, k_codes, k_scale, batch, q_heads, q_len,
-                                    kv_heads, k_len, head_dim, cta_k, q_stride_b, q_stride_h,
-                                    q_stride_n, k_stride_b, k_stride_h, k_stride_n, dtype_code,
-                                    anchors, q_perm, kv_perm, &range_job,
-                                    codes_fused ? &codes_job : nullptr, stream_ptr);
-  if (status != RISA_B200_OK) return status;
-  return quantize_v_after_range(v, v_codes, v_scale, v_center, batch, kv_heads, k_len, head_dim,
-                                padded_len, v_stride_b, v_stride_h, v_stride_n, dtype_code,
-                                midpoint_affine, kv_perm, workspace, codes_fused, stream_ptr);
+  return quantize_qkv_narrow(q, q_codes, q_scale, k, k_codes, k_scale, v, v_codes, v_scale, v_center,
+                             batch, q_heads, q_len, kv_heads, k_len, head_dim, head_dim, cta_k,
+                             padded_len, q_stride_b, q_stride_h, q_stride_n, k_stride_b, k_stride_h,
+                             k_stride_n, v_stride_b, v_stride_h, v_stride_n, dtype_code,
+                             midpoint_affine, anchors, q_perm, kv_perm, workspace, workspace_bytes,
+                             stream_ptr);
 }

@@ -14,6 +14,7 @@
 //   3. finish:   (midpoint-affine only) combines the residual sums in the reference order.
 // Compiled with --use_fast_math like the reference so 1.f / x and x / float(L) lower identically.
 #include "prep_v_steps.cuh"
+#include <algorithm>
 #include <mutex>
 
 namespace risa_b200 {
@@ -85,7 +86,7 @@ __global__ __launch_bounds__(kSlotsPerCta) void v_quantize_kernel(
     for (int src = k_len - 1 - slot; src >= 0; src -= slots) {
       float t[8];
       const int64_t row = row_map ? __ldg(row_map + src) : src;
-      load8(in + row * stride_n, t);
+      load8(in + row * stride_n, t, 8);
       const int dst = storage_position(src);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -110,12 +111,12 @@ __global__ __launch_bounds__(kSlotsPerCta) void v_quantize_kernel(
   }
 }
 
-// grid (slots / 32, B*Hkv*D / 64), 512 threads.
+// grid (VCodesJob::parts, B*Hkv*D / 64), 512 threads.
 template <typename T, bool AFFINE>
-__global__ __launch_bounds__(kTiledThreads) void v_quantize_tiled_kernel(const VCodesJob job) {
+__global__ __launch_bounds__(kVThreads, 2) void v_codes_kernel(const VCodesJob job) {
   chain_wait();
   chain_release();
-  v_codes_tiled_block<T, AFFINE>(job, blockIdx.x, blockIdx.y);
+  v_codes_block<T, AFFINE>(job, blockIdx.x, blockIdx.y);
 }
 
 // grid (B*Hkv*D), `slots` threads: xor butterfly per warp, warps added in order by thread 0.
@@ -183,11 +184,10 @@ extern "C" size_t risa_b200_quantize_v_workspace_size(int batch, int kv_heads, i
 }
 
 namespace {
-// 16-byte code stores need whole storage groups and an aligned destination; a CTA of the tiled
-// kernel owns kTiledChannels channels of one head, so the head must split into whole groups.
-bool tiled_form(const void* v_codes, int k_len, int head_dim) {
-  return k_len % 16 == 0 && reinterpret_cast<uintptr_t>(v_codes) % 16 == 0 &&
-         head_dim % kTiledChannels == 0;
+// 16-byte code stores need an aligned destination (rows are whole storage groups), and a CTA of the
+// register form owns 64 channels of one head.
+bool packed_in_registers(const void* v_codes, int head_dim) {
+  return reinterpret_cast<uintptr_t>(v_codes) % 16 == 0 && head_dim % kVChannels == 0;
 }
 }  // namespace
 
@@ -196,7 +196,7 @@ int risa_b200::v_quantize_jobs(const void* v, void* v_codes, float* v_scale, flo
                                int64_t stride_b, int64_t stride_h, int64_t stride_n,
                                int dtype_code, int midpoint_affine, const int32_t* perm,
                                void* workspace, size_t workspace_bytes, VRangeJob* range,
-                               VCodesJob* codes) {
+                               VCodesJob* codes, int in_dim) {
   RISA_REQUIRE(v && v_codes && v_scale && v_center, "quantize_v: null tensor");
   RISA_REQUIRE(batch > 0 && kv_heads > 0 && k_len > 0, "quantize_v: sizes must be positive");
   RISA_REQUIRE(head_dim > 0 && head_dim % 8 == 0 && head_dim <= 256,
@@ -228,8 +228,9 @@ int risa_b200::v_quantize_jobs(const void* v, void* v_codes, float* v_scale, flo
   range->stride_h = stride_h;
   range->stride_n = stride_n;
   range->perm = perm;
+  range->in_dim = in_dim > 0 ? in_dim : head_dim;
   codes->v = nullptr;
-  if (tiled_form(v_codes, k_len, head_dim)) {
+  if (packed_in_registers(v_codes, head_dim)) {
     codes->v = v;
     codes->out = static_cast<int8_t*>(v_codes);
     codes->scale_out = v_scale;
@@ -248,6 +249,18 @@ int risa_b200::v_quantize_jobs(const void* v, void* v_codes, float* v_scale, flo
     codes->stride_n = stride_n;
     codes->perm = perm;
     codes->midpoint_affine = midpoint_affine;
+    codes->in_dim = range->in_dim;
+    if (midpoint_affine) {
+      codes->steps = 0;
+      codes->parts = p.slots / 128;  // a CTA keeps four windows of 32 residue classes
+    } else {
+      // CTAs repeat the range reduction of their channels, so long sequences give them several
+      // pieces each, as long as about two CTAs per SM remain
+      const int64_t blocks = int64_t(batch) * kv_heads * (head_dim / kVChannels);
+      const int pieces = (padded_len + kVPiece - 1) / kVPiece;
+      codes->steps = int(std::max<int64_t>(1, std::min<int64_t>(4, pieces * blocks / 296)));
+      codes->parts = (pieces + codes->steps - 1) / codes->steps;
+    }
   }
   return RISA_B200_OK;
 }
@@ -267,19 +280,17 @@ int risa_b200::quantize_v_after_range(const void* v, void* v_codes, float* v_sca
   RISA_DISPATCH_FLOAT(dtype_code, T, {
     if (codes_done) {
       // the code step has run next to the K quantiser
-    } else if (tiled_form(v_codes, k_len, head_dim)) {
+    } else if (packed_in_registers(v_codes, head_dim)) {
       VRangeJob range;
       VCodesJob codes;
       v_quantize_jobs(v, v_codes, v_scale, v_center, batch, kv_heads, k_len, head_dim, padded_len,
                       stride_b, stride_h, stride_n, dtype_code, midpoint_affine, perm, workspace,
                       p.range_bytes + p.residual_bytes, &range, &codes);
-      const dim3 tiled_grid(p.slots / kTiledSlots, channels / kTiledChannels);
+      const dim3 grid(codes.parts, channels / kVChannels);
       if (midpoint_affine)
-        launch_chained(v_quantize_tiled_kernel<T, true>, tiled_grid, dim3(kTiledThreads), 0, stream,
-                       codes);
+        launch_chained(v_codes_kernel<T, true>, grid, dim3(kVThreads), 0, stream, codes);
       else
-        launch_chained(v_quantize_tiled_kernel<T, false>, tiled_grid, dim3(kTiledThreads), 0,
-                       stream, codes);
+        launch_chained(v_codes_kernel<T, false>, grid, dim3(kVThreads), 0, stream, codes);
     } else {
       const dim3 grid(p.slots / kSlotsPerCta, channels / 8);
       if (midpoint_affine)

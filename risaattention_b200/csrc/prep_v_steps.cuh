@@ -4,6 +4,7 @@
 #pragma once
 #include "common.cuh"
 #include <cfloat>
+#include <type_traits>
 
 namespace risa_b200 {
 
@@ -17,12 +18,17 @@ struct VRangeJob {
   int k_len, head_dim, kv_heads, batch, chunks;
   int64_t stride_b, stride_h, stride_n;
   const int32_t* perm;
+  int in_dim;  // channels the input has; channels from here to head_dim are zeros (a multiple of 4)
 };
 
+// Eight channels of a row, of which the input has `have` (channels it lacks are zeros).
 template <typename T>
-__device__ __forceinline__ void load8(const T* p, float* v) {
-  Load4<T>::load(p, v);
-  Load4<T>::load(p + 4, v + 4);
+__device__ __forceinline__ void load8(const T* p, float* v, int have) {
+#pragma unroll
+  for (int i = 0; i < 8; i += 4) {
+    if (have > i) Load4<T>::load(p + i, v + i);
+    else v[i] = v[i + 1] = v[i + 2] = v[i + 3] = 0.0f;
+  }
 }
 
 // One CTA of 256 threads = one 512-token chunk of one (batch, kv head): thread = (token lane,
@@ -48,7 +54,7 @@ __device__ __forceinline__ void v_range_block(const VRangeJob& job, int chunk, i
   for (int n = begin + tl; n < end; n += tokens_per_step) {
     float t[8];
     const int64_t src = row_map ? __ldg(row_map + n) : n;
-    load8(in + src * job.stride_n, t);
+    load8(in + src * job.stride_n, t, job.in_dim - 8 * g);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       mn[i] = fminf(mn[i], t[i]);
@@ -79,16 +85,19 @@ __device__ __forceinline__ int storage_position(int token) {
          (((w >> 2) & 1) << 3);
 }
 
-// Same work as v_quantize_kernel for key lengths that are a multiple of 16, organised for the memory
-// system: a CTA owns 32 consecutive slots x 64 channels (thread = one slot, four channels), so a
-// half-warp reads one token's 64 channels as one contiguous segment, and the codes of a 32-token
-// window go through shared memory to leave as 16-byte stores (one aligned 16-token storage group
-// of one channel each) instead of single bytes.  Each (slot, channel) residual is still summed by
-// one thread over tokens Lk-1-slot, Lk-1-slot-slots, ... in that order.
-// CTA (bx, by) of a (slots / 32) x (B*Hkv*D / 64) grid, 512 threads.
-constexpr int kTiledSlots = 32, kTiledChannels = 64, kTiledThreads = 512;
+// The code step, for head dims of whole 64-channel blocks: a warp takes windows of 32 tokens x 16
+// channels, a lane the four tokens of one storage word (2w, 2w+1, 2w+8, 2w+9 of a 16-token group) x
+// four channels.  The four code words of a lane -- one per channel -- are exchanged between the four
+// lanes of a group with two shuffle steps, after which a lane holds the whole 16-byte storage group
+// of one channel; neighbouring groups of a channel leave in the same store.  No shared memory and no
+// barrier per window, and key lengths need not be multiples of anything: missing tokens give code 0.
+//   absmax: a CTA walks `steps` pieces of 512 tokens x 64 channels, four windows in flight per lane.
+//   midpoint-affine: the residuals have an order of their own (slot t of `slots` sums tokens Lk-1-t,
+//   Lk-1-t-slots, ...), so a lane keeps four residue classes of tokens modulo `slots` -- a class is
+//   one slot -- and walks them from the last token down.
+constexpr int kVChannels = 64, kVThreads = 512, kVPiece = 512;
 
-// What the code step of one risa_b200_quantize_v call reads and writes (tiled form).
+// What the code step of one risa_b200_quantize_v call reads and writes.
 struct VCodesJob {
   const void* v;
   int8_t* out;
@@ -100,57 +109,101 @@ struct VCodesJob {
   int64_t stride_b, stride_h, stride_n;
   const int32_t* perm;
   int midpoint_affine;
+  int in_dim;        // as in VRangeJob
+  int steps, parts;  // 512-token pieces per CTA; CTAs per 64-channel block
 };
 
+// Four channels of a row as they are in memory, converted when they are used.
+template <typename T> struct Raw4 {
+  uint2 raw;
+  __device__ __forceinline__ void load(const T* p) { raw = __ldg(reinterpret_cast<const uint2*>(p)); }
+  __device__ __forceinline__ void get(float (&x)[4]) const {
+    if constexpr (sizeof(T) == 2) {
+      const uint32_t w[2] = {raw.x, raw.y};
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        if constexpr (std::is_same<T, __half>::value) {
+          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+          x[2 * i] = f.x;
+          x[2 * i + 1] = f.y;
+        } else {
+          x[2 * i] = __uint_as_float(w[i] << 16);
+          x[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+        }
+      }
+    }
+  }
+};
+template <> struct Raw4<float> {
+  float4 raw;
+  __device__ __forceinline__ void load(const float* p) {
+    raw = __ldg(reinterpret_cast<const float4*>(p));
+  }
+  __device__ __forceinline__ void get(float (&x)[4]) const {
+    x[0] = raw.x;
+    x[1] = raw.y;
+    x[2] = raw.z;
+    x[3] = raw.w;
+  }
+};
+
+// words[c] of lane w (of four neighbouring lanes) <-> word w of channel c: a 4 x 4 transposition.
+__device__ __forceinline__ void transpose_words(uint32_t (&words)[4], int lane) {
+  const bool odd = lane & 1, upper = lane & 2;
+  const uint32_t a = __shfl_xor_sync(0xffffffffu, odd ? words[0] : words[1], 1);
+  const uint32_t b = __shfl_xor_sync(0xffffffffu, odd ? words[2] : words[3], 1);
+  if (odd) {
+    words[0] = a;
+    words[2] = b;
+  } else {
+    words[1] = a;
+    words[3] = b;
+  }
+  const uint32_t c = __shfl_xor_sync(0xffffffffu, upper ? words[0] : words[2], 2);
+  const uint32_t d = __shfl_xor_sync(0xffffffffu, upper ? words[1] : words[3], 2);
+  if (upper) {
+    words[0] = c;
+    words[1] = d;
+  } else {
+    words[2] = c;
+    words[3] = d;
+  }
+}
+
+// CTA `part` of 64-channel block `by`, 512 threads.
 template <typename T, bool AFFINE>
-__device__ __forceinline__ void v_codes_tiled_block(const VCodesJob& job, int bx, int by) {
-  const T* __restrict__ v = static_cast<const T*>(job.v);
-  int8_t* __restrict__ out = job.out;
-  float* __restrict__ scale_out = job.scale_out;
-  float* __restrict__ center_out = job.center_out;
-  const float2* __restrict__ ranges = job.ranges;
-  float* __restrict__ residuals = job.residuals;
-  const int k_len = job.k_len, padded_len = job.padded_len, kv_heads = job.kv_heads;
-  const int head_dim = job.head_dim, chunks = job.chunks, slots = job.slots;
-  const int64_t stride_b = job.stride_b, stride_h = job.stride_h, stride_n = job.stride_n;
-  const int32_t* __restrict__ perm = job.perm;
-  __shared__ float s_inv[kTiledChannels], s_center[kTiledChannels];
-  // 32 positions per channel; a row pitch of 36 bytes (9 words) spreads the 16 channel quads of a
-  // half-warp over 8 banks (any pitch that is a multiple of 16 bytes would put them on 2)
-  __shared__ __align__(4) unsigned char s_tile[2][kTiledChannels][36];
-  const int d_tiles = head_dim / kTiledChannels;
-  const int d_tile = by % d_tiles, bh = by / d_tiles;
-  const int h = bh % kv_heads, b = bh / kv_heads;
-  const int d0 = d_tile * kTiledChannels;
-  const int sl = threadIdx.x >> 4, quad = threadIdx.x & 15;
-  const int slot = bx * kTiledSlots + sl;
-  const T* in = v + b * stride_b + h * stride_h + d0 + 4 * quad;
-  const int32_t* row_map = perm ? perm + static_cast<int64_t>(bh) * k_len : nullptr;
+__device__ __forceinline__ void v_codes_block(const VCodesJob& job, int part, int by) {
+  const int k_len = job.k_len, padded_len = job.padded_len, head_dim = job.head_dim;
+  const int chunks = job.chunks, slots = job.slots;
+  __shared__ float s_inv[kVChannels], s_center[kVChannels];
+  const int d_tiles = head_dim / kVChannels;
+  const int bh = by / d_tiles, d0 = (by % d_tiles) * kVChannels;
+  const int h = bh % job.kv_heads, b = bh / job.kv_heads;
   const int64_t out_row = static_cast<int64_t>(bh) * head_dim + d0;
 
   // channel range = min / max over the per-chunk partials: spread over the whole CTA (eight chunk
   // subsets per channel) so that the loads overlap instead of forming one long dependent loop
-  __shared__ float s_lo[kTiledThreads / kTiledChannels][kTiledChannels];
-  __shared__ float s_hi[kTiledThreads / kTiledChannels][kTiledChannels];
+  __shared__ float s_lo[kVThreads / kVChannels][kVChannels];
+  __shared__ float s_hi[kVThreads / kVChannels][kVChannels];
   {
-    const int channel = threadIdx.x % kTiledChannels, part = threadIdx.x / kTiledChannels;
+    const int channel = threadIdx.x % kVChannels, subset = threadIdx.x / kVChannels;
     float lo = FLT_MAX, hi = -FLT_MAX;
-    const float2* r = ranges + static_cast<int64_t>(bh) * chunks * head_dim + d0 + channel;
-    for (int c = part; c < chunks; c += kTiledThreads / kTiledChannels) {
+    const float2* r = job.ranges + static_cast<int64_t>(bh) * chunks * head_dim + d0 + channel;
+    for (int c = subset; c < chunks; c += kVThreads / kVChannels) {
       const float2 x = __ldg(r + static_cast<int64_t>(c) * head_dim);
       lo = fminf(lo, x.x);
       hi = fmaxf(hi, x.y);
     }
-    s_lo[part][channel] = lo;
-    s_hi[part][channel] = hi;
+    s_lo[subset][channel] = lo;
+    s_hi[subset][channel] = hi;
   }
   __syncthreads();
-  if (threadIdx.x < kTiledChannels) {
+  if (threadIdx.x < kVChannels) {
     float lo = FLT_MAX, hi = -FLT_MAX;
 #pragma unroll
-    for (int part = 0; part < kTiledThreads / kTiledChannels; ++part) {
-      lo = fminf(lo, s_lo[part][threadIdx.x]);
-      hi = fmaxf(hi, s_hi[part][threadIdx.x]);
+    for (int subset = 0; subset < kVThreads / kVChannels; ++subset) {
+      lo = fminf(lo, s_lo[subset][threadIdx.x]);
+      hi = fmaxf(hi, s_hi[subset][threadIdx.x]);
     }
     float center, radius;
     if constexpr (AFFINE) {
@@ -163,91 +216,121 @@ __device__ __forceinline__ void v_codes_tiled_block(const VCodesJob& job, int bx
     const float sc = fmaxf(radius * (1.f / 127.f), 1e-12f);
     s_inv[threadIdx.x] = 1.f / sc;
     s_center[threadIdx.x] = center;
-    if (bx == 0) {
-      scale_out[out_row + threadIdx.x] = sc;
-      if constexpr (!AFFINE) center_out[out_row + threadIdx.x] = 0.0f;
+    if (part == 0) {
+      job.scale_out[out_row + threadIdx.x] = sc;
+      if constexpr (!AFFINE) job.center_out[out_row + threadIdx.x] = 0.0f;
     }
   }
   __syncthreads();
-  float inv[4], center[4], residual[4];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int word = lane & 3, group = (lane >> 2) & 1;          // of the window's two storage groups
+  const int ch0 = (warp & 3) * 16 + (lane >> 3) * 4;           // the lane's four channels
+  const int first_token = 16 * group + 2 * word;               // of the window: +0, +1, +8, +9
+  float inv[4], center[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    inv[i] = s_inv[4 * quad + i];
-    center[i] = s_center[4 * quad + i];
-    residual[i] = 0.f;
+  for (int c = 0; c < 4; ++c) {
+    inv[c] = s_inv[ch0 + c];
+    center[c] = s_center[ch0 + c];
   }
-  // Window of iteration `it`: tokens [hi - 31, hi], hi = k_len - 1 - 32 * bx - slots * it;
-  // with k_len a multiple of 16 the window is two aligned 16-token storage groups.
-  const int first_hi = k_len - 1 - bx * kTiledSlots;
-  int buffer = 0;
-  // The loads of kBatch consecutive windows are issued together (a token's row is only read once,
-  // so nothing but the number of loads in flight hides the memory latency), then the windows are
-  // converted and written one after the other.
-  constexpr int kBatch = 8;
-  for (int batch_hi = first_hi; batch_hi >= 0; batch_hi -= kBatch * slots) {
-    float t[kBatch][4];
+  const bool present = d0 + ch0 < job.in_dim;
+  const T* in = static_cast<const T*>(job.v) + b * job.stride_b + h * job.stride_h + d0 + ch0;
+  const int32_t* row_map = job.perm ? job.perm + static_cast<int64_t>(bh) * k_len : nullptr;
+  // after the exchange the lane stores channel ch0 + word of its group
+  int8_t* out = job.out + (out_row + ch0 + word) * padded_len + 16 * group;
+  auto load_tokens = [&](int base, Raw4<T> (&t)[4], bool (&have)[4]) {
 #pragma unroll
-    for (int u = 0; u < kBatch; ++u) {
-      const int src = batch_hi - u * slots - sl;
-      if (src >= 0) {
-        const int64_t row = row_map ? __ldg(row_map + src) : src;
-        Load4<T>::load(in + row * stride_n, t[u]);
+    for (int j = 0; j < 4; ++j) {
+      const int token = base + first_token + (j & 1) + 8 * (j >> 1);
+      have[j] = token < k_len && present;
+      if (have[j]) {
+        const int64_t row = row_map ? __ldg(row_map + token) : token;
+        t[j].load(in + row * job.stride_n);
       }
     }
+  };
+  if constexpr (!AFFINE) {
+    constexpr int U = sizeof(T) == 2 ? 4 : 2;  // windows in flight
+    const int end = min(padded_len, (part + 1) * job.steps * kVPiece);
+    for (int base0 = part * job.steps * kVPiece + (warp >> 2) * 32; base0 < end; base0 += U * 128) {
+      Raw4<T> t[U][4];
+      bool have[U][4];
 #pragma unroll
-    for (int u = 0; u < kBatch; ++u) {
-      const int hi = batch_hi - u * slots;
-      if (hi < 0) break;  // uniform over the CTA
-      const int lo = hi - (kTiledSlots - 1);
-      const int src = hi - sl;
-      if (src >= 0) {
-        const int position = storage_position(src) - lo;
+      for (int u = 0; u < U; ++u) load_tokens(base0 + 128 * u, t[u], have[u]);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float normalized = (t[u][i] - center[i]) * inv[i];
-          const uint32_t code = to_s8(normalized);
-          s_tile[buffer][4 * quad + i][position] = static_cast<unsigned char>(code);
-          if constexpr (AFFINE)
-            residual[i] += normalized - static_cast<float>(static_cast<int8_t>(code));
+      for (int u = 0; u < U; ++u) {
+        float x[4][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          t[u][j].get(x[j]);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) x[j][c] = have[u][j] ? x[j][c] * inv[c] : 0.0f;
         }
+        uint32_t words[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) words[c] = pack4_s8(x[0][c], x[1][c], x[2][c], x[3][c]);
+        transpose_words(words, lane);
+        if (base0 + 128 * u < end)
+          *reinterpret_cast<uint4*>(out + base0 + 128 * u) =
+              make_uint4(words[0], words[1], words[2], words[3]);
       }
-      __syncthreads();  // the other buffer was read before the previous barrier: safe to refill
-      if (threadIdx.x < 2 * kTiledChannels) {
-        const int channel = threadIdx.x >> 1, group = threadIdx.x & 1;
-        const int base = lo + 16 * group;
-        if (base >= 0) {
-          const uint32_t* w = reinterpret_cast<const uint32_t*>(&s_tile[buffer][channel][16 * group]);
-          *reinterpret_cast<uint4*>(out + (out_row + channel) * padded_len + base) =
-              make_uint4(w[0], w[1], w[2], w[3]);
-        }
-      }
-      buffer ^= 1;
     }
-  }
-  if constexpr (AFFINE) {
+  } else {
+    const int residue = (part * 4 + (warp >> 2)) * 32;  // first class of this warp's window
+    if (residue >= slots) return;
+    float residual[4][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      residuals[(out_row + 4 * quad + i) * slots + slot] = residual[i];
-  }
-  // zero tail [k_len, padded_len): whole 16-byte groups because k_len is a multiple of 16
-  for (int idx = bx * kTiledThreads + threadIdx.x;
-       idx < kTiledChannels * ((padded_len - k_len) / 16); idx += job.slots / kTiledSlots * kTiledThreads) {
-    const int channel = idx % kTiledChannels, group = idx / kTiledChannels;
-    *reinterpret_cast<uint4*>(out + (out_row + channel) * padded_len + k_len + 16 * group) =
-        make_uint4(0u, 0u, 0u, 0u);
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) residual[j][c] = 0.0f;
+    const int top = (padded_len - 1) / slots * slots + residue;
+#pragma unroll 2
+    for (int base = top; base >= 0; base -= slots) {
+      Raw4<T> t[4];
+      bool have[4];
+      load_tokens(base, t, have);
+      uint32_t code[4][4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float x[4];
+        t[j].get(x);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          // (a channel the input lacks has centre 0, so the centre stands for its zeros too)
+          const float value = have[j] ? x[c] : center[c];
+          const float normalized = (value - center[c]) * inv[c];
+          code[j][c] = to_s8(normalized);
+          residual[j][c] += normalized - static_cast<float>(static_cast<int8_t>(code[j][c]));
+        }
+      }
+      uint32_t words[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        words[c] = __byte_perm(__byte_perm(code[0][c], code[1][c], 0x0040),
+                               __byte_perm(code[2][c], code[3][c], 0x0040), 0x5410);
+      transpose_words(words, lane);
+      if (base < padded_len)
+        *reinterpret_cast<uint4*>(out + base) = make_uint4(words[0], words[1], words[2], words[3]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int token_class = residue + first_token + (j & 1) + 8 * (j >> 1);
+      const int slot = ((k_len - 1 - token_class) % slots + slots) % slots;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) job.residuals[(out_row + ch0 + c) * slots + slot] = residual[j][c];
+    }
   }
 }
 
 // Host side of the V quantiser split into its steps (prep_v.cu): v_quantize_jobs() checks the
-// arguments of a risa_b200_quantize_v call and describes its range step and -- when the tiled form
-// applies, else codes->v stays null -- its code step, launching nothing;
+// arguments of a risa_b200_quantize_v call and describes its range step and -- for head dims
+// of whole 64-channel blocks, else codes->v stays null -- its code step, launching nothing;
 // quantize_v_after_range() launches what follows the range step, without the code step if that has
 // been run by somebody else.
 int v_quantize_jobs(const void* v, void* v_codes, float* v_scale, float* v_center, int batch,
                     int kv_heads, int k_len, int head_dim, int padded_len, int64_t stride_b,
                     int64_t stride_h, int64_t stride_n, int dtype_code, int midpoint_affine,
                     const int32_t* perm, void* workspace, size_t workspace_bytes, VRangeJob* range,
-                    VCodesJob* codes);
+                    VCodesJob* codes, int in_dim = 0);
 int quantize_v_after_range(const void* v, void* v_codes, float* v_scale, float* v_center, int batch,
                            int kv_heads, int k_len, int head_dim, int padded_len, int64_t stride_b,
                            int64_t stride_h, int64_t stride_n, int dtype_code, int midpoint_affine,
@@ -262,6 +345,6 @@ int quantize_qk_with_v_steps(const void* q, void* q_codes, float* q_scale, const
                              int64_t k_stride_h, int64_t k_stride_n, int dtype_code,
                              int32_t* anchors, const int32_t* q_perm, const int32_t* k_perm,
                              const VRangeJob* range_job, const VCodesJob* codes_job,
-                             void* stream_ptr);
+                             void* stream_ptr, int in_dim = 0);
 
 }  // namespace risa_b200
