@@ -119,30 +119,42 @@ __global__ __launch_bounds__(kVThreads, 2) void v_codes_kernel(const VCodesJob j
   v_codes_block<T, AFFINE>(job, blockIdx.x, blockIdx.y);
 }
 
-// grid (B*Hkv*D), `slots` threads: xor butterfly per warp, warps added in order by thread 0.
-__global__ void v_center_kernel(const float* __restrict__ residuals,
-                                const float2* __restrict__ ranges, float* __restrict__ center_out,
-                                int k_len, int head_dim, int chunks, int slots) {
+// One warp per channel: an xor butterfly per group of 32 slots, groups added in order, as the
+// reference adds them.  Sixteen groups and the chunk ranges are loaded at once, so the kernel is one
+// round trip and a few shuffles (with a CTA per channel and one thread for the rest it was 8 us).
+constexpr int kCenterThreads = 256;
+__global__ __launch_bounds__(kCenterThreads) void v_center_kernel(
+    const float* __restrict__ residuals, const float2* __restrict__ ranges,
+    float* __restrict__ center_out, int channels, int k_len, int head_dim, int chunks, int slots) {
   chain_wait();
   chain_release();
-  __shared__ float warp_sum[16];
-  const int channel = blockIdx.x;
-  float r = residuals[static_cast<int64_t>(channel) * slots + threadIdx.x];
+  const int lane = threadIdx.x & 31;
+  const int channel = blockIdx.x * (kCenterThreads / 32) + (threadIdx.x >> 5);
+  if (channel >= channels) return;
+  const float* sums = residuals + static_cast<int64_t>(channel) * slots + lane;
+  float r[16];
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) r += __shfl_xor_sync(0xffffffffu, r, off);
-  if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = r;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float total = 0.0f;
-    for (int w = 0; w < slots / 32; ++w) total += warp_sum[w];
-    const int bh = channel / head_dim, c = channel % head_dim;
-    float lo = FLT_MAX, hi = -FLT_MAX;
-    const float2* rg = ranges + static_cast<int64_t>(bh) * chunks * head_dim + c;
-    for (int i = 0; i < chunks; ++i) {
-      const float2 x = __ldg(rg + static_cast<int64_t>(i) * head_dim);
-      lo = fminf(lo, x.x);
-      hi = fmaxf(hi, x.y);
-    }
+  for (int g = 0; g < 16; ++g) r[g] = 32 * g < slots ? __ldg(sums + 32 * g) : 0.0f;
+  const int bh = channel / head_dim, c = channel % head_dim;
+  const float2* rg = ranges + static_cast<int64_t>(bh) * chunks * head_dim + c;
+  float lo = FLT_MAX, hi = -FLT_MAX;
+  for (int i = lane; i < chunks; i += 32) {
+    const float2 x = __ldg(rg + static_cast<int64_t>(i) * head_dim);
+    lo = fminf(lo, x.x);
+    hi = fmaxf(hi, x.y);
+  }
+  float total = 0.0f;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, off));
+    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, off));
+#pragma unroll
+    for (int g = 0; g < 16; ++g) r[g] += __shfl_xor_sync(0xffffffffu, r[g], off);
+  }
+#pragma unroll
+  for (int g = 0; g < 16; ++g)
+    if (32 * g < slots) total += r[g];
+  if (lane == 0) {
     const float center = 0.5f * (lo + hi);
     const float radius = 0.5f * (hi - lo);
     const float sc = fmaxf(radius * (1.f / 127.f), 1e-12f);
@@ -159,6 +171,7 @@ __global__ void v_center_kernel(const float* __restrict__ residuals,
 struct VPlan {
   int chunks, slots;
   size_t range_bytes, residual_bytes;
+  size_t bytes() const { return range_bytes + residual_bytes; }
 };
 
 VPlan plan(int batch, int kv_heads, int k_len, int head_dim) {
@@ -180,7 +193,7 @@ extern "C" size_t risa_b200_quantize_v_workspace_size(int batch, int kv_heads, i
                                                       int head_dim) {
   if (batch <= 0 || kv_heads <= 0 || k_len <= 0 || head_dim <= 0) return 0;
   const VPlan p = plan(batch, kv_heads, k_len, head_dim);
-  return p.range_bytes + p.residual_bytes;
+  return p.bytes();
 }
 
 namespace {
@@ -213,8 +226,8 @@ int risa_b200::v_quantize_jobs(const void* v, void* v_codes, float* v_scale, flo
                "quantize_v: V base pointer and batch/head/sequence strides must be 16-byte "
                "aligned");
   const VPlan p = plan(batch, kv_heads, k_len, head_dim);
-  RISA_REQUIRE(workspace != nullptr && workspace_bytes >= p.range_bytes + p.residual_bytes,
-               "quantize_v: workspace of %zu bytes required", p.range_bytes + p.residual_bytes);
+  RISA_REQUIRE(workspace != nullptr && workspace_bytes >= p.bytes(),
+               "quantize_v: workspace of %zu bytes required", p.bytes());
   RISA_REQUIRE(reinterpret_cast<uintptr_t>(workspace) % 16 == 0,
                "quantize_v: workspace must be 16-byte aligned");
   range->v = v;
@@ -254,11 +267,11 @@ int risa_b200::v_quantize_jobs(const void* v, void* v_codes, float* v_scale, flo
       codes->steps = 0;
       codes->parts = p.slots / 128;  // a CTA keeps four windows of 32 residue classes
     } else {
-      // CTAs repeat the range reduction of their channels, so long sequences give them several
+      // CTAs repeat the range reduction of their channels, so long sequences give them up to sixteen
       // pieces each, as long as about two CTAs per SM remain
       const int64_t blocks = int64_t(batch) * kv_heads * (head_dim / kVChannels);
       const int pieces = (padded_len + kVPiece - 1) / kVPiece;
-      codes->steps = int(std::max<int64_t>(1, std::min<int64_t>(4, pieces * blocks / 296)));
+      codes->steps = int(std::max<int64_t>(1, std::min<int64_t>(16, pieces * blocks / 296)));
       codes->parts = (pieces + codes->steps - 1) / codes->steps;
     }
   }
@@ -285,7 +298,7 @@ int risa_b200::quantize_v_after_range(const void* v, void* v_codes, float* v_sca
       VCodesJob codes;
       v_quantize_jobs(v, v_codes, v_scale, v_center, batch, kv_heads, k_len, head_dim, padded_len,
                       stride_b, stride_h, stride_n, dtype_code, midpoint_affine, perm, workspace,
-                      p.range_bytes + p.residual_bytes, &range, &codes);
+                      p.bytes(), &range, &codes);
       const dim3 grid(codes.parts, channels / kVChannels);
       if (midpoint_affine)
         launch_chained(v_codes_kernel<T, true>, grid, dim3(kVThreads), 0, stream, codes);
@@ -305,8 +318,10 @@ int risa_b200::quantize_v_after_range(const void* v, void* v_codes, float* v_sca
             stride_h, stride_n, perm);
     }
     if (midpoint_affine)
-      launch_chained(v_center_kernel, dim3(channels), dim3(p.slots), 0, stream, residuals, ranges,
-                     v_center, k_len, head_dim, p.chunks, p.slots);
+      launch_chained(v_center_kernel,
+                     dim3((channels + kCenterThreads / 32 - 1) / (kCenterThreads / 32)),
+                     dim3(kCenterThreads), 0, stream, residuals, ranges, v_center, channels, k_len,
+                     head_dim, p.chunks, p.slots);
   });
   return check_launch("quantize_v");
 }

@@ -91,11 +91,11 @@ __device__ __forceinline__ int storage_position(int token) {
 // lanes of a group with two shuffle steps, after which a lane holds the whole 16-byte storage group
 // of one channel; neighbouring groups of a channel leave in the same store.  No shared memory and no
 // barrier per window, and key lengths need not be multiples of anything: missing tokens give code 0.
-//   absmax: a CTA walks `steps` pieces of 512 tokens x 64 channels, four windows in flight per lane.
+//   absmax: a CTA walks `steps` pieces of 128 tokens x 64 channels, up to four in flight per lane.
 //   midpoint-affine: the residuals have an order of their own (slot t of `slots` sums tokens Lk-1-t,
 //   Lk-1-t-slots, ...), so a lane keeps four residue classes of tokens modulo `slots` -- a class is
 //   one slot -- and walks them from the last token down.
-constexpr int kVChannels = 64, kVThreads = 512, kVPiece = 512;
+constexpr int kVChannels = 64, kVThreads = 512, kVPiece = 128;  // kVPiece: tokens of four windows
 
 // What the code step of one risa_b200_quantize_v call reads and writes.
 struct VCodesJob {
@@ -110,7 +110,7 @@ struct VCodesJob {
   const int32_t* perm;
   int midpoint_affine;
   int in_dim;        // as in VRangeJob
-  int steps, parts;  // 512-token pieces per CTA; CTAs per 64-channel block
+  int steps, parts;  // 128-token pieces per CTA; CTAs per 64-channel block
 };
 
 // Four channels of a row as they are in memory, converted when they are used.
@@ -237,11 +237,11 @@ __device__ __forceinline__ void v_codes_block(const VCodesJob& job, int part, in
   const int32_t* row_map = job.perm ? job.perm + static_cast<int64_t>(bh) * k_len : nullptr;
   // after the exchange the lane stores channel ch0 + word of its group
   int8_t* out = job.out + (out_row + ch0 + word) * padded_len + 16 * group;
-  auto load_tokens = [&](int base, Raw4<T> (&t)[4], bool (&have)[4]) {
+  auto load_tokens = [&](int base, int limit, Raw4<T> (&t)[4], bool (&have)[4]) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int token = base + first_token + (j & 1) + 8 * (j >> 1);
-      have[j] = token < k_len && present;
+      have[j] = token < limit && present;
       if (have[j]) {
         const int64_t row = row_map ? __ldg(row_map + token) : token;
         t[j].load(in + row * job.stride_n);
@@ -251,11 +251,13 @@ __device__ __forceinline__ void v_codes_block(const VCodesJob& job, int part, in
   if constexpr (!AFFINE) {
     constexpr int U = sizeof(T) == 2 ? 4 : 2;  // windows in flight
     const int end = min(padded_len, (part + 1) * job.steps * kVPiece);
-    for (int base0 = part * job.steps * kVPiece + (warp >> 2) * 32; base0 < end; base0 += U * 128) {
+    for (int base0 = part * job.steps * kVPiece + (warp >> 2) * 32; base0 < end;
+         base0 += U * kVPiece) {
       Raw4<T> t[U][4];
       bool have[U][4];
 #pragma unroll
-      for (int u = 0; u < U; ++u) load_tokens(base0 + 128 * u, t[u], have[u]);
+      for (int u = 0; u < U; ++u)
+        load_tokens(base0 + kVPiece * u, min(k_len, end), t[u], have[u]);
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         float x[4][4];
@@ -269,14 +271,13 @@ __device__ __forceinline__ void v_codes_block(const VCodesJob& job, int part, in
 #pragma unroll
         for (int c = 0; c < 4; ++c) words[c] = pack4_s8(x[0][c], x[1][c], x[2][c], x[3][c]);
         transpose_words(words, lane);
-        if (base0 + 128 * u < end)
-          *reinterpret_cast<uint4*>(out + base0 + 128 * u) =
+        if (base0 + kVPiece * u < end)
+          *reinterpret_cast<uint4*>(out + base0 + kVPiece * u) =
               make_uint4(words[0], words[1], words[2], words[3]);
       }
     }
   } else {
     const int residue = (part * 4 + (warp >> 2)) * 32;  // first class of this warp's window
-    if (residue >= slots) return;
     float residual[4][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j)
@@ -287,7 +288,7 @@ __device__ __forceinline__ void v_codes_block(const VCodesJob& job, int part, in
     for (int base = top; base >= 0; base -= slots) {
       Raw4<T> t[4];
       bool have[4];
-      load_tokens(base, t, have);
+      load_tokens(base, k_len, t, have);
       uint32_t code[4][4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
