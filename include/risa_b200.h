@@ -64,7 +64,7 @@ int risa_b200_quantize_v(const void* v, void* v_codes, float* v_scale, float* v_
  * Same results as risa_b200_quantize_qk followed by risa_b200_quantize_v with the same arguments
  * (kv_perm is the gather table of both K and V) in two launches: the steps that depend on nothing
  * (K anchor detection, V range pass, Q quantiser), then the steps that depend on those (K quantiser,
- * V code pass; key lengths that are not a multiple of 16 keep a separate V launch). */
+ * V code pass). */
 int risa_b200_quantize_qkv(const void* q, void* q_codes, float* q_scale, const void* k,
                            void* k_codes, float* k_scale, const void* v, void* v_codes,
                            float* v_scale, float* v_center, int batch, int q_heads, int q_len,
@@ -195,6 +195,51 @@ int risa_b200_dense_attention(const void* q, const void* k, const void* v, void*
                               int dtype_code, int midpoint_affine, float sm_scale,
                               int out_dtype_code, int64_t o_stride_b, int64_t o_stride_n,
                               int64_t o_stride_h, int is_causal, void* stream);
+
+/* ---- struct form (the torch binding's) ---------------------------------------------------------
+ * The same work as the entries above for callers that hold a whole call together, with three things
+ * those do not have: inputs whose head dim `in_dim` (a multiple of 4) is narrower than the kernel's
+ * `head_dim` are read as if padded with zeros, without a padded copy; outputs may be stored as FP32
+ * (dtype_code 0: the bf16 values, `cols` channels per row); and the LSE may have a per-row shift
+ * added where it is written.  The last two need the tensor-core kernel:
+ * risa_b200_finishes_outputs() says whether it takes a shape on the calling thread.  Strides are in
+ * elements, [batch, head, sequence].  No counterpart in the reference. */
+typedef struct risa_b200_operands {
+  const void *q, *k, *v;
+  int64_t q_strides[3], k_strides[3], v_strides[3];
+  int batch, q_heads, kv_heads, q_len, k_len;
+  int head_dim, in_dim; /* kernel head dim (64, 128, 256) and that of q, k, v */
+  int cta_k, dtype_code, midpoint_affine;
+  const int32_t* kv_perm; /* gather table of K and V, or NULL */
+} risa_b200_operands;
+typedef struct risa_b200_packed {
+  void *q_codes, *k_codes, *v_codes;
+  float *q_scale, *k_scale, *v_scale, *v_center;
+  int32_t* anchors;
+  void* workspace;
+  size_t workspace_bytes;
+} risa_b200_packed;
+typedef struct risa_b200_attention_out {
+  void* o;
+  int64_t o_strides[3];
+  int dtype_code, cols;
+  float* lse;             /* or NULL */
+  const float* lse_shift; /* added to lse, or NULL */
+} risa_b200_attention_out;
+int risa_b200_finishes_outputs(int head_dim, int cta_k, int k_len);
+/* Bytes of one block (256-byte aligned) that holds a call's packed operands, quantiser workspace and
+ * last-wave parts; with `packed` non-NULL also fills in the addresses inside the block at `base`. */
+size_t risa_b200_packed_layout(const risa_b200_operands* shape, char* base, risa_b200_packed* packed,
+                               void** tail, size_t* tail_bytes);
+/* lse_shift: [B,Hq,Lq] floats to receive the LSE correction of the K anchors, or NULL. */
+int risa_b200_quantize_operands(const risa_b200_operands* in, const risa_b200_packed* out,
+                                float sm_scale, float* lse_shift, void* stream);
+int risa_b200_attend(const risa_b200_operands* shape, const risa_b200_packed* packed,
+                     const risa_b200_attention_out* out, float sm_scale, int is_causal,
+                     const void* mask, const int64_t* mask_strides, int mask_dtype_code,
+                     const int32_t* key_mask_tiles, const int32_t* row_offsets,
+                     const int32_t* block_indices, void* scratch, size_t scratch_bytes,
+                     void* stream);
 
 /* Selects which attention kernel family calls made BY THE CALLING THREAD may use: 0 = automatic
  * (tensor-core kernel where it applies, in the instantiation for the call's class: no mask / causal

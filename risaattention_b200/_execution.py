@@ -8,21 +8,67 @@ import math
 import torch
 
 from . import _backend
-from ._key_mask import prepare_key_mask_tiles
-from ._quantization import (PackedBuffers, pad_head_dim, quantize_into, resolve_scale)
+from ._key_mask import prepare_key_mask_tiles, wants_key_mask_tiles
+from ._quantization import (PackedBuffers, pad_head_dim, prequantize_int8_attention, quantize_into,
+                            resolve_scale)
 from ._types import PrequantizedInt8Attention, RetainedMassPattern
 from ._validation import (DTYPE_CODES, MIN_PATTERN_SPARSITY, OUTPUT_LAYOUTS, UNAVAILABLE,
-                          is_available, mask_signature, select_key_block_size, validate_inputs)
+                          is_available, kernel_head_dim, mask_signature, select_key_block_size,
+                          uses_centered_values, validate_inputs)
 
 
 def _output_dtype(input_dtype):
     return torch.bfloat16 if input_dtype == torch.float32 else input_dtype
 
 
+def _whole_call(call, q, k, v, attn_mask, kv_table, scale, use_midpoint_affine, is_causal,
+                return_lse):
+    """Everything of a dense call -- buffers, quantisation, attention, LSE -- in one native call;
+    inputs narrower than the kernel's head dim are not copied and FP32 results come from the kernel."""
+    head_dim = q.shape[-1]
+    attention_scale = resolve_scale(scale, head_dim)
+    dim = kernel_head_dim(head_dim)
+    key_block_size = select_key_block_size(
+        dim, k.shape[2], has_mask=attn_mask is not None and attn_mask.stride(-2) != 0)
+    return call(q, k, v, attn_mask, kv_table, key_block_size, dim, use_midpoint_affine,
+                attention_scale, is_causal,
+                wants_key_mask_tiles(attn_mask, q.shape[2], attention_scale, is_causal), return_lse,
+                _backend.current_stream_ptr(q.device))
+
+
+def execute_permuted_or_lse_attention(q, k, v, *, scale, attn_mask, v_quantization, is_causal,
+                                      return_lse, kv_permutation, fuse_gather):
+    """``int8_attention`` with LSE output or a K/V permutation: quantisation and attention as in
+    ``prequantize_int8_attention`` + ``int8_attention_from_prequantized``, in one native call."""
+    call = getattr(_backend._C, "attention_call", None)
+    if call is None:
+        packed = prequantize_int8_attention(
+            q, k, v, scale=scale, attn_mask=attn_mask, v_quantization=v_quantization,
+            is_causal=is_causal, return_lse=return_lse, kv_permutation=kv_permutation,
+            fuse_gather=fuse_gather)
+        return int8_attention_from_prequantized(packed, return_lse=return_lse)
+    attn_mask = validate_inputs(q, k, v, attn_mask)
+    kv_table = None
+    if kv_permutation is not None:
+        from .permutation import prepare_inputs
+
+        q, k, v, kv_table = prepare_inputs(q, k, v, permutation=kv_permutation, mask=attn_mask,
+                                           causal=is_causal, return_lse=return_lse,
+                                           fuse=fuse_gather)
+    output, lse = _whole_call(call, q, k, v, attn_mask, kv_table, scale,
+                              uses_centered_values(v_quantization), is_causal, return_lse)
+    return (output, lse) if return_lse else output
+
+
 def execute_dense_attention(q, k, v, *, scale=None, attn_mask=None, use_midpoint_affine=False,
                             is_causal=False):
     """Single-call path: quantise and attend on the current stream; scratch lives only for the call."""
     attn_mask = validate_inputs(q, k, v, attn_mask)
+    call = getattr(_backend._C, "attention_call", None)
+    if call is not None:
+        return _whole_call(call, q, k, v, attn_mask, None, scale, use_midpoint_affine, is_causal,
+                           False)[0]
+    # a native surface without whole calls (an older build of the library under comparison)
     input_dtype = q.dtype
     q, k, v, original_head_dim, dim = pad_head_dim(q, k, v)
     attention_scale = resolve_scale(scale, original_head_dim)
@@ -145,6 +191,19 @@ def int8_attention_from_prequantized(quantized, *, sparse_pattern=None, output_l
         raise RuntimeError(UNAVAILABLE)
 
     batch, q_heads, q_len, dim = quantized.q.shape
+    call = getattr(_backend._C, "attend_call", None)
+    if call is not None and _block_mass is None:
+        output, lse = call(
+            quantized.q, quantized.k, quantized.v, quantized.q_scale, quantized.k_scale,
+            quantized.v_scale, quantized.v_center, quantized.cta_k, quantized.attention_scale,
+            DTYPE_CODES[quantized.input_dtype], quantized.original_head_dim, quantized.attn_mask,
+            None if sparse_pattern is None else sparse_pattern.row_offsets,
+            None if sparse_pattern is None else sparse_pattern.block_indices, quantized.is_causal,
+            sparse_pattern is None and wants_key_mask_tiles(
+                quantized.attn_mask, q_len, quantized.attention_scale, quantized.is_causal),
+            quantized.lse_shift if return_lse else None, output_layout == "nhd",
+            _backend.current_stream_ptr(device))
+        return (output, lse) if return_lse else output
     out_dtype = _output_dtype(quantized.input_dtype)
     output = allocate_output(quantized, output_layout)
     lse = torch.empty((batch, q_heads, q_len), dtype=torch.float32, device=device) \

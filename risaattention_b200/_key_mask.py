@@ -5,9 +5,13 @@ import torch
 from . import _backend
 
 
+def wants_key_mask_tiles(mask, query_length, scale, is_causal) -> bool:
+    return (mask is not None and mask.stride(-2) == 0 and mask.shape[-1] > 1024
+            and query_length >= 256 and scale > 0 and not is_causal)
+
+
 def prepare_key_mask_tiles(mask, key_block_size, query_length, scale, is_causal):
-    if mask is None or mask.stride(-2) != 0 or mask.shape[-1] <= 1024 or query_length < 256 \
-            or scale <= 0 or is_causal:
+    if not wants_key_mask_tiles(mask, query_length, scale, is_causal):
         return None
     batch, heads, _, length = mask.shape
     tiles = torch.empty((batch, heads, -(-length // key_block_size) + 1), device=mask.device,

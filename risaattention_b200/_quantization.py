@@ -88,6 +88,23 @@ def prequantize_int8_attention(q, k, v, *, scale=None, attn_mask=None, v_quantiz
                                            fuse=fuse_gather)
     use_midpoint_affine = uses_centered_values(v_quantization)
     input_dtype = q.dtype
+    call = getattr(_backend._C, "quantize_call", None)
+    if call is not None:
+        head_dim = q.shape[-1]
+        attention_scale = resolve_scale(scale, head_dim)
+        dim = kernel_head_dim(head_dim)
+        key_block_size = select_key_block_size(
+            dim, k.shape[2], has_mask=attn_mask is not None and attn_mask.stride(-2) != 0)
+        (q_codes, k_codes, v_codes, q_scale, k_scale, v_scale, v_center, lse_shift) = call(
+            q, k, v, kv_table, key_block_size, dim, use_midpoint_affine, attention_scale,
+            return_lse, _backend.current_stream_ptr(q.device))
+        return PrequantizedInt8Attention(
+            q=q_codes, k=k_codes, v=v_codes, q_scale=q_scale, k_scale=k_scale, v_scale=v_scale,
+            v_center=v_center, original_head_dim=head_dim, input_dtype=input_dtype,
+            attention_scale=attention_scale, cta_k=key_block_size, attn_mask=attn_mask,
+            v_quantization=v_quantization, is_causal=is_causal, lse_shift=lse_shift,
+            kv_permuted=kv_permutation is not None)
+    # a native surface without whole calls (an older build of the library under comparison)
     q, k, v, original_head_dim, _ = pad_head_dim(q, k, v)
     attention_scale = resolve_scale(scale, original_head_dim)
     key_block_size = select_key_block_size(

@@ -90,7 +90,7 @@ int run_attention(
     int out_dtype_code, const int32_t* sparse_row_offsets, const int32_t* sparse_block_indices,
     float* block_mass, int is_causal, float* lse, const int32_t* key_mask_tiles,
     void* stream_ptr, const SelectRequest* select, float* tail_scratch = nullptr,
-    size_t tail_scratch_bytes = 0) {
+    size_t tail_scratch_bytes = 0, int out_cols = 0, const float* lse_shift = nullptr) {
   RISA_REQUIRE(cta_k == 64 || cta_k == 128, "risa_attention: cta_k must be 64 or 128");
   RISA_REQUIRE(head_dim == 64 || head_dim == 128 || head_dim == 256,
                "risa_attention: unsupported head_dim");
@@ -105,7 +105,7 @@ int run_attention(
   RISA_REQUIRE(batch > 0 && q_len > 0 && k_len > 0 && q_heads > 0 && kv_heads > 0 &&
                    q_heads % kv_heads == 0,
                "risa_attention: sizes must be positive and q heads divisible by kv heads");
-  RISA_REQUIRE(out_dtype_code == 1 || out_dtype_code == 2,
+  RISA_REQUIRE(out_dtype_code == 1 || out_dtype_code == 2 || (out_dtype_code == 0 && out_cols > 0),
                "risa_attention: output_dtype_code must be 1 (fp16) or 2 (bf16)");
   RISA_REQUIRE(mask == nullptr || (mask_dtype_code >= 0 && mask_dtype_code <= 3),
                "risa_attention: attention mask must be bool, float16, bfloat16, or float32");
@@ -142,6 +142,8 @@ int run_attention(
   a.o_stride_h = o_stride_h;
   a.sm_scale = sm_scale;
   a.out_dtype_code = out_dtype_code;
+  a.out_cols = out_cols;
+  a.lse_shift = lse_shift;
   a.row_offsets = sparse_row_offsets;
   a.block_indices = sparse_block_indices;
   a.block_mass = block_mass;
@@ -173,8 +175,11 @@ int run_attention(
   int status;
   if (g_attention_path != 1 && attention_tc_supported(a))
     status = attention_tc(a, stream, g_attention_path == 2);
-  else
+  else {
+    RISA_REQUIRE(out_dtype_code != 0 && lse_shift == nullptr,
+                 "risa_attention: FP32 outputs and LSE shifts are the tensor-core kernel's");
     status = attention_rows(a, stream);
+  }
   if (status != RISA_B200_OK) return status;
   if (block_mass) {
     const int n_q = (q_len + 127) / 128, n_k = (k_len + cta_k - 1) / cta_k;
@@ -374,4 +379,77 @@ extern "C" int risa_b200_dense_attention(
                        q_heads, kv_heads, head_dim, o_stride_b, o_stride_n, o_stride_h, sm_scale,
                        out_dtype_code, nullptr, nullptr, nullptr, is_causal, nullptr, nullptr,
                        stream, nullptr, reinterpret_cast<float*>(base + s.tail), s.total - s.tail);
+}
+
+// ---- one call over unpacked or packed operands (struct form, the torch binding's) ----------------
+extern "C" int risa_b200_finishes_outputs(int head_dim, int cta_k, int k_len) {
+  return g_attention_path != 1 && risa_b200::attention_tc_shape(head_dim, cta_k, k_len) ? 1 : 0;
+}
+
+extern "C" int risa_b200_quantize_operands(const risa_b200_operands* in,
+                                           const risa_b200_packed* out, float sm_scale,
+                                           float* lse_shift, void* stream) {
+  using namespace risa_b200;
+  RISA_REQUIRE(in != nullptr && out != nullptr, "quantize_operands: null argument");
+  RISA_REQUIRE(in->cta_k == 64 || in->cta_k == 128, "quantize_operands: cta_k must be 64 or 128");
+  const int padded = (in->k_len + in->cta_k - 1) / in->cta_k * in->cta_k;
+  const int status = quantize_qkv_narrow(
+      in->q, out->q_codes, out->q_scale, in->k, out->k_codes, out->k_scale, in->v, out->v_codes,
+      out->v_scale, out->v_center, in->batch, in->q_heads, in->q_len, in->kv_heads, in->k_len,
+      in->head_dim, in->in_dim, in->cta_k, padded, in->q_strides[0], in->q_strides[1],
+      in->q_strides[2], in->k_strides[0], in->k_strides[1], in->k_strides[2], in->v_strides[0],
+      in->v_strides[1], in->v_strides[2], in->dtype_code, in->midpoint_affine, out->anchors, nullptr,
+      in->kv_perm, out->workspace, out->workspace_bytes, stream);
+  if (status != RISA_B200_OK || lse_shift == nullptr) return status;
+  return risa_b200_correct_lse(in->q, in->k, out->anchors, lse_shift, in->batch, in->q_heads,
+                               in->kv_heads, in->q_len, in->in_dim, in->q_strides[0],
+                               in->q_strides[1], in->q_strides[2], in->k_strides[0],
+                               in->k_strides[1], in->k_strides[2], sm_scale, in->dtype_code, stream);
+}
+
+extern "C" int risa_b200_attend(const risa_b200_operands* shape, const risa_b200_packed* packed,
+                                const risa_b200_attention_out* out, float sm_scale, int is_causal,
+                                const void* mask, const int64_t* mask_strides, int mask_dtype_code,
+                                const int32_t* key_mask_tiles, const int32_t* row_offsets,
+                                const int32_t* block_indices, void* scratch, size_t scratch_bytes,
+                                void* stream) {
+  using namespace risa_b200;
+  RISA_REQUIRE(shape && packed && out, "attend: null argument");
+  static const int64_t none[4] = {0, 0, 0, 0};
+  const int64_t* ms = mask ? mask_strides : none;
+  return run_attention(packed->q_codes, packed->k_codes, packed->v_codes, out->o, packed->q_scale,
+                       packed->k_scale, packed->v_scale, packed->v_center, mask, ms[0], ms[1], ms[2],
+                       ms[3], mask_dtype_code, shape->cta_k, shape->batch, shape->q_len,
+                       shape->k_len, shape->q_heads, shape->kv_heads, shape->head_dim,
+                       out->o_strides[0], out->o_strides[2], out->o_strides[1], sm_scale,
+                       out->dtype_code, row_offsets, block_indices, nullptr, is_causal, out->lse,
+                       key_mask_tiles, stream, nullptr, static_cast<float*>(scratch), scratch_bytes,
+                       out->cols, out->lse_shift);
+}
+
+// Offsets of the packed operands of a call inside one block, in the order of risa_b200_packed.
+extern "C" size_t risa_b200_packed_layout(const risa_b200_operands* shape, char* base,
+                                          risa_b200_packed* packed, void** tail,
+                                          size_t* tail_bytes) {
+  using namespace risa_b200;
+  const size_t need = risa_b200_dense_scratch_size(shape->batch, shape->q_heads, shape->q_len,
+                                                   shape->kv_heads, shape->k_len, shape->head_dim,
+                                                   shape->cta_k);
+  if (need == 0 || packed == nullptr) return need;
+  const DenseScratch s = dense_scratch_layout(shape->batch, shape->q_heads, shape->q_len,
+                                              shape->kv_heads, shape->k_len, shape->head_dim,
+                                              shape->cta_k);
+  packed->q_codes = base + s.q_codes;
+  packed->k_codes = base + s.k_codes;
+  packed->v_codes = base + s.v_codes;
+  packed->q_scale = reinterpret_cast<float*>(base + s.q_scale);
+  packed->k_scale = reinterpret_cast<float*>(base + s.k_scale);
+  packed->v_scale = reinterpret_cast<float*>(base + s.v_scale);
+  packed->v_center = reinterpret_cast<float*>(base + s.v_center);
+  packed->anchors = reinterpret_cast<int32_t*>(base + s.anchors);
+  packed->workspace = base + s.v_work;
+  packed->workspace_bytes = s.tail - s.v_work;
+  *tail = base + s.tail;
+  *tail_bytes = s.total - s.tail;
+  return need;
 }

@@ -37,7 +37,9 @@ struct AttentionArgs {
   int cta_k, batch, q_len, k_len, q_heads, kv_heads, head_dim;
   int64_t o_stride_b, o_stride_n, o_stride_h;  // in elements
   float sm_scale;
-  int out_dtype_code;  // 1 = fp16, 2 = bf16
+  int out_dtype_code;  // 1 = fp16, 2 = bf16; 0 = values rounded to bf16 and stored as fp32 (TC kernel)
+  int out_cols;        // channels of a row that are stored (out_dtype_code 0; a multiple of 4)
+  const float* lse_shift;  // [B,Hq,Lq] added to the LSE, or null (TC kernel)
   const int32_t* row_offsets;
   const int32_t* block_indices;
   float* block_mass;
@@ -141,6 +143,8 @@ bool attention_tc_supported(const AttentionArgs& a);
 // call's class (the results are the same bits; a diagnostic).
 int attention_tc(const AttentionArgs& a, cudaStream_t stream, bool every_path = false);
 int attention_tc_select_max_tiles(int cta_k);
+// Whether the tensor-core kernel takes a call of this shape on this thread (operand alignment aside).
+bool attention_tc_shape(int head_dim, int cta_k, int k_len);
 // Parts per CTA of the last wave (0: whole CTAs) for a dense unmasked launch; attention_tc.cu.
 int attention_tc_split_parts(int ctas, int n_k, int cta_k, int sms);
 

@@ -1332,6 +1332,43 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       uint4* staged = reinterpret_cast<uint4*>(smem + L::out_stage) + (warp & 3) * 32 * L::kOutPitch;
 #pragma unroll
       for (int c0 = 0; c0 < kOut; c0 += 64) {
+        if (MODE == kDense && a.out_dtype_code == 0) {
+          // FP32 callers: the bf16 value of each element stored as FP32, 32 channels at a time
+#pragma unroll
+          for (int c1 = c0; c1 < c0 + 64; c1 += 32) {
+#pragma unroll
+            for (int ch = c1; ch < c1 + 32; ch += 4) {
+              const ulonglong2 scale4 = *reinterpret_cast<const ulonglong2*>(vs + ch);
+              const ulonglong2 centre4 = *reinterpret_cast<const ulonglong2*>(vc + ch);
+              uint32_t word[4];
+#pragma unroll
+              for (int i = 0; i < 2; ++i) {
+                float r0, r1;
+                unpack_f32x2(fma_f32x2(mul_f32x2(O2[(ch >> 1) + i], inv2), i ? scale4.y : scale4.x,
+                                       i ? centre4.y : centre4.x), r0, r1);
+                const __nv_bfloat162 h = __floats2bfloat162_rn(r0, r1);
+                uint32_t both = *reinterpret_cast<const uint32_t*>(&h);
+                if (!PLAIN) both = zero ? 0u : both;
+                word[2 * i] = both << 16;
+                word[2 * i + 1] = both & 0xffff0000u;
+              }
+              staged[lane * L::kOutPitch + (ch - c1) / 4] =
+                  make_uint4(word[0], word[1], word[2], word[3]);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int r = 4 * i + lane / 8, col = kOut * half + c1 + 4 * (lane % 8);
+              const uint4 piece = staged[r * L::kOutPitch + lane % 8];
+              if (row - lane + r < a.q_len && col < a.out_cols)
+                *reinterpret_cast<uint4*>(static_cast<float*>(a.o) + batch * a.o_stride_b +
+                                          head * a.o_stride_h +
+                                          int64_t(row - lane + r) * a.o_stride_n + col) = piece;
+            }
+            __syncwarp();
+          }
+          continue;
+        }
         // the element type is the same for the whole launch: one branch per 64 channels
         auto finish = [&](auto to_half) {
 #pragma unroll
@@ -1377,15 +1414,20 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
         __syncwarp();
       }
       // the LSE wants the denominator's own reference point: the stale maximum without capture
-      if (a.lse && half == 0 && row_ok) a.lse[grow] = row_lse(denom, CAPTURE ? st.m : m_o);
+      if (a.lse && half == 0 && row_ok) {
+        const float lse = row_lse(denom, CAPTURE ? st.m : m_o);
+        a.lse[grow] = a.lse_shift ? lse + __ldg(a.lse_shift + grow) : lse;
+      }
     } else if (row_ok) {
       // a wait of this CTA expired: mark the rows it owns, so that a failed launch cannot be taken
-      // for a result (NaN in both 16-bit output formats, NaN LSE)
-      char* o_row = static_cast<char*>(a.o) + 2 * kOut * half +
-                    2 * (batch * a.o_stride_b + head * a.o_stride_h + int64_t(row) * a.o_stride_n);
-#pragma unroll
-      for (int ch = 0; ch < kOut; ch += 8)
-        *reinterpret_cast<uint4*>(o_row + 2 * ch) =
+      // for a result (NaN in every output format, NaN LSE)
+      const int esize = a.out_dtype_code == 0 ? 4 : 2;
+      const int cols = a.out_dtype_code == 0 ? min(kOut, a.out_cols - kOut * half) : kOut;
+      char* o_row = static_cast<char*>(a.o) +
+                    esize * (kOut * half + batch * a.o_stride_b + head * a.o_stride_h +
+                             int64_t(row) * a.o_stride_n);
+      for (int at = 0; at < cols * esize; at += 16)
+        *reinterpret_cast<uint4*>(o_row + at) =
             make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
       if (a.lse && half == 0) a.lse[grow] = __int_as_float(0x7fffffff);
     }
@@ -1643,8 +1685,9 @@ __global__ __launch_bounds__(128) void tail_merge_kernel(const AttentionArgs a, 
   const float inv = rcp_approx(denom);
   const float* vs = a.v_scale + kvh * a.head_dim + k_out * half + ch0;
   const float* vc = a.v_center + kvh * a.head_dim + k_out * half + ch0;
-  char* o_row = static_cast<char*>(a.o) + 2 * (k_out * half + ch0) +
-                2 * (batch * a.o_stride_b + head * a.o_stride_h + int64_t(row) * a.o_stride_n);
+  const int64_t o_at = k_out * half + ch0 + batch * a.o_stride_b + head * a.o_stride_h +
+                       int64_t(row) * a.o_stride_n;
+  char* o_row = static_cast<char*>(a.o) + 2 * o_at;
 #pragma unroll
   for (int ch = 0; ch < kMergeChannels; ch += 8) {
     uint32_t packed[4];
@@ -1668,10 +1711,23 @@ __global__ __launch_bounds__(128) void tail_merge_kernel(const AttentionArgs a, 
         packed[i] = *reinterpret_cast<const uint32_t*>(&h);
       }
     }
-    *reinterpret_cast<uint4*>(o_row + 2 * ch) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+    if (a.out_dtype_code == 0) {  // the bf16 values as FP32
+#pragma unroll
+      for (int i = 0; i < 4; i += 2)
+        if (k_out * half + ch0 + ch + 2 * i < a.out_cols)
+          *reinterpret_cast<uint4*>(static_cast<float*>(a.o) + o_at + ch + 2 * i) =
+              make_uint4(packed[i] << 16, packed[i] & 0xffff0000u, packed[i + 1] << 16,
+                         packed[i + 1] & 0xffff0000u);
+    } else {
+      *reinterpret_cast<uint4*>(o_row + 2 * ch) =
+          make_uint4(packed[0], packed[1], packed[2], packed[3]);
+    }
   }
-  if (a.lse && half == 0 && blockIdx.y == 0)
-    a.lse[(int64_t(batch) * a.q_heads + head) * a.q_len + row] = row_lse(denom, m);
+  if (a.lse && half == 0 && blockIdx.y == 0) {
+    const int64_t grow = (int64_t(batch) * a.q_heads + head) * a.q_len + row;
+    const float lse = row_lse(denom, m);
+    a.lse[grow] = a.lse_shift ? lse + __ldg(a.lse_shift + grow) : lse;
+  }
 }
 
 // How the last, partial wave of a dense unmasked launch is split (0 = not at all).  With C whole
@@ -1810,15 +1866,18 @@ int launch_tc(const AttentionArgs& a, const CUtensorMap& map_q, const CUtensorMa
 // the packed formats define for it); every mask form, causal, tile lists, capture.  The packed V row
 // must hold at least one 128-key slab (the V box is always 128 keys wide) and TMA needs 16-byte
 // aligned operand bases; anything else goes to the row-per-thread kernel.
+bool attention_tc_shape(int head_dim, int cta_k, int k_len) {
+  const int64_t padded = int64_t((k_len + cta_k - 1) / cta_k) * cta_k;
+  return (((head_dim == 128 || head_dim == 256) && (cta_k == 128 || cta_k == 64)) ||
+          (head_dim == 64 && cta_k == 64)) && padded >= 128;
+}
+
 bool attention_tc_supported(const AttentionArgs& a) {
-  const int64_t padded = int64_t((a.k_len + a.cta_k - 1) / a.cta_k) * a.cta_k;
-  const bool shape = ((a.head_dim == 128 || a.head_dim == 256) &&
-                      (a.cta_k == 128 || a.cta_k == 64)) ||
-                     (a.head_dim == 64 && a.cta_k == 64);
+  const int pieces = a.out_dtype_code == 0 ? 4 : 8;  // elements of a 16-byte store
   auto aligned16 = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
-  return shape && padded >= 128 && encode_fn() != nullptr && aligned16(a.q) && aligned16(a.k) &&
-         aligned16(a.v) && aligned16(a.o) && a.o_stride_b % 8 == 0 &&
-         a.o_stride_h % 8 == 0 && a.o_stride_n % 8 == 0;
+  return attention_tc_shape(a.head_dim, a.cta_k, a.k_len) && encode_fn() != nullptr && aligned16(a.q) && aligned16(a.k) &&
+         aligned16(a.v) && aligned16(a.o) && a.o_stride_b % pieces == 0 &&
+         a.o_stride_h % pieces == 0 && a.o_stride_n % pieces == 0;
 }
 
 int attention_tc(const AttentionArgs& args, cudaStream_t stream, bool every_path) {

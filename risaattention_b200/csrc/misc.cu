@@ -28,6 +28,8 @@ __global__ __launch_bounds__(kShiftThreads) void lse_shift_rows_kernel(
     float* __restrict__ out, int q_heads, int kv_heads, int q_len, int head_dim, int64_t q_stride_b,
     int64_t q_stride_h, int64_t q_stride_n, int64_t k_stride_b, int64_t k_stride_h,
     int64_t k_stride_n, float scale) {
+  chain_wait();
+  chain_release();
   __shared__ float anchor_row[256];
   const int head = blockIdx.y, batch = blockIdx.z;
   const int kv_head = head / (q_heads / kv_heads);
@@ -241,7 +243,7 @@ extern "C" int risa_b200_correct_lse(const void* q, const void* k, const int32_t
   RISA_REQUIRE(head_dim <= 256, "lse_shift: head_dim must not exceed 256");
   const dim3 grid((q_len + kShiftRows - 1) / kShiftRows, q_heads, batch);
   RISA_DISPATCH_FLOAT(dtype_code, T, {
-    lse_shift_rows_kernel<T><<<grid, kShiftThreads, 0, stream>>>(
+    launch_chained(lse_shift_rows_kernel<T>, grid, dim3(kShiftThreads), 0, stream,
         static_cast<const T*>(q), static_cast<const T*>(k), anchors, out, q_heads, kv_heads, q_len,
         head_dim, qb, qh, qn, kb, kh, kn, scale);
   });

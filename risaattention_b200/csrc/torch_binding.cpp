@@ -156,14 +156,17 @@ void attend_tensors(const at::Tensor& q_int8, const at::Tensor& k_int8, const at
                     const std::optional<at::Tensor>& block_indices,
                     const std::optional<at::Tensor>& block_mass, bool is_causal,
                     const std::optional<at::Tensor>& lse,
-                    const std::optional<at::Tensor>& key_mask_tiles) {
+                    const std::optional<at::Tensor>& key_mask_tiles,
+                    const float* lse_shift = nullptr, int fp32_cols = 0) {
+  // lse_shift, fp32_cols: see risa_b200_attention_out; an FP32 output has fp32_cols channels
   const c10::DeviceGuard on_device(q_int8.device());
   // checked in the order of the reference module (csrc/bindings.cpp:290-432)
   if (q_int8.dim() != 4 || k_int8.dim() != 4 || v_int8.dim() != 2 || o.dim() != 4)
     throw std::runtime_error("risa_sdpa_prequantized: q/k/o must be 4D and packed v must be 2D");
   if (cta_k != 64 && cta_k != 128)
     throw std::runtime_error("risa_sdpa_prequantized: cta_k must be 64 or 128");
-  if (output_dtype_code != 1 && output_dtype_code != 2)
+  if (output_dtype_code != 1 && output_dtype_code != 2 &&
+      !(output_dtype_code == 0 && fp32_cols > 0))
     throw std::runtime_error(
         "risa_sdpa_prequantized: output_dtype_code must be 1 (fp16) or 2 (bf16)");
   const int64_t b = q_int8.size(0), hq = q_int8.size(1), lq = q_int8.size(2), d = q_int8.size(3);
@@ -177,12 +180,14 @@ void attend_tensors(const at::Tensor& q_int8, const at::Tensor& k_int8, const at
   if (block_mass.has_value() && row_offsets.has_value())
     throw std::runtime_error("risa_sdpa_prequantized: block mass requires dense attention");
   if (v_int8.size(0) != b * hkv * d || v_int8.size(1) != padded ||
-      o.size(0) != b || o.size(1) != hq || o.size(2) != lq || o.size(3) != d ||
+      o.size(0) != b || o.size(1) != hq || o.size(2) != lq || o.size(3) != (fp32_cols > 0 ? fp32_cols : d) ||
       k_int8.size(0) != b || k_int8.size(3) != d)
     throw std::runtime_error("risa_sdpa_prequantized: incompatible quantized tensor shapes");
   if (q_int8.scalar_type() != at::kChar || k_int8.scalar_type() != at::kChar ||
       v_int8.scalar_type() != at::kChar ||
-      o.scalar_type() != (output_dtype_code == 1 ? at::kHalf : at::kBFloat16))
+      o.scalar_type() != (output_dtype_code == 1   ? at::kHalf
+                          : output_dtype_code == 2 ? at::kBFloat16
+                                                   : at::kFloat))
     throw std::runtime_error("risa_sdpa_prequantized: packed operands must be int8 and the "
                              "output of the type output_dtype_code names");
   const int64_t q_blocks = (lq + 127) / 128, k_tiles = padded / cta_k;
@@ -192,8 +197,9 @@ void attend_tensors(const at::Tensor& q_int8, const at::Tensor& k_int8, const at
       !v_scale.is_contiguous() || !v_center.is_contiguous())
     throw std::runtime_error("risa_sdpa_prequantized: scale and centre tensors must be "
                              "contiguous float32 with one entry per quantization group");
-  const bool hnd = (lq <= 1 || o.stride(2) == d) && (hq <= 1 || o.stride(1) == lq * d);
-  const bool nhd = (hq <= 1 || o.stride(1) == d) && (lq <= 1 || o.stride(2) == hq * d);
+  const int64_t od = o.size(3);
+  const bool hnd = (lq <= 1 || o.stride(2) == od) && (hq <= 1 || o.stride(1) == lq * od);
+  const bool nhd = (hq <= 1 || o.stride(1) == od) && (lq <= 1 || o.stride(2) == hq * od);
   if (!q_int8.is_contiguous() || !k_int8.is_contiguous() || !v_int8.is_contiguous() ||
       o.stride(3) != 1 || !(hnd || nhd))
     throw std::runtime_error("risa_sdpa_prequantized: quantized tensors must be contiguous and "
@@ -233,9 +239,9 @@ void attend_tensors(const at::Tensor& q_int8, const at::Tensor& k_int8, const at
     throw std::runtime_error("risa_sdpa_prequantized: block_mass workspace must contain "
                              "mass rows followed by captured tile statistics and softmax state");
   if (key_mask_tiles.has_value()) require_key_mask_tiles(*key_mask_tiles, b, hq, lk, cta_k);
-  const int64_t o_b = b <= 1 ? hq * lq * d : o.stride(0);
-  const int64_t o_n = lq <= 1 ? d : o.stride(2);
-  const int64_t o_h = hq <= 1 ? lq * d : o.stride(1);
+  const int64_t o_b = b <= 1 ? hq * lq * od : o.stride(0);
+  const int64_t o_n = lq <= 1 ? od : o.stride(2);
+  const int64_t o_h = hq <= 1 ? lq * od : o.stride(1);
   auto i32 = [](const std::optional<at::Tensor>& t) {
     return t.has_value() ? static_cast<const int32_t*>(t->data_ptr()) : nullptr;
   };
@@ -245,6 +251,28 @@ void attend_tensors(const at::Tensor& q_int8, const at::Tensor& k_int8, const at
     const size_t bytes =
         risa_b200_attention_scratch_size(int(b), int(hq), int(lq), int(lk), int(d), cta_k);
     if (bytes > 0) scratch = at::empty({int64_t(bytes)}, q_int8.options().dtype(at::kByte));
+  }
+  if (lse_shift != nullptr || fp32_cols > 0) {
+    risa_b200_operands shape{};
+    shape.batch = int(b);
+    shape.q_heads = int(hq);
+    shape.kv_heads = int(hkv);
+    shape.q_len = int(lq);
+    shape.k_len = int(lk);
+    shape.head_dim = int(d);
+    shape.cta_k = cta_k;
+    const risa_b200_packed packed{q_int8.data_ptr(), k_int8.data_ptr(), v_int8.data_ptr(),
+                                  q_scale.data_ptr<float>(), k_scale.data_ptr<float>(),
+                                  v_scale.data_ptr<float>(), v_center.data_ptr<float>(), nullptr,
+                                  nullptr, 0};
+    const risa_b200_attention_out out{o.data_ptr(), {o_b, o_h, o_n}, output_dtype_code, fp32_cols,
+                                      lse.has_value() ? lse->data_ptr<float>() : nullptr, lse_shift};
+    check(risa_b200_attend(&shape, &packed, &out, sm_scale, is_causal ? 1 : 0, mask_ptr, ms, mask_code,
+                           i32(key_mask_tiles), i32(row_offsets), i32(block_indices),
+                           scratch.has_value() ? scratch->data_ptr() : nullptr,
+                           scratch.has_value() ? size_t(scratch->numel()) : 0,
+                           stream_of(stream_ptr)));
+    return;
   }
   check(risa_b200_attention_scratch(
       q_int8.data_ptr(), k_int8.data_ptr(), v_int8.data_ptr(), o.data_ptr(),
@@ -484,6 +512,188 @@ py::tuple allocate_packed(const at::Tensor& q, const at::Tensor& k, int cta_k) {
                 q.options().dtype(at::kByte)));
 }
 
+// ---- whole calls: every allocation and launch of a public call from one foreign call -----------
+// Short calls are bounded by the host: an FP32 call with LSE at 1024 keys spent 110 us in Python
+// between its launches (buffers, quantisation, LSE shift, attention, FP32 copy, LSE sum), 68 us back
+// to back.
+using MaybeTensor = std::optional<at::Tensor>;
+
+struct Inputs {
+  at::Tensor q, k, v;  // what the quantisers read (padded copies only where they cannot pad)
+  risa_b200_operands operands;
+};
+
+Inputs operands_of(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
+                   const MaybeTensor& kv_table, int cta_k, int head_dim, bool affine) {
+  const int64_t in_dim = q.size(3), esize = q.element_size();
+  // channels up to the kernel's head dim are read as zeros when rows are aligned for vector loads
+  auto aligned = [&](const at::Tensor& t, int64_t bytes) {
+    if (reinterpret_cast<uintptr_t>(t.data_ptr()) % bytes != 0) return false;
+    for (int i = 0; i < 3; ++i)
+      if (t.size(i) > 1 && (t.stride(i) <= 0 || t.stride(i) * esize % bytes != 0)) return false;
+    return true;
+  };
+  const bool narrow = in_dim < head_dim && in_dim % 4 == 0 && aligned(q, 4 * esize) &&
+                      aligned(k, 4 * esize) && aligned(v, 16);
+  auto padded = [&](const at::Tensor& t) {
+    return in_dim < head_dim && !narrow ? at::constant_pad_nd(t, {0, head_dim - in_dim}) : t;
+  };
+  Inputs in{padded(q), padded(k), padded(v), {}};
+  risa_b200_operands& o = in.operands;
+  o.q = in.q.data_ptr();
+  o.k = in.k.data_ptr();
+  o.v = in.v.data_ptr();
+  for (int i = 0; i < 3; ++i) {
+    o.q_strides[i] = in.q.stride(i);
+    o.k_strides[i] = in.k.stride(i);
+    o.v_strides[i] = in.v.stride(i);
+  }
+  o.batch = int(q.size(0));
+  o.q_heads = int(q.size(1));
+  o.q_len = int(q.size(2));
+  o.kv_heads = int(k.size(1));
+  o.k_len = int(k.size(2));
+  o.head_dim = head_dim;
+  o.in_dim = int(in.q.size(3));
+  o.cta_k = cta_k;
+  o.dtype_code = dtype_code(q);
+  o.midpoint_affine = affine ? 1 : 0;
+  o.kv_perm = kv_table.has_value() ? kv_table->data_ptr<int32_t>() : nullptr;
+  return in;
+}
+
+MaybeTensor key_tiles_of(const MaybeTensor& mask, bool wanted, int cta_k, uintptr_t stream_ptr) {
+  if (!wanted) return std::nullopt;
+  const at::Tensor& m = *mask;
+  at::Tensor tiles = at::empty({m.size(0), m.size(1), (m.size(3) + cta_k - 1) / cta_k + 1},
+                               m.options().dtype(at::kInt));
+  check(risa_b200_prepare_key_mask_tiles(m.data_ptr(), tiles.data_ptr<int32_t>(), int(m.size(0)),
+                                         int(m.size(1)), int(m.size(3)), cta_k, m.stride(0),
+                                         m.stride(1), m.stride(3), dtype_code(m),
+                                         stream_of(stream_ptr)));
+  return tiles;
+}
+
+// Output of a call: FP32 callers get FP32 rows of their own width straight from the kernel where it
+// can write them, everybody else rows of the kernel's width of which they see theirs.
+struct Output {
+  at::Tensor storage;  // what the kernel writes
+  int dtype_code, fp32_cols;
+  at::Tensor result(int64_t dim, bool fp32) const {
+    const at::Tensor seen = storage.size(3) == dim ? storage : storage.narrow(3, 0, dim);
+    return fp32 && dtype_code != 0 ? seen.to(at::kFloat) : seen;
+  }
+};
+
+Output output_for(const at::TensorOptions& options, int input_code, int64_t b, int64_t hq,
+                  int64_t lq, int64_t head_dim, int64_t dim, bool finishes, bool nhd) {
+  const bool fp32 = input_code == 0 && finishes && dim % 4 == 0;
+  const at::ScalarType type = fp32 ? at::kFloat : input_code == 1 ? at::kHalf : at::kBFloat16;
+  const int64_t cols = fp32 ? dim : head_dim;
+  at::Tensor o = nhd ? at::empty({b, lq, hq, cols}, options.dtype(type)).permute({0, 2, 1, 3})
+                     : at::empty({b, hq, lq, cols}, options.dtype(type));
+  return {o, fp32 ? 0 : input_code == 1 ? 1 : 2, fp32 ? int(dim) : 0};
+}
+
+// int8_attention of validated arguments (`mask` expanded to [B,Hq,Lq,Lk]); returns (out, lse or None).
+py::tuple attention_call(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
+                         const MaybeTensor& mask, const MaybeTensor& kv_table, int cta_k,
+                         int head_dim, bool affine, float sm_scale, bool is_causal,
+                         bool key_tiles, bool return_lse, uintptr_t stream_ptr) {
+  const c10::DeviceGuard on_device(q.device());
+  const Inputs in = operands_of(q, k, v, kv_table, cta_k, head_dim, affine);
+  const risa_b200_operands& shape = in.operands;
+  const int64_t b = shape.batch, hq = shape.q_heads, lq = shape.q_len, dim = q.size(3);
+  const bool finishes = risa_b200_finishes_outputs(head_dim, cta_k, shape.k_len) != 0;
+  const Output out = output_for(q.options(), shape.dtype_code, b, hq, lq, head_dim, dim, finishes, false);
+  const size_t bytes = risa_b200_packed_layout(&shape, nullptr, nullptr, nullptr, nullptr);
+  const at::Tensor scratch = at::empty({int64_t(bytes)}, q.options().dtype(at::kByte));
+  risa_b200_packed packed;
+  void* tail = nullptr;
+  size_t tail_bytes = 0;
+  risa_b200_packed_layout(&shape, static_cast<char*>(scratch.data_ptr()), &packed, &tail, &tail_bytes);
+  MaybeTensor lse, shift;
+  if (return_lse) {
+    lse = at::empty({b, hq, lq}, q.options().dtype(at::kFloat));
+    shift = at::empty_like(*lse);
+  }
+  const MaybeTensor tiles = key_tiles_of(mask, key_tiles, cta_k, stream_ptr);
+  check(risa_b200_quantize_operands(&shape, &packed, sm_scale,
+                                    return_lse ? shift->data_ptr<float>() : nullptr,
+                                    stream_of(stream_ptr)));
+  int64_t ms[4] = {0, 0, 0, 0};
+  if (mask.has_value())
+    for (int i = 0; i < 4; ++i) ms[i] = mask->stride(i);
+  const at::Tensor& o = out.storage;
+  const risa_b200_attention_out target{
+      o.data_ptr(), {o.stride(0), o.stride(1), o.stride(2)}, out.dtype_code, out.fp32_cols,
+      return_lse ? lse->data_ptr<float>() : nullptr,
+      return_lse && finishes ? shift->data_ptr<float>() : nullptr};
+  check(risa_b200_attend(&shape, &packed, &target, sm_scale, is_causal ? 1 : 0,
+                         mask.has_value() ? mask->data_ptr() : nullptr, ms,
+                         mask.has_value() ? dtype_code(*mask) : -1,
+                         tiles.has_value() ? tiles->data_ptr<int32_t>() : nullptr, nullptr, nullptr,
+                         tail, tail_bytes, stream_of(stream_ptr)));
+  if (return_lse && !finishes) lse->add_(*shift);
+  return py::make_tuple(out.result(dim, shape.dtype_code == 0), lse);
+}
+
+// prequantize_int8_attention of validated arguments: the packed buffers (as allocate_packed hands
+// them out, without the scratch) and the LSE shift or None.
+py::tuple quantize_call(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
+                        const MaybeTensor& kv_table, int cta_k, int head_dim, bool affine,
+                        float sm_scale, bool want_shift, uintptr_t stream_ptr) {
+  const c10::DeviceGuard on_device(q.device());
+  const Inputs in = operands_of(q, k, v, kv_table, cta_k, head_dim, affine);
+  const risa_b200_operands& s = in.operands;
+  const int64_t b = s.batch, hq = s.q_heads, hkv = s.kv_heads, lq = s.q_len, lk = s.k_len;
+  const int64_t d = head_dim, padded = (lk + cta_k - 1) / cta_k * cta_k;
+  const auto bytes = q.options().dtype(at::kChar), floats = q.options().dtype(at::kFloat);
+  const at::Tensor qc = at::empty({b, hq, lq, d}, bytes), kc = at::empty({b, hkv, lk, d}, bytes),
+                   qs = at::empty({b, hq, (lq + 127) / 128 * (d == 256 ? 64 : 32)}, floats),
+                   ks = at::empty({b, hkv, padded / cta_k * 4}, floats),
+                   vc = at::empty({b * hkv * d, padded}, bytes), vs = at::empty({b * hkv * d}, floats),
+                   centers = at::empty({b * hkv * d}, floats),
+                   anchors = at::empty({b, hkv}, q.options().dtype(at::kInt)),
+                   work = at::empty({int64_t(risa_b200_quantize_v_workspace_size(
+                                        int(b), int(hkv), int(lk), int(d)))},
+                                    q.options().dtype(at::kByte));
+  MaybeTensor shift;
+  if (want_shift) shift = at::empty({b, hq, lq}, floats);
+  const risa_b200_packed packed{qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), qs.data_ptr<float>(),
+                                ks.data_ptr<float>(), vs.data_ptr<float>(),
+                                centers.data_ptr<float>(), anchors.data_ptr<int32_t>(),
+                                work.data_ptr(), size_t(work.numel())};
+  check(risa_b200_quantize_operands(&s, &packed, sm_scale,
+                                    want_shift ? shift->data_ptr<float>() : nullptr,
+                                    stream_of(stream_ptr)));
+  return py::make_tuple(qc, kc, vc, qs, ks, vs, centers, shift);
+}
+
+// int8_attention_from_prequantized of validated arguments (no capture); returns (out, lse or None).
+py::tuple attend_call(const at::Tensor& qc, const at::Tensor& kc, const at::Tensor& vc,
+                      const at::Tensor& qs, const at::Tensor& ks, const at::Tensor& vs,
+                      const at::Tensor& centers, int cta_k, float sm_scale, int input_code,
+                      int64_t dim, const MaybeTensor& mask, const MaybeTensor& row_offsets,
+                      const MaybeTensor& block_indices, bool is_causal, bool key_tiles,
+                      const MaybeTensor& lse_shift, bool nhd, uintptr_t stream_ptr) {
+  const c10::DeviceGuard on_device(qc.device());
+  const int64_t b = qc.size(0), hq = qc.size(1), lq = qc.size(2), d = qc.size(3);
+  const bool finishes = risa_b200_finishes_outputs(int(d), cta_k, int(kc.size(2))) != 0;
+  const Output out = output_for(qc.options(), input_code, b, hq, lq, d, dim, finishes, nhd);
+  MaybeTensor lse;
+  if (lse_shift.has_value()) lse = at::empty({b, hq, lq}, qc.options().dtype(at::kFloat));
+  const bool add_here = lse.has_value() && !(finishes && lse_shift->is_contiguous() &&
+                                             lse_shift->scalar_type() == at::kFloat &&
+                                             lse_shift->sizes() == lse->sizes());
+  attend_tensors(qc, kc, vc, out.storage, qs, ks, vs, centers, cta_k, sm_scale, out.dtype_code,
+                 stream_ptr, mask, row_offsets, block_indices, std::nullopt, is_causal, lse,
+                 key_tiles_of(mask, key_tiles, cta_k, stream_ptr),
+                 lse.has_value() && !add_here ? lse_shift->data_ptr<float>() : nullptr, out.fp32_cols);
+  if (add_here) lse->add_(*lse_shift);
+  return py::make_tuple(out.result(dim, input_code == 0), lse);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_C, m) {
@@ -522,6 +732,9 @@ PYBIND11_MODULE(_C, m) {
   m.def("dense_scratch_size", &dense_scratch_size);
   m.def("risa_dense_attention", &risa_dense_attention);
   m.def("quantize_v_workspace_size", &quantize_v_workspace_size);
+  m.def("attention_call", &attention_call);
+  m.def("quantize_call", &quantize_call);
+  m.def("attend_call", &attend_call);
   m.def("allocate_packed", &allocate_packed, py::arg("q"), py::arg("k"), py::arg("cta_k"));
   m.def("select_scratch_size",
         [](int k_len, int cta_k) { return risa_b200_select_scratch_size(k_len, cta_k); });

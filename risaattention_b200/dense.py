@@ -5,8 +5,7 @@ from __future__ import annotations
 
 import torch
 
-from ._execution import execute_dense_attention, int8_attention_from_prequantized
-from ._quantization import prequantize_int8_attention
+from ._execution import execute_dense_attention, execute_permuted_or_lse_attention
 from ._validation import uses_centered_values
 
 
@@ -62,11 +61,10 @@ def int8_attention(q, k, v, *, scale=None, attn_mask=None, v_quantization="absma
     residual-corrected centre).  Scores, maxima, exponentials, denominators and V dequantisation
     are FP32; the denominator uses the same rounded U8 probabilities as P*V."""
     if return_lse or kv_permutation is not None:
-        packed = prequantize_int8_attention(
+        return execute_permuted_or_lse_attention(
             q, k, v, scale=scale, attn_mask=attn_mask, v_quantization=v_quantization,
             is_causal=is_causal, return_lse=return_lse, kv_permutation=kv_permutation,
             fuse_gather=fuse_gather)
-        return int8_attention_from_prequantized(packed, return_lse=return_lse)
     affine = uses_centered_values(v_quantization)
     if not torch.compiler.is_compiling() and type(q) is torch.Tensor:
         # eager call on plain tensors: same implementation as the registered operators, without
