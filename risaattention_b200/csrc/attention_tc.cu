@@ -221,6 +221,8 @@ __device__ __forceinline__ void softmax_tile_int(uint32_t tmem_row, const float 
   // Pass 1 lands two 32-column chunks per wait (nothing else is live yet, so 64 landing registers
   // are free); pass 2 walks the chunks backwards so that it starts on chunk 3, which is still in
   // registers, and every later chunk is fetched underneath the previous chunk's exponentials.
+  // (A 64-key tile stays in registers altogether.)
+  constexpr bool RESIDENT = CTA_K == 64;
   uint32_t raw_a[32], raw[32];
   // max_floor: where the lane maxima start; the last visited tile starts them at -50000 (the
   // reference's generic arithmetic), every other tile below any score
@@ -266,11 +268,14 @@ __device__ __forceinline__ void softmax_tile_int(uint32_t tmem_row, const float 
   // the next chunk's load to overlap the exponentials.
 #pragma unroll kExpUnroll
   for (int c = CTA_K / 32 - 1; c >= 0; --c) {
-    tmem_load_wait();
-    tmem_regs_ready<32>(raw);
+    if constexpr (!RESIDENT) {
+      tmem_load_wait();
+      tmem_regs_ready<32>(raw);
+    }
     float x[32];
 #pragma unroll
-    for (int i = 0; i < 32; ++i) x[i] = static_cast<float>(int(raw[i]));
+    for (int i = 0; i < 32; ++i)
+      x[i] = static_cast<float>(int(RESIDENT && c == 0 ? raw_a[i] : raw[i]));
     if constexpr (KIND == kScoresScaled) {
 #pragma unroll
       // one rounding for the product, a second one when the maximum is subtracted (the reference's
@@ -283,7 +288,7 @@ __device__ __forceinline__ void softmax_tile_int(uint32_t tmem_row, const float 
       for (int i = 0; i < 32; ++i)
         if (((keep[c] >> i) & 1u) == 0u) x[i] = -INFINITY;
     }
-    if (c > 0) tmem_load32(tmem_row + 32 * (c - 1), raw);
+    if (!RESIDENT && c > 0) tmem_load32(tmem_row + 32 * (c - 1), raw);
     uint32_t P[8], s4[8];
     tile_exp_chunk<KIND, CAPTURE, 32, true>(x, sc, neg_m, P, numer, s4, mul);
     if constexpr (CAPTURE) {
@@ -291,6 +296,46 @@ __device__ __forceinline__ void softmax_tile_int(uint32_t tmem_row, const float 
       for (int i = 0; i < 8; i += 2)
         *reinterpret_cast<uint32_t*>(sums + 8 * c + i) = s4[i] | (s4[i + 1] << 16);
     }
+    *reinterpret_cast<uint4*>(p_row + (((2 * c) ^ swz) << 4)) = make_uint4(P[0], P[1], P[2], P[3]);
+    *reinterpret_cast<uint4*>(p_row + (((2 * c + 1) ^ swz) << 4)) =
+        make_uint4(P[4], P[5], P[6], P[7]);
+  }
+  *stat = make_float2(tile_m, __uint_as_float(numer));
+}
+
+// A 64-key tile in the pre-scaled arithmetic with the whole row in registers: the scores are loaded
+// once, converted and scaled in place, changed by `adjust(x, first column)` 32 at a time (mask bits, a
+// bias), and the maxima and exponents are taken from the same registers.  One conversion and one
+// select per score where maxima on integers and a second pass from tensor memory need two of each.
+// The values are those of the general path on the same tile (the scaled maximum is the maximum of the
+// scaled scores), so the bits are too.
+template <typename Adjust>
+__device__ __forceinline__ void softmax_tile_floats64(uint32_t tmem_row, const float (&sc)[4],
+                                                      unsigned char* p_row, int swz, float2* stat,
+                                                      PackMultipliers mul, Adjust&& adjust) {
+  uint32_t raw[64];
+  tmem_load32(tmem_row, raw);
+  tmem_load32(tmem_row + 32, raw + 32);
+  tmem_load_wait();
+  tmem_regs_ready<64>(raw);
+  float x[64];
+  float top[4] = {-50000.0f, -50000.0f, -50000.0f, -50000.0f};
+#pragma unroll
+  for (int c = 0; c < 64; c += 32) {
+#pragma unroll
+    for (int i = c; i < c + 32; ++i)
+      x[i] = __fmul_rn(static_cast<float>(int(raw[i])), sc[(i & 7) >> 1]);
+    adjust(x + c, c);
+#pragma unroll
+    for (int i = c; i < c + 32; i += 2)
+      top[(i >> 1) & 3] = fmaxf(top[(i >> 1) & 3], fmaxf(x[i], x[i + 1]));
+  }
+  const float tile_m = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) - kU8Offset;
+  uint32_t numer = 0;
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    uint32_t P[8], s4[8];
+    tile_exp_chunk<kScoresScaled, false, 32, true>(x + 32 * c, sc, -tile_m, P, numer, s4, mul);
     *reinterpret_cast<uint4*>(p_row + (((2 * c) ^ swz) << 4)) = make_uint4(P[0], P[1], P[2], P[3]);
     *reinterpret_cast<uint4*>(p_row + (((2 * c + 1) ^ swz) << 4)) =
         make_uint4(P[4], P[5], P[6], P[7]);
@@ -609,7 +654,9 @@ __device__ __forceinline__ void softmax_tile_general(const AttentionArgs& a, int
 // folds and output rows.  Attention alone, before -> after: causal 4096 at head_dim 64 (32 heads) 176
 // -> 137 us, 8192 keys at head_dim 128 426 -> 405, 2048 keys 40.4 -> 37.6, 480 heads of 333 x 333 94
 // -> 75.  Capture and selection use the idle rings after their last tile and keep a CTA per unit.
-template <int MODE, int CTA_K, int D, int VARIANT = 0>
+// SPLIT: some units are key-range parts of a (query block, head) pair (an instantiation of its own:
+// the part's bookkeeping costs the tile loop registers, 75 -> 88 us in the last of the cases above).
+template <int MODE, int CTA_K, int D, int VARIANT = 0, bool SPLIT = false>
 __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, const AttentionArgs a) {
@@ -625,9 +672,9 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
                  PLAIN = VARIANT == 2 || WHOLE, CAUSAL = VARIANT == 3,
                  KEYBITS = VARIANT == 7,
                  MASKED = VARIANT == 4, KEYMASK = VARIANT == 5;
-  constexpr bool kHasInt = VARIANT == 0 || PLAIN, kHasScaled = VARIANT == 0 || CAUSAL,
+  constexpr bool kHasInt = VARIANT == 0 || PLAIN, kHasScaled = VARIANT == 0 || (CAUSAL && CTA_K != 64),
                  kHasMasked = VARIANT == 0 || BOOLROWS || MASKED || KEYMASK,
-                 kHasUnmasked = VARIANT == 0 || VARIANT == 2 || CAUSAL;
+                 kHasUnmasked = VARIANT == 0 || VARIANT == 2 || (CAUSAL && CTA_K != 64);
   using L = SmemLayout<D, CTA_K, MODE>;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
@@ -655,7 +702,7 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
   auto place = [&] {
     if constexpr (PERSIST) {
       int pair = unit;
-      if (PLAIN || VARIANT == 0) {  // the calls whose last wave may be split
+      if constexpr (SPLIT) {
         parts = 1;
         if (unit >= a.tail_begin) {
           tail_unit = (unit - a.tail_begin) / a.tail_splits;
@@ -1031,12 +1078,31 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
             keep[c] = __ballot_sync(0xffffffffu, key_bytes[c] != 0);
             all &= keep[c];
           }
-          if (all == 0xffffffffu)
+          if constexpr (CTA_K == 64)
+            softmax_tile_floats64(tmem_row, sc, p_row, swz, stat, pack_mul, [&](float* x, int c0) {
+              if (all == 0xffffffffu) return;
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                if (((keep[c0 / 32] >> i) & 1u) == 0u) x[i] = -INFINITY;
+            });
+          else if (all == 0xffffffffu)
             softmax_tile_int<CAPTURE, CTA_K, kScoresScaled>(tmem_row, sc, p_row, swz, stat,
                                                             my_sums, pack_mul);
           else
             softmax_tile_int<CAPTURE, CTA_K, kScoresScaled, true, true>(
                 tmem_row, sc, p_row, swz, stat, my_sums, pack_mul, INT_MIN, keep);
+        }
+      } else if (CAUSAL && CTA_K == 64) {
+        if constexpr (CAUSAL && CTA_K == 64) {
+          // one path for every tile; on the diagonal and at a ragged end the keys this row sees count
+          const int seen = min(row + 1, a.k_len) - tile * CTA_K;
+          const bool whole = below_diagonal && (tile + 1) * CTA_K <= a.k_len;
+          softmax_tile_floats64(tmem_row, sc, p_row, swz, stat, pack_mul, [&](float* x, int c0) {
+            if (whole) return;
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (c0 + i >= seen) x[i] = -INFINITY;
+          });
         }
       } else if (kHasScaled && below_diagonal && !last)
         softmax_tile_int<CAPTURE, CTA_K, kScoresScaled>(tmem_row, sc, p_row, swz, stat,
@@ -1048,8 +1114,11 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
             mask_prefetch_runs(a, batch, head, row, tile * CTA_K + kMaskRunKeys);
           uint32_t keep[2];
           mask_row_bits64(mask_bytes, keep);  // rows past the end hold zeros: nothing visible
-          softmax_tile_int<CAPTURE, CTA_K, kScoresScaled, true>(
-              tmem_row, sc, p_row, swz, stat, my_sums, pack_mul, INT_MIN, keep);
+          softmax_tile_floats64(tmem_row, sc, p_row, swz, stat, pack_mul, [&](float* x, int c0) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (((keep[c0 / 32] >> i) & 1u) == 0u) x[i] = -INFINITY;
+          });
         }
       } else if (kHasMasked && (!kHasUnmasked || a.mask != nullptr))
         softmax_tile_general<CAPTURE, CTA_K, true, KEYMASK>(a, batch, head, row_ok, tmem_row, sc,
@@ -1297,7 +1366,7 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       }
     }
     const float denom = st.d[0];
-    if (MODE == kDense && parts > 1) {
+    if (SPLIT && parts > 1) {
       // part of a split key range: channel-major unnormalised rows (in units of 2^m_o), then m_o
       // and the denominator; NaN when a wait of this CTA expired, so the merged rows show it
       float* mine = a.tail_scratch + (size_t(tail_unit) * parts + part) * (130 * 128) + row_in;
@@ -1332,43 +1401,6 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       uint4* staged = reinterpret_cast<uint4*>(smem + L::out_stage) + (warp & 3) * 32 * L::kOutPitch;
 #pragma unroll
       for (int c0 = 0; c0 < kOut; c0 += 64) {
-        if (MODE == kDense && a.out_dtype_code == 0) {
-          // FP32 callers: the bf16 value of each element stored as FP32, 32 channels at a time
-#pragma unroll
-          for (int c1 = c0; c1 < c0 + 64; c1 += 32) {
-#pragma unroll
-            for (int ch = c1; ch < c1 + 32; ch += 4) {
-              const ulonglong2 scale4 = *reinterpret_cast<const ulonglong2*>(vs + ch);
-              const ulonglong2 centre4 = *reinterpret_cast<const ulonglong2*>(vc + ch);
-              uint32_t word[4];
-#pragma unroll
-              for (int i = 0; i < 2; ++i) {
-                float r0, r1;
-                unpack_f32x2(fma_f32x2(mul_f32x2(O2[(ch >> 1) + i], inv2), i ? scale4.y : scale4.x,
-                                       i ? centre4.y : centre4.x), r0, r1);
-                const __nv_bfloat162 h = __floats2bfloat162_rn(r0, r1);
-                uint32_t both = *reinterpret_cast<const uint32_t*>(&h);
-                if (!PLAIN) both = zero ? 0u : both;
-                word[2 * i] = both << 16;
-                word[2 * i + 1] = both & 0xffff0000u;
-              }
-              staged[lane * L::kOutPitch + (ch - c1) / 4] =
-                  make_uint4(word[0], word[1], word[2], word[3]);
-            }
-            __syncwarp();
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int r = 4 * i + lane / 8, col = kOut * half + c1 + 4 * (lane % 8);
-              const uint4 piece = staged[r * L::kOutPitch + lane % 8];
-              if (row - lane + r < a.q_len && col < a.out_cols)
-                *reinterpret_cast<uint4*>(static_cast<float*>(a.o) + batch * a.o_stride_b +
-                                          head * a.o_stride_h +
-                                          int64_t(row - lane + r) * a.o_stride_n + col) = piece;
-            }
-            __syncwarp();
-          }
-          continue;
-        }
         // the element type is the same for the whole launch: one branch per 64 channels
         auto finish = [&](auto to_half) {
 #pragma unroll
@@ -1404,12 +1436,30 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
         if (a.out_dtype_code == 1) finish(std::true_type{});
         else finish(std::false_type{});
         __syncwarp();
+        if (MODE != kDense || a.out_dtype_code != 0) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int r = 4 * i + lane / 8;
-          const uint4 piece = staged[r * L::kOutPitch + lane % 8];
-          if (row - lane + r < a.q_len)
-            *reinterpret_cast<uint4*>(o_block + 2 * r * a.o_stride_n + 2 * c0 + 16 * (lane % 8)) = piece;
+          for (int i = 0; i < 8; ++i) {
+            const int r = 4 * i + lane / 8;
+            const uint4 piece = staged[r * L::kOutPitch + lane % 8];
+            if (row - lane + r < a.q_len)
+              *reinterpret_cast<uint4*>(o_block + 2 * r * a.o_stride_n + 2 * c0 + 16 * (lane % 8)) =
+                  piece;
+          }
+        } else {
+          // FP32 callers: the bf16 values stored as FP32 (rolled: this is not the common case)
+          const int col = kOut * half + c0 + 8 * (lane % 8);
+          float* o_rows = static_cast<float*>(a.o) + batch * a.o_stride_b + head * a.o_stride_h + col;
+#pragma unroll 1
+          for (int r = lane / 8; r < 32 && row - lane + r < a.q_len; r += 4) {
+            const uint4 piece = staged[r * L::kOutPitch + lane % 8];
+            uint4* to = reinterpret_cast<uint4*>(o_rows + int64_t(row - lane + r) * a.o_stride_n);
+            if (col < a.out_cols)
+              to[0] = make_uint4(piece.x << 16, piece.x & 0xffff0000u, piece.y << 16,
+                                 piece.y & 0xffff0000u);
+            if (col + 4 < a.out_cols)
+              to[1] = make_uint4(piece.z << 16, piece.z & 0xffff0000u, piece.w << 16,
+                                 piece.w & 0xffff0000u);
+          }
         }
         __syncwarp();
       }
@@ -1806,10 +1856,10 @@ int sms_of_device(int device) {
   return sms;
 }
 
-template <int MODE, int CTA_K, int D, int VARIANT = 0>
+template <int MODE, int CTA_K, int D, int VARIANT = 0, bool SPLIT = false>
 int launch_tc(const AttentionArgs& a, const CUtensorMap& map_q, const CUtensorMap& map_k,
               const CUtensorMap& map_v, cudaStream_t stream) {
-  auto kernel = attention_tc_kernel<MODE, CTA_K, D, VARIANT>;
+  auto kernel = attention_tc_kernel<MODE, CTA_K, D, VARIANT, SPLIT>;
   static thread_local int configured = -1;  // per instantiation, thread and device
   int device = -1;
   cudaGetDevice(&device);
@@ -1836,22 +1886,26 @@ int launch_tc(const AttentionArgs& a, const CUtensorMap& map_q, const CUtensorMa
   const dim3 grid((a.q_len + 127) / 128, a.q_heads * SmemLayout<D, CTA_K, MODE>::kHalves, a.batch);
   if constexpr (MODE == kDense) {
     // resident CTAs, one per SM, over all units; the rest of the last round may be split into parts
-    const int sms = sms_of_device(device), n_k = (a.k_len + CTA_K - 1) / CTA_K;
-    const int ctas = int(grid.x * grid.y * grid.z), parts = tail_split_factor(a, ctas, n_k, sms);
+    const int sms = sms_of_device(device), ctas = int(grid.x * grid.y * grid.z);
     AttentionArgs all = a;
     all.tail_begin = all.units = ctas;
-    all.tail_splits = 0;
-    const int rest = parts > 0 ? ctas % sms : 0;
-    if (parts > 0) {
+    if constexpr (SPLIT) {
+      const int rest = ctas % sms;
       all.tail_begin = ctas - rest;
-      all.tail_splits = parts;
-      all.units = all.tail_begin + rest * parts;
+      all.units = all.tail_begin + rest * a.tail_splits;
+    } else if constexpr (VARIANT == 0 || VARIANT == 2 || VARIANT == 6) {
+      const int parts = tail_split_factor(a, ctas, (a.k_len + CTA_K - 1) / CTA_K, sms);
+      if (parts > 0) {
+        all.tail_splits = parts;
+        return launch_tc<MODE, CTA_K, D, VARIANT, true>(all, map_q, map_k, map_v, stream);
+      }
     }
     launch_chained(kernel, dim3(std::min(all.units, sms)), dim3(kThreads),
                    SmemLayout<D, CTA_K, MODE>::bytes, stream, map_q, map_k, map_v, all);
-    if (parts > 0)
-      launch_chained(tail_merge_kernel, dim3(rest, SmemLayout<D, CTA_K, MODE>::kOut / kMergeChannels),
-                     dim3(128), 0, stream, all, SmemLayout<D, CTA_K, MODE>::kHalves,
+    if constexpr (SPLIT)
+      launch_chained(tail_merge_kernel,
+                     dim3(ctas % sms, SmemLayout<D, CTA_K, MODE>::kOut / kMergeChannels), dim3(128), 0,
+                     stream, all, SmemLayout<D, CTA_K, MODE>::kHalves,
                      SmemLayout<D, CTA_K, MODE>::kOut);
   } else {
     launch_chained(kernel, grid, dim3(kThreads), SmemLayout<D, CTA_K, MODE>::bytes, stream, map_q,
