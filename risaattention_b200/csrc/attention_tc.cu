@@ -78,28 +78,41 @@ constexpr unsigned int kSelfTestSite = 900;  // site number reported by the boun
 // for with shallower rings.  Kernels with 64-key tiles (per-query masks, short sequences,
 // head_dim 64) have smaller K stages and spend the difference on a per-warp staging area through
 // which mask values are loaded with coalesced accesses and handed to the row-owning threads.
-template <int D, int CTA_K, int MODE>
+// MASK (mask_ring()): the kernels whose per-query masks come by TMA hold a ring of mask tiles instead of
+// the staging area: 128 rows of 64 entries, 1 = boolean (8 KB), 2 = FP32 (two boxes of 32 entries,
+// 32 KB), 3 = 16-bit (16 KB).
+constexpr int mask_ring(int variant) { return variant == 1 ? 1 : variant == 8 ? 2 : variant == 9 ? 3 : 0; }
+
+template <int D, int CTA_K, int MODE, int MASK = 0>
 struct SmemLayout {
   static constexpr int kOut = D == 256 ? 128 : D;          // output channels per CTA
   static constexpr int kHalves = D == 256 ? 2 : 1;         // CTAs per (query block, head)
   static constexpr int kPanels = D == 256 ? 2 : 1;         // column panels of a Q / K tile
   static constexpr int kPanelBytes = D == 64 ? 64 : 128;   // bytes per row of a panel
   static constexpr int kKSt = D == 256 ? 2 : kKStages;     // K ring depth
-  static constexpr int kVSt = D == 256 ? 2 : D == 64 ? 6 : 3;  // V ring depth
+  static constexpr int kVSt = D == 256 || (D == 128 && MASK == 2) ? 2
+                                  : D == 64 && MASK != 2 ? 6 : 3;  // V ring depth
   // Tensor memory: accumulator buffers as wide as the wider of the scores and the output, so 64-key
   // tiles at head_dim 64 have eight of 64 columns, everything else four of 128.
   static constexpr int kBuffers = D == 64 ? 8 : 4;
   static constexpr int kBufferCols = 512 / kBuffers;
-  static constexpr int kSlots = D == 256 ? 3 : kBuffers;   // P tiles and per-row statistics
+  static constexpr int kSlots = D == 256 ? 3 : MASK == 2 ? 4 : kBuffers;  // P tiles and per-row statistics
   static constexpr int kQBytes = kPanels * 128 * kPanelBytes;  // the Q tile
-  static constexpr int kQStages = MODE == kDense && D != 256 ? 2 : 1;  // Q tiles held at once
+  static constexpr int kQStages =
+      MODE == kDense && D != 256 && !(D == 128 && MASK == 2) ? 2 : 1;  // Q tiles held at once
   static constexpr int kKPanel = CTA_K * kPanelBytes;      // one column panel of a K stage
   static constexpr int kVStage = kOut * 128;               // one V stage
   static constexpr int kPTile = 128 * CTA_K;               // one P tile: rows of CTA_K bytes
   static constexpr int kKStage = kPanels * kKPanel;        // one K stage
   static constexpr int kMaskStageWords = 32 * 33;          // 32 x 32 values, rows padded to 33
+  // One mask stage per softmax group: the tile that reuses a stage then belongs to the group that has
+  // read the stage's previous tile.  With fewer, a group could test a stage's barrier for a phase
+  // whose predecessor is still to come, and a parity test cannot tell those apart.
+  static constexpr int kMaskStages = MASK == 0 ? 0 : kSoftmaxGroups;
+  static constexpr int kMaskTile = MASK == 1 ? 8192 : MASK == 2 ? 32768 : 16384;
   static constexpr int kMaskStageBytes =
-      CTA_K == 64 ? kSoftmaxGroups * 4 * kMaskStageWords * 4 : 0;  // one area per softmax warp
+      MASK != 0 ? kMaskStages * kMaskTile
+      : CTA_K == 64 ? kSoftmaxGroups * 4 * kMaskStageWords * 4 : 0;  // one area per softmax warp
   static constexpr int q = 0;
   static constexpr int k = q + kQStages * kQBytes;
   static constexpr int v = k + kKSt * kKStage;
@@ -110,14 +123,15 @@ struct SmemLayout {
       MODE == kDense ? 0 : (kSlots < 4 ? 4 : kSlots) * 128 * (CTA_K / 2);
   static constexpr int mask_stage = sums + sums_bytes;
   static constexpr int rowstate = mask_stage + kMaskStageBytes;  // float [5][128]: m, d[4] (capture)
-  static constexpr int v_affine = rowstate + 5 * 128 * 4;  // float [2][128]: V scales, V centres
+  // float [2][128]: V scales, V centres
+  static constexpr int v_affine = rowstate + (MODE == kDense ? 0 : 5 * 128 * 4);
   // Output rows on their way out: per warp 32 rows of 64 channels (128 bytes, rows 144 bytes apart).
   // Capture and selection write their rows when the K / V rings are idle and stage them there.
   static constexpr int kOutPitch = 9;                      // 16-byte pieces
   static constexpr int out_stage = MODE == kDense ? v_affine + 2 * 128 * 4 : k;
   static constexpr int bars = v_affine + 2 * 128 * 4 +
                               (MODE == kDense ? 4 * 32 * kOutPitch * 16 : 0);  // 8-byte mbarriers
-  static constexpr int n_bars = 1 + 2 * kKStages + 2 * kVStages + 6 * kMaxBuffers + 2 + 3;
+  static constexpr int n_bars = 1 + 2 * kKStages + 2 * kVStages + 6 * kMaxBuffers + 2 + 3 + 6;
   static constexpr int tmem_slot = bars + n_bars * 8;
   static constexpr int gave_up = tmem_slot + 8;            // site of the first expired wait, or 0
   static constexpr int total = tmem_slot + 16;
@@ -129,6 +143,15 @@ constexpr bool layouts_fit() {
          SmemLayout<256, 64, MODE>::bytes <= 232448 && SmemLayout<128, 64, MODE>::bytes <= 232448 &&
          SmemLayout<64, 64, MODE>::bytes <= 232448;
 }
+static_assert(SmemLayout<64, 64, kDense, 1>::bytes <= 232448 &&
+                  SmemLayout<128, 64, kDense, 1>::bytes <= 232448 &&
+                  SmemLayout<256, 64, kDense, 1>::bytes <= 232448 &&
+                  SmemLayout<64, 64, kDense, 2>::bytes <= 232448 &&
+                  SmemLayout<128, 64, kDense, 2>::bytes <= 232448 &&
+                  SmemLayout<64, 64, kDense, 3>::bytes <= 232448 &&
+                  SmemLayout<128, 64, kDense, 3>::bytes <= 232448 &&
+                  SmemLayout<256, 64, kDense, 3>::bytes <= 232448,
+              "shared memory per CTA with a mask ring");
 static_assert(layouts_fit<kDense>() && layouts_fit<kCapture>() && layouts_fit<kSelect>(),
               "shared memory per CTA");
 
@@ -184,7 +207,8 @@ struct Bars {
                        BUFFREE = SFULL + kMaxBuffers, PFULL = BUFFREE + kMaxBuffers,
                        SLOTFREE = PFULL + kMaxBuffers, OFULL = SLOTFREE + kMaxBuffers,
                        WFULL = OFULL + kMaxBuffers,
-                       PAIRS = WFULL + kMaxBuffers;  // two: the selection epilogue's bulk copies
+                       MFULL = WFULL + kMaxBuffers, MEMPTY = MFULL + kSoftmaxGroups,
+                       PAIRS = MEMPTY + kSoftmaxGroups;  // two: the selection epilogue's bulk copies
   // Tensor memory is four accumulator buffers of 128 columns; tile it owns buffer it % 4 for its
   // whole life: Q.K^T writes the scores there (SFULL), the softmax group reads them, P.V then
   // overwrites the same columns with the tile's integer output (OFULL) and the correction group
@@ -303,13 +327,22 @@ __device__ __forceinline__ void softmax_tile_int(uint32_t tmem_row, const float 
   *stat = make_float2(tile_m, __uint_as_float(numer));
 }
 
+// The larger of two, NaN if either is NaN (the hardware's NaN is positive: 0x7fffffff).
+__device__ __forceinline__ float fmax_nan(float a, float b) {
+  float r;
+  asm("max.NaN.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
 // A 64-key tile in the pre-scaled arithmetic with the whole row in registers: the scores are loaded
 // once, converted and scaled in place, changed by `adjust(x, first column)` 32 at a time (mask bits, a
 // bias), and the maxima and exponents are taken from the same registers.  One conversion and one
 // select per score where maxima on integers and a second pass from tensor memory need two of each.
 // The values are those of the general path on the same tile (the scaled maximum is the maximum of the
 // scaled scores), so the bits are too.
-template <typename Adjust>
+// UNCHECKED: scores may have become +inf or NaN (a non-finite bias hides its key, whatever its sign);
+// the maxima let both through, and only then are the scores gone over.
+template <bool UNCHECKED, typename Adjust>
 __device__ __forceinline__ void softmax_tile_floats64(uint32_t tmem_row, const float (&sc)[4],
                                                       unsigned char* p_row, int swz, float2* stat,
                                                       PackMultipliers mul, Adjust&& adjust) {
@@ -328,9 +361,21 @@ __device__ __forceinline__ void softmax_tile_floats64(uint32_t tmem_row, const f
     adjust(x + c, c);
 #pragma unroll
     for (int i = c; i < c + 32; i += 2)
-      top[(i >> 1) & 3] = fmaxf(top[(i >> 1) & 3], fmaxf(x[i], x[i + 1]));
+      top[(i >> 1) & 3] = UNCHECKED ? fmax_nan(top[(i >> 1) & 3], fmax_nan(x[i], x[i + 1]))
+                                    : fmaxf(top[(i >> 1) & 3], fmaxf(x[i], x[i + 1]));
   }
-  const float tile_m = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) - kU8Offset;
+  float highest = UNCHECKED ? fmax_nan(fmax_nan(top[0], top[1]), fmax_nan(top[2], top[3]))
+                            : fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
+  if (UNCHECKED && !(__float_as_uint(highest) < 0x7f800000u || __float_as_uint(highest) >= 0x80000000u)) {
+    highest = -50000.0f;
+#pragma unroll
+    for (int i = 0; i < 64; ++i) {
+      const uint32_t bits = __float_as_uint(x[i]);  // +inf, or NaN of either sign
+      if (bits - 0x7f800000u < 0x80000000u - 0x7f800000u || bits > 0xff800000u) x[i] = -INFINITY;
+      highest = fmaxf(highest, x[i]);
+    }
+  }
+  const float tile_m = highest - kU8Offset;
   uint32_t numer = 0;
 #pragma unroll
   for (int c = 0; c < 2; ++c) {
@@ -481,14 +526,8 @@ __device__ __forceinline__ void mask_block_rows(const AttentionArgs& a, int batc
   __syncwarp();
 }
 
-// 64 consecutive entries of one row of a boolean mask (16-byte aligned) as 64 bits: bit i of
-// keep[c] = entry 32 c + i is non-zero.  Four 16-byte loads by the thread that owns the row (issued
-// before the thread waits for the tile's scores, so that their latency passes during that wait);
-// a word of four bytes, each made 0 / 1, times 0x01020408 leaves its four bits in the top nibble.
-__device__ __forceinline__ void mask_row_load64(const unsigned char* entries, uint4 (&v)[4]) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j) v[j] = __ldg(reinterpret_cast<const uint4*>(entries) + j);
-}
+// 64 entries of one row of a boolean mask as 64 bits: bit i of keep[c] = entry 32 c + i is non-zero.
+// A word of four bytes, each made 0 / 1, times 0x01020408 leaves its four bits in the top nibble.
 __device__ __forceinline__ void mask_row_bits64(const uint4 (&v)[4], uint32_t (&keep)[2]) {
 #pragma unroll
   for (int c = 0; c < 2; ++c) {
@@ -659,7 +698,8 @@ __device__ __forceinline__ void softmax_tile_general(const AttentionArgs& a, int
 template <int MODE, int CTA_K, int D, int VARIANT = 0, bool SPLIT = false>
 __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-    const __grid_constant__ CUtensorMap map_v, const AttentionArgs a) {
+    const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_mask,
+    const AttentionArgs a) {
   constexpr bool CAPTURE = MODE != kDense;  // exact per-tile statistics and denominators
   constexpr bool PERSIST = !CAPTURE;
   // Which softmax paths an instantiation holds (the host picks the instantiation, launch_tc):
@@ -667,15 +707,16 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
   // 3 causal without mask, positive scale; 4 any other per-query mask; 5 masks broadcast over the
   // queries (their entries are read as 16-byte pieces shared by all rows); 6 as 2 with a key length
   // that is a whole number of tiles (no ragged last tile: the integer fast path alone); 7 boolean
-  // masks broadcast over the queries, their keys as bits.
+  // masks broadcast over the queries, their keys as bits; 8 FP32 and 9 16-bit per-query masks whose
+  // tiles TMA can fetch.
   constexpr bool BOOLROWS = VARIANT == 1, WHOLE = VARIANT == 6,
                  PLAIN = VARIANT == 2 || WHOLE, CAUSAL = VARIANT == 3,
-                 KEYBITS = VARIANT == 7,
+                 KEYBITS = VARIANT == 7, BIASTILES = VARIANT == 8 || VARIANT == 9,
                  MASKED = VARIANT == 4, KEYMASK = VARIANT == 5;
   constexpr bool kHasInt = VARIANT == 0 || PLAIN, kHasScaled = VARIANT == 0 || (CAUSAL && CTA_K != 64),
-                 kHasMasked = VARIANT == 0 || BOOLROWS || MASKED || KEYMASK,
+                 kHasMasked = VARIANT == 0 || MASKED || KEYMASK,
                  kHasUnmasked = VARIANT == 0 || VARIANT == 2 || (CAUSAL && CTA_K != 64);
-  using L = SmemLayout<D, CTA_K, MODE>;
+  using L = SmemLayout<D, CTA_K, MODE, mask_ring(VARIANT)>;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -753,6 +794,10 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
     }
     if constexpr (MODE == kSelect)
       for (int i = 0; i < 2; ++i) mbar_init(bar(Bars::PAIRS + i), 1);
+    for (int i = 0; i < L::kMaskStages; ++i) {
+      mbar_init(bar(Bars::MFULL + i), 1);
+      mbar_init(bar(Bars::MEMPTY + i), 4);
+    }
     mbar_init_fence();
   }
   if (warp == kIssueWarp + 1) tmem_alloc(sbase + L::tmem_slot, 512);
@@ -840,14 +885,42 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       }
     } else if (warp == kIssueWarp + 3) {
       // ---------------------------------------------------------------- producer: V
-      if (elect_one()) tma_prefetch_descriptor(&map_v);
+      // (and mask tiles, which the softmax needs two tiles before P.V needs V)
+      constexpr int kLead = L::kMaskStages > 0 ? 2 : 0;
+      if (elect_one()) {
+        tma_prefetch_descriptor(&map_v);
+        if constexpr (L::kMaskStages > 0) tma_prefetch_descriptor(&map_mask);
+      }
       RingPos<L::kVSt> vs;
-      int v_loads = 0;
+      RingPos<kSoftmaxGroups> ms;
+      int v_loads = 0, mask_loads = 0;
       bool ok = true;
       do {
         const int n_iter = uniform(seq.n_iter), row_v = uniform(L::kOut * half),
                   slab_v = uniform(int(kvh));
-        for (int it = 0; it < n_iter; ++it) {
+        for (int step = 0; step < n_iter + kLead; ++step) {
+          if constexpr (L::kMaskStages > 0) {
+            if (step < n_iter) {
+              ok = mbar_wait<true>(bar(Bars::MEMPTY + ms.stage), ms.phase ^ 1, gave_up, 104);
+              if (!__all_sync(0xffffffffu, ok)) break;
+              constexpr int kEntry = VARIANT == 1 ? 1 : VARIANT == 8 ? 4 : 2;  // bytes
+              const int at = seq.tile(step) * CTA_K * kEntry, row_m = uniform(bx * 128);
+              const int head_m = uniform(a.mask_stride_h != 0 ? head : 0);
+              const int batch_m = uniform(a.mask_stride_b != 0 ? batch : 0);
+              if (elect_one()) {
+                mbar_expect_tx(bar(Bars::MFULL + ms.stage), L::kMaskTile);
+#pragma unroll
+                for (int box = 0; box < (VARIANT == 8 ? 2 : 1); ++box)
+                  tma_load_4d(sbase + L::mask_stage + ms.stage * L::kMaskTile + box * 16384, &map_mask,
+                              bar(Bars::MFULL + ms.stage), at + 128 * box, row_m, head_m, batch_m);
+              }
+              __syncwarp();
+              ++mask_loads;
+              ms.next();
+            }
+          }
+          const int it = step - kLead;
+          if (it < 0) continue;
           ok = mbar_wait<true>(bar(Bars::VEMPTY + vs.stage), vs.phase ^ 1, gave_up, 102);
           if (!__all_sync(0xffffffffu, ok)) break;
           // V always arrives as the 128-key slab that holds the tile (64-key tiles use half of it):
@@ -867,6 +940,9 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       if (!__all_sync(0xffffffffu, ok)) {
         for (int j = max(0, v_loads - L::kVSt); j < v_loads; ++j)
           mbar_drain(bar(Bars::VFULL + j % L::kVSt), (j / L::kVSt) & 1);
+        if constexpr (L::kMaskStages > 0)
+          for (int j = max(0, mask_loads - L::kMaskStages); j < mask_loads; ++j)
+            mbar_drain(bar(Bars::MFULL + j % L::kMaskStages), (j / L::kMaskStages) & 1);
       }
     } else if (warp == kIssueWarp + 1) {
       // ---------------------------------------------------------------- MMA issue: S = Q.K^T
@@ -964,10 +1040,6 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
         PLAIN || (kHasInt && !a.is_causal && a.sm_scale > 0.0f && a.mask == nullptr);
     const bool causal_fast =
         CAUSAL || (kHasScaled && a.is_causal && a.sm_scale > 0.0f && a.mask == nullptr);
-    const unsigned char* bool_row = nullptr;  // this row of a boolean per-query mask
-    if constexpr (BOOLROWS)
-      bool_row = static_cast<const unsigned char*>(a.mask) + int64_t(batch) * a.mask_stride_b +
-                 int64_t(head) * a.mask_stride_h + int64_t(row) * a.mask_stride_q;
     const unsigned char* key_row = nullptr;  // the visible keys of a boolean mask without query axis
     if constexpr (KEYBITS)
       key_row = static_cast<const unsigned char*>(a.mask) + int64_t(batch) * a.mask_stride_b +
@@ -1052,9 +1124,10 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
           if (key < a.k_len) key_bytes[c] = __ldg(key_row + key * a.mask_stride_k);
         }
       }
-      uint4 mask_bytes[4] = {};
-      if constexpr (BOOLROWS) {
-        if (!last && row_ok) mask_row_load64(bool_row + tile * CTA_K, mask_bytes);
+      if constexpr (L::kMaskStages > 0) {
+        ok = mbar_wait(bar(Bars::MFULL + ring % kSoftmaxGroups), (ring / kSoftmaxGroups) & 1, gave_up,
+                       304);
+        if (!ok) break;
       }
       ok = mbar_wait2(bar(Bars::SLOTFREE + slot), ((ring / L::kSlots) & 1) ^ 1,
                       bar(Bars::SFULL + sb), u & 1, gave_up, 301);
@@ -1079,7 +1152,7 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
             all &= keep[c];
           }
           if constexpr (CTA_K == 64)
-            softmax_tile_floats64(tmem_row, sc, p_row, swz, stat, pack_mul, [&](float* x, int c0) {
+            softmax_tile_floats64<false>(tmem_row, sc, p_row, swz, stat, pack_mul, [&](float* x, int c0) {
               if (all == 0xffffffffu) return;
 #pragma unroll
               for (int i = 0; i < 32; ++i)
@@ -1097,7 +1170,7 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
           // one path for every tile; on the diagonal and at a ragged end the keys this row sees count
           const int seen = min(row + 1, a.k_len) - tile * CTA_K;
           const bool whole = below_diagonal && (tile + 1) * CTA_K <= a.k_len;
-          softmax_tile_floats64(tmem_row, sc, p_row, swz, stat, pack_mul, [&](float* x, int c0) {
+          softmax_tile_floats64<false>(tmem_row, sc, p_row, swz, stat, pack_mul, [&](float* x, int c0) {
             if (whole) return;
 #pragma unroll
             for (int i = 0; i < 32; ++i)
@@ -1107,17 +1180,69 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       } else if (kHasScaled && below_diagonal && !last)
         softmax_tile_int<CAPTURE, CTA_K, kScoresScaled>(tmem_row, sc, p_row, swz, stat,
                                                         my_sums, pack_mul);
-      else if (BOOLROWS && !last) {
-        // boolean per-query mask, tile wholly inside the key range: the row's 64 entries as bits
+      else if (BOOLROWS) {
+        // boolean per-query mask: the row's 64 entries of the mask tile as bits (entries past the end of
+        // a row or of the mask arrive as zeros: hidden)
         if constexpr (BOOLROWS) {
-          if (tile * CTA_K % kMaskRunKeys == 0)
-            mask_prefetch_runs(a, batch, head, row, tile * CTA_K + kMaskRunKeys);
+          const int stage = ring % kSoftmaxGroups;
+          const uint4* pieces = reinterpret_cast<const uint4*>(smem + L::mask_stage +
+                                                               stage * L::kMaskTile + row_in * 64);
+          uint4 entries[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) entries[j] = pieces[j ^ ((row_in >> 1) & 3)];
           uint32_t keep[2];
-          mask_row_bits64(mask_bytes, keep);  // rows past the end hold zeros: nothing visible
-          softmax_tile_floats64(tmem_row, sc, p_row, swz, stat, pack_mul, [&](float* x, int c0) {
+          mask_row_bits64(entries, keep);
+          mbar_arrive_warp(bar(Bars::MEMPTY + stage));
+          softmax_tile_floats64<false>(tmem_row, sc, p_row, swz, stat, pack_mul,
+                                       [&](float* x, int c0) {
 #pragma unroll
             for (int i = 0; i < 32; ++i)
               if (((keep[c0 / 32] >> i) & 1u) == 0u) x[i] = -INFINITY;
+          });
+        }
+      } else if (BIASTILES) {
+        if constexpr (BIASTILES) {
+          const int stage = ring % kSoftmaxGroups, inside = a.k_len - tile * CTA_K;
+          const unsigned char* mask_row = smem + L::mask_stage + stage * L::kMaskTile + row_in * 128;
+          softmax_tile_floats64<true>(tmem_row, sc, p_row, swz, stat, pack_mul,
+                                      [&](float* x, int c0) {
+            // score * scale and + bias * log2(e) are separate roundings, as in apply_mask; -inf hides
+            // by itself, +inf and NaN are looked for in the maxima
+            if constexpr (VARIANT == 8) {
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                const float4 bias = *reinterpret_cast<const float4*>(
+                    mask_row + (c0 / 32) * 16384 + ((j ^ (row_in & 7)) << 4));
+                x[4 * j] = __fadd_rn(x[4 * j], bias.x * kLog2e);
+                x[4 * j + 1] = __fadd_rn(x[4 * j + 1], bias.y * kLog2e);
+                x[4 * j + 2] = __fadd_rn(x[4 * j + 2], bias.z * kLog2e);
+                x[4 * j + 3] = __fadd_rn(x[4 * j + 3], bias.w * kLog2e);
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const uint4 piece = *reinterpret_cast<const uint4*>(
+                    mask_row + (((c0 / 8 + j) ^ (row_in & 7)) << 4));
+                const uint32_t w[4] = {piece.x, piece.y, piece.z, piece.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                  float lo = __uint_as_float(w[i] << 16), hi = __uint_as_float(w[i] & 0xffff0000u);
+                  if (a.mask_dtype_code == 1) {
+                    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+                    lo = f.x;
+                    hi = f.y;
+                  }
+                  x[8 * j + 2 * i] = __fadd_rn(x[8 * j + 2 * i], lo * kLog2e);
+                  x[8 * j + 2 * i + 1] = __fadd_rn(x[8 * j + 2 * i + 1], hi * kLog2e);
+                }
+              }
+            }
+            if (c0 == 32) mbar_arrive_warp(bar(Bars::MEMPTY + stage));
+            if (inside < CTA_K) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                if (c0 + i >= inside) x[i] = -INFINITY;
+            }
           });
         }
       } else if (kHasMasked && (!kHasUnmasked || a.mask != nullptr))
@@ -1813,16 +1938,40 @@ int tail_split_factor(const AttentionArgs& a, int ctas, int n_k, int sms) {
   return parts;
 }
 
-// Dense calls whose mask is boolean, per query, with contiguous keys and rows that start on 16-byte
-// boundaries (base and every stride a multiple of 16 entries), a positive scale and neither causal
-// rule nor tile lists: the kernel instantiation that reads such rows as bits (64-key tiles only,
-// which per-query masks always have).
+// Dense calls with a per-query mask of contiguous keys whose base and strides are multiples of 16
+// bytes (what a tensor map takes), without the causal rule.
+bool mask_rows_by_tma(const AttentionArgs& a) {
+  const int64_t entry = a.mask_dtype_code == 3 ? 1 : a.mask_dtype_code == 0 ? 4 : 2;
+  return a.cta_k == 64 && a.mask != nullptr && a.mask_stride_k == 1 && a.mask_stride_q > 0 &&
+         a.mask_stride_b >= 0 && a.mask_stride_h >= 0 && !a.is_causal && a.block_mass == nullptr &&
+         a.select_scratch == nullptr &&
+         (reinterpret_cast<uintptr_t>(a.mask) | uintptr_t(a.mask_stride_b * entry) |
+          uintptr_t(a.mask_stride_h * entry) | uintptr_t(a.mask_stride_q * entry)) % 16 == 0;
+}
+
+// Mask as bytes [batch][head][query][entries], axes it is broadcast over with one element; boxes of 128
+// queries x 128 bytes (64 for boolean entries), swizzled by that width.
+bool make_mask_map(CUtensorMap* map, const AttentionArgs& a) {
+  const cuuint64_t entry = a.mask_dtype_code == 3 ? 1 : a.mask_dtype_code == 0 ? 4 : 2;
+  const cuuint64_t row = cuuint64_t(a.mask_stride_q) * entry;
+  const cuuint64_t dims[4] = {cuuint64_t(a.k_len) * entry, cuuint64_t(a.q_len),
+                              cuuint64_t(a.mask_stride_h != 0 ? a.q_heads : 1),
+                              cuuint64_t(a.mask_stride_b != 0 ? a.batch : 1)};
+  const cuuint64_t strides[3] = {row, a.mask_stride_h != 0 ? a.mask_stride_h * entry : row,
+                                 a.mask_stride_b != 0 ? a.mask_stride_b * entry : row};
+  const cuuint32_t box[4] = {entry == 1 ? 64u : 128u, 128, 1, 1};
+  const cuuint32_t elem[4] = {1, 1, 1, 1};
+  return encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void*>(a.mask), dims, strides,
+                     box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     entry == 1 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
+                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Boolean masks among them, with a positive scale and no tile lists: their rows are read as bits.
 bool reads_mask_rows_as_bits(const AttentionArgs& a) {
-  return a.cta_k == 64 && a.mask != nullptr && a.mask_dtype_code == 3 && a.mask_stride_k == 1 &&
-         a.mask_stride_q != 0 && a.sm_scale > 0.0f && !a.is_causal && a.row_offsets == nullptr &&
-         a.key_mask_tiles == nullptr && a.block_mass == nullptr && a.select_scratch == nullptr &&
-         (reinterpret_cast<uintptr_t>(a.mask) | uintptr_t(a.mask_stride_b) |
-          uintptr_t(a.mask_stride_h) | uintptr_t(a.mask_stride_q)) % 16 == 0;
+  return a.mask_dtype_code == 3 && a.sm_scale > 0.0f && a.row_offsets == nullptr &&
+         a.key_mask_tiles == nullptr;
 }
 
 // Dense calls whose mask is boolean and broadcast over the queries, with a positive scale and no
@@ -1858,17 +2007,17 @@ int sms_of_device(int device) {
 
 template <int MODE, int CTA_K, int D, int VARIANT = 0, bool SPLIT = false>
 int launch_tc(const AttentionArgs& a, const CUtensorMap& map_q, const CUtensorMap& map_k,
-              const CUtensorMap& map_v, cudaStream_t stream) {
+              const CUtensorMap& map_v, cudaStream_t stream, const CUtensorMap* map_mask = nullptr) {
   auto kernel = attention_tc_kernel<MODE, CTA_K, D, VARIANT, SPLIT>;
   static thread_local int configured = -1;  // per instantiation, thread and device
   int device = -1;
   cudaGetDevice(&device);
   if (configured != device) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(SmemLayout<D, CTA_K, MODE>::bytes));
+                                         int(SmemLayout<D, CTA_K, MODE, mask_ring(VARIANT)>::bytes));
     if (e != cudaSuccess)
       return fail(RISA_B200_CUDA, "attention: cannot reserve %zu bytes of shared memory: %s",
-                  SmemLayout<D, CTA_K, MODE>::bytes, cudaGetErrorString(e));
+                  SmemLayout<D, CTA_K, MODE, mask_ring(VARIANT)>::bytes, cudaGetErrorString(e));
     // setmaxnreg hands out the registers the CTA is launched with; if the compiler ever gave this
     // kernel fewer than the roles ask for, the increase could never be granted (it blocks, beyond
     // the reach of the bounded waits), so such a build must not run
@@ -1883,7 +2032,7 @@ int launch_tc(const AttentionArgs& a, const CUtensorMap& map_q, const CUtensorMa
                   "need a pool of %d", attr.numRegs, kPool / kThreads);
     configured = device;
   }
-  const dim3 grid((a.q_len + 127) / 128, a.q_heads * SmemLayout<D, CTA_K, MODE>::kHalves, a.batch);
+  const dim3 grid((a.q_len + 127) / 128, a.q_heads * SmemLayout<D, CTA_K, MODE, mask_ring(VARIANT)>::kHalves, a.batch);
   if constexpr (MODE == kDense) {
     // resident CTAs, one per SM, over all units; the rest of the last round may be split into parts
     const int sms = sms_of_device(device), ctas = int(grid.x * grid.y * grid.z);
@@ -1901,15 +2050,16 @@ int launch_tc(const AttentionArgs& a, const CUtensorMap& map_q, const CUtensorMa
       }
     }
     launch_chained(kernel, dim3(std::min(all.units, sms)), dim3(kThreads),
-                   SmemLayout<D, CTA_K, MODE>::bytes, stream, map_q, map_k, map_v, all);
+                   SmemLayout<D, CTA_K, MODE, mask_ring(VARIANT)>::bytes, stream, map_q, map_k, map_v,
+                   map_mask ? *map_mask : map_v, all);
     if constexpr (SPLIT)
       launch_chained(tail_merge_kernel,
-                     dim3(ctas % sms, SmemLayout<D, CTA_K, MODE>::kOut / kMergeChannels), dim3(128), 0,
-                     stream, all, SmemLayout<D, CTA_K, MODE>::kHalves,
-                     SmemLayout<D, CTA_K, MODE>::kOut);
+                     dim3(ctas % sms, SmemLayout<D, CTA_K, MODE, mask_ring(VARIANT)>::kOut / kMergeChannels), dim3(128), 0,
+                     stream, all, SmemLayout<D, CTA_K, MODE, mask_ring(VARIANT)>::kHalves,
+                     SmemLayout<D, CTA_K, MODE, mask_ring(VARIANT)>::kOut);
   } else {
-    launch_chained(kernel, grid, dim3(kThreads), SmemLayout<D, CTA_K, MODE>::bytes, stream, map_q,
-                   map_k, map_v, a);
+    launch_chained(kernel, grid, dim3(kThreads), SmemLayout<D, CTA_K, MODE, mask_ring(VARIANT)>::bytes, stream, map_q,
+                   map_k, map_v, map_v, a);
   }
   return check_launch("attention (tensor-core kernel)");
 }
@@ -1973,8 +2123,21 @@ int attention_tc(const AttentionArgs& args, cudaStream_t stream, bool every_path
       return plain ? launch_tc<kCapture, K, HD, 2>(a, map_q, map_k, map_v, stream)
                    : launch_tc<kCapture, K, HD>(a, map_q, map_k, map_v, stream);
     if constexpr (K == 64) {
-      if (reads_mask_rows_as_bits(a))
-        return launch_tc<kDense, K, HD, 1>(a, map_q, map_k, map_v, stream);
+      // Per-query masks whose rows TMA can fetch.  Attention alone, rows fetched and turned around by
+      // the softmax warps -> tiles by TMA: a 4096 x 4096 FP32 mask for each of 32 heads of 64 channels
+      // 735 -> 363 us (6.0 TB/s of mask), boolean rows of the same shape 421 -> 344.
+      CUtensorMap map_mask;
+      if (mask_rows_by_tma(a) && make_mask_map(&map_mask, a)) {
+        if (reads_mask_rows_as_bits(a))
+          return launch_tc<kDense, K, HD, 1>(a, map_q, map_k, map_v, stream, &map_mask);
+        // (FP32 tiles of head_dim 256 do not fit beside its operands)
+        if constexpr (HD != 256) {
+          if (a.mask_dtype_code == 0)
+            return launch_tc<kDense, K, HD, 8>(a, map_q, map_k, map_v, stream, &map_mask);
+        }
+        if (a.mask_dtype_code == 1 || a.mask_dtype_code == 2)
+          return launch_tc<kDense, K, HD, 9>(a, map_q, map_k, map_v, stream, &map_mask);
+      }
     }
     if (plain) {
       if (a.k_len % K == 0) return launch_tc<kDense, K, HD, 6>(a, map_q, map_k, map_v, stream);

@@ -1,0 +1,95 @@
+"""Calls that one native call carries out as a whole (buffers, quantisation without padded copies, LSE
+shift, FP32 rows) against the same work done in separate steps through the ctypes surface, resident
+CTAs that walk many units, and per-query masks fetched as tiles.  Everything here keeps every operation
+and its order, so bits are compared."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+import risaattention_b200 as risa  # noqa: E402
+from risaattention_b200 import _backend, compare_native  # noqa: E402
+
+
+def _inputs(head_dim, q_len, k_len, dtype, q_heads=4, kv_heads=2, batch=2, token_major=False):
+    g = torch.Generator(device="cuda").manual_seed(head_dim * 10007 + k_len)
+
+    def make(heads, n):
+        x = torch.randn(batch, heads, n, head_dim, device="cuda", generator=g).to(dtype)
+        return x.transpose(1, 2).contiguous().transpose(1, 2) if token_major else x
+
+    return make(q_heads, q_len), make(kv_heads, k_len), make(kv_heads, k_len)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("head_dim,k_len", [(40, 300), (64, 63), (80, 1025), (77, 200), (128, 129),
+                                            (200, 1500), (256, 257)])
+@pytest.mark.parametrize("mode", ["absmax", "midpoint_affine"])
+def test_whole_calls_give_the_bits_of_the_separate_steps(dtype, head_dim, k_len, mode):
+    q, k, v = _inputs(head_dim, 130, k_len, dtype, token_major=k_len % 2 == 0)
+
+    def calls():
+        out, lse = risa.int8_attention(q, k, v, v_quantization=mode, return_lse=True)
+        packed = risa.prequantize_int8_attention(q, k, v, v_quantization=mode, return_lse=True)
+        nhd, lse2 = risa.int8_attention_from_prequantized(packed, output_layout="nhd",
+                                                          return_lse=True)
+        return [risa.int8_attention(q, k, v, v_quantization=mode), out, lse, nhd, lse2, packed.q,
+                packed.k, packed.v, packed.q_scale, packed.k_scale, packed.v_scale,
+                packed.v_center, packed.lse_shift]
+
+    whole = calls()
+    steps = compare_native.with_native(_backend._ABI, calls)
+    for ours, want in zip(whole, steps):
+        assert ours.dtype == want.dtype and ours.shape == want.shape
+        assert ours.stride() == want.stride() and torch.equal(ours, want)
+    _backend._C.device_status()
+
+
+@pytest.mark.parametrize("is_causal", [False, True])
+@pytest.mark.parametrize("head_dim,q_len,k_len", [(64, 700, 333), (128, 700, 320), (128, 300, 1500),
+                                                  (256, 500, 129)])
+def test_resident_ctas_over_many_units(head_dim, q_len, k_len, is_causal):
+    """More (query block, head) units than SMs: each head alone -- a launch whose CTAs have one unit
+    each -- gives the same rows.  (No shape here is one whose last round is cut into parts.)"""
+    q, k, v = _inputs(head_dim, q_len, k_len, torch.bfloat16, q_heads=40, kv_heads=20, batch=3)
+    out = risa.int8_attention(q, k, v, is_causal=is_causal)
+    for b, h in ((0, 0), (1, 17), (2, 39), (2, 24)):
+        alone = risa.int8_attention(q[b:b + 1, h:h + 1], k[b:b + 1, h // 2:h // 2 + 1],
+                                    v[b:b + 1, h // 2:h // 2 + 1], is_causal=is_causal)
+        assert torch.equal(alone[0, 0], out[b, h])
+    _backend._C.device_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.bool, torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("head_dim,k_len,heads", [(64, 1000, 4), (64, 64, 4), (128, 1025, 4),
+                                                  (256, 700, 4), (64, 200, 48), (128, 260, 48),
+                                                  (256, 130, 48)])
+@pytest.mark.parametrize("shared_heads", [False, True])
+def test_mask_tiles_give_the_bits_of_the_all_paths_kernel(dtype, head_dim, k_len, heads, shared_heads):
+    """Masks that are windows of wider rows (aligned rows of any length), with entries that hide: false,
+    -inf, and the +inf and NaN that an additive mask also hides by; few units and several per CTA."""
+    q, k, v = _inputs(head_dim, 300, k_len, torch.bfloat16, q_heads=heads)
+    g = torch.Generator(device="cuda").manual_seed(k_len)
+    wide = torch.randn(2, 1 if shared_heads else heads, 300, (k_len + 127) // 64 * 64, device="cuda",
+                       generator=g)
+    if dtype is torch.bool:
+        wide = wide > -1
+    else:
+        wide = wide.to(dtype)
+        wide[..., 7::13] = float("-inf")
+        wide[..., 5, 9] = float("inf")
+        wide[..., 6, 11] = float("nan")
+    wide[..., 130, :] = False if dtype is torch.bool else float("-inf")
+    mask = wide[..., :k_len]
+    results = []
+    for path in (0, 2):
+        previous = _backend._C.set_attention_path(path)
+        try:
+            results.append(risa.int8_attention(q, k, v, attn_mask=mask, return_lse=True))
+        finally:
+            _backend._C.set_attention_path(previous)
+    (own, own_lse), (every, every_lse) = results
+    assert torch.equal(own, every)
+    assert torch.equal(own_lse.view(torch.int32), every_lse.view(torch.int32))
+    assert own[:, :, 130].count_nonzero() == 0
+    _backend._C.device_status()
