@@ -3,7 +3,7 @@
 // TMA into 128-byte-swizzled shared memory; the FP32 online softmax, the per-tile FP32 rescale of
 // the output and the epilogue run on ordinary warps that read the accumulators with tcgen05.ld.
 //
-// One CTA = 128 queries of one (batch, head); key tiles of 64 or 128 and head_dim 64 or 128 are
+// One unit = 128 queries of one (batch, head); key tiles of 64 or 128 and head_dim 64 or 128 are
 // template parameters (the description below uses 128 / 128).  Five warpgroups:
 //   WG0-WG2    softmax of tiles it % 3 == 0 / 1 / 2.  Thread r owns query row r (tensor-memory lane
 //              r) and makes two passes over the tile's 128 scores: maxima on the raw integers, then
@@ -13,19 +13,23 @@
 //   WG3        correction.  Thread r owns the FP32 output row r in registers (as packed FP32 pairs)
 //              and everything that is sequential over tiles: running maximum, denominator, per-tile
 //              weights, O = O * o_scale + float(P.V) * w, capture statistics, epilogue and store.
-//   WG4        warp 16: TMA producer (Q, K ring, V ring); warp 17: issues the QK^T MMAs, up to four
-//              tiles ahead of the read-back; warp 18: issues the P.V MMAs.  Both walk their loop as
-//              whole converged warps and elect one lane for the MMAs.
-// Tensor memory (512 columns) is four accumulator buffers of 128 columns.  Tile it owns buffer
-// it % 4 from its Q.K^T until its P.V result has been read back: the scores are written there, the
-// softmax group reads them, P.V overwrites the same columns and the correction group takes the
-// result into registers.  Probabilities are scaled to the tile maximum (full 8-bit resolution in
-// every tile), so each tile's integer P.V has its own weight and is folded into FP32 by the
-// correction group; nothing accumulates across tiles inside tensor memory.
+//   WG4        warp 16: TMA producer of Q and K; warp 17: issues the QK^T MMAs, as many tiles ahead
+//              of the read-back as there are accumulator buffers; warp 18: issues the P.V MMAs;
+//              warp 19: TMA producer of V and of mask tiles.  All walk their loop as whole converged
+//              warps and elect one lane for what a single thread issues.
+// Tensor memory (512 columns) is four accumulator buffers of 128 columns, or eight of 64 at head_dim
+// 64.  Tile it owns buffer it % kBuffers from its Q.K^T until its P.V result has been read back: the
+// scores are written there, the softmax group reads them, P.V overwrites the same columns and the
+// correction group takes the result into registers.  Probabilities are scaled to the tile maximum
+// (full 8-bit resolution in every tile), so each tile's integer P.V has its own weight and is folded
+// into FP32 by the correction group; nothing accumulates across tiles inside tensor memory.
 // Numerics: reference csrc/kernels/attention_int8.cuh:427-1026 via softmax_row.cuh.  The integer
 // products are exact, so probabilities, capture statistics and block masses are bit-identical to
 // the row-per-thread kernel; without capture the denominator is kept in one partial instead of four.
-// Dense unmasked launches may cut the CTAs of their last, partial wave into key-range parts (see
+// Dense launches are resident: one CTA per SM walks (query block, head) units, the rings and the
+// accumulator buffers running on across units, so the next unit's loads, MMAs and softmax overlap the
+// previous unit's epilogue.  Capture and selection launch one CTA per unit.
+// Dense unmasked launches may cut the units of their last, partial wave into key-range parts (see
 // split_parts below): a part runs the same loop over its share of the key tiles and leaves its
 // unnormalised rows, maximum and denominator in scratch for tail_merge_kernel.
 // Every mbarrier wait is bounded (tc_ptx.cuh): when one expires the CTA's waiters leave, the producer
@@ -209,14 +213,14 @@ struct Bars {
                        WFULL = OFULL + kMaxBuffers,
                        MFULL = WFULL + kMaxBuffers, MEMPTY = MFULL + kSoftmaxGroups,
                        PAIRS = MEMPTY + kSoftmaxGroups;  // two: the selection epilogue's bulk copies
-  // Tensor memory is four accumulator buffers of 128 columns; tile it owns buffer it % 4 for its
-  // whole life: Q.K^T writes the scores there (SFULL), the softmax group reads them, P.V then
-  // overwrites the same columns with the tile's integer output (OFULL) and the correction group
-  // hands the buffer back once it has it in registers (BUFFREE).  Three tiles can be in the
-  // softmax stage while a fourth is in P.V / read-back, so no stage waits for another tile's
-  // accumulator.  The probability tiles and the per-row statistics have four slots
-  // (it % L::kSlots), handed back together (SLOTFREE) by the correction group when it has read the
-  // statistics: it does that after P.V of the tile has completed, so the probabilities are free too.
+  // Tile it owns accumulator buffer it % kBuffers of tensor memory for its whole life: Q.K^T writes the
+  // scores there (SFULL), the softmax group reads them, P.V then overwrites the same columns with the
+  // tile's integer output (OFULL) and the correction group hands the buffer back once it has it in
+  // registers (BUFFREE).  Three tiles can be in the softmax stage while a fourth is in P.V /
+  // read-back, so no stage waits for another tile's accumulator.  The probability tiles and the
+  // per-row statistics have kSlots slots (it % L::kSlots), handed back together (SLOTFREE) by the
+  // correction group when it has read the statistics: it does that after P.V of the tile has
+  // completed, so the probabilities are free too.
   // Where a warpgroup hands something over its warps arrive once each (mbar_arrive_warp): 4 arrivals
   // on the barrier's word instead of 128.
   // Measured with the uniform issue warps below, dense 32K (B1 Hq16 Hkv4 D128): 6.50 -> 6.39 ms of
