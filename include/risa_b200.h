@@ -157,7 +157,8 @@ int risa_b200_attention_scratch(const void* q, const void* k, const void* v, voi
  * total mass (doubles); block_masses (optional, may be NULL) = f32 [rows, n_k].
  * risa_b200_pack_selected then turns counts + bitmaps into CSR row offsets and ascending tile ids
  * and writes summary = {kept mass, total mass, kept tiles} (stages 2-3 of the reference selector,
- * sparse_selection.cu:69-127).  Limits: tensor-core kernel shapes only, n_k <=
+ * sparse_selection.cu:69-127); summary may be pinned host memory, so that a caller reads it after a
+ * stream synchronisation without a copy.  Limits: tensor-core kernel shapes only, n_k <=
  * risa_b200_select_max_key_tiles(cta_k); scratch 256-byte aligned, at least
  * risa_b200_select_scratch_size() bytes; its slot flags are cleared on `stream` by the call. */
 size_t risa_b200_select_scratch_size(int k_len, int cta_k);

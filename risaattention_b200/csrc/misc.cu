@@ -152,13 +152,18 @@ __global__ __launch_bounds__(32 * kSelectRowsPerCta) void close_prefix_kernel(
 }
 
 // Stage 2, single CTA: exclusive scan of the row counts (integer, order-free) and the FP64 summary,
-// whose 256 strided partials and halving tree follow reference sparse_selection.cu:69-101.
+// whose 256 strided partials and halving tree follow reference sparse_selection.cu:69-101.  One CTA's
+// latency is what the host waits for in a pattern construction: the 256 slice counts are scanned by
+// shuffles (by one thread the scan alone was 3 of the kernel's 4.3 us at 1024 rows), and this kernel
+// and the next are chained to the attention kernel, so their launches pass while it drains.
 __global__ __launch_bounds__(256) void offsets_and_summary_kernel(
     const int32_t* __restrict__ counts, const double* __restrict__ row_totals,
     int32_t* __restrict__ row_offsets, double* __restrict__ summary, uint32_t row_count) {
   __shared__ double s_sel[256], s_tot[256];
-  __shared__ int32_t s_scan[256];
-  const uint32_t tid = threadIdx.x;
+  __shared__ int32_t s_scan[8];
+  chain_wait();
+  chain_release();
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double selected = 0.0, total = 0.0;
   for (uint32_t row = tid; row < row_count; row += 256) {
     selected += row_totals[row * 2];
@@ -171,8 +176,25 @@ __global__ __launch_bounds__(256) void offsets_and_summary_kernel(
   const uint32_t begin = min(row_count, tid * per), end = min(row_count, begin + per);
   int32_t local = 0;
   for (uint32_t r = begin; r < end; ++r) local += counts[r];
-  s_scan[tid] = local;
+  int32_t upto = local;  // counts of the warp's slices up to and with this one
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int32_t before = __shfl_up_sync(0xffffffffu, upto, off);
+    if (lane >= uint32_t(off)) upto += before;
+  }
+  if (lane == 31) s_scan[warp] = upto;
   __syncthreads();
+  int32_t running = upto - local;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) running += uint32_t(w) < warp ? s_scan[w] : 0;
+  if (tid == 255) {
+    row_offsets[row_count] = running + local;
+    summary[2] = static_cast<double>(running + local);
+  }
+  for (uint32_t r = begin; r < end; ++r) {
+    row_offsets[r] = running;
+    running += counts[r];
+  }
   for (uint32_t stride = 128; stride > 0; stride >>= 1) {
     if (tid < stride) {
       s_sel[tid] += s_sel[tid + stride];
@@ -181,22 +203,8 @@ __global__ __launch_bounds__(256) void offsets_and_summary_kernel(
     __syncthreads();
   }
   if (tid == 0) {
-    int32_t running = 0;
-    for (int i = 0; i < 256; ++i) {
-      const int32_t c = s_scan[i];
-      s_scan[i] = running;
-      running += c;
-    }
-    row_offsets[row_count] = running;
     summary[0] = s_sel[0];
     summary[1] = s_tot[0];
-    summary[2] = static_cast<double>(running);
-  }
-  __syncthreads();
-  int32_t running = s_scan[tid];
-  for (uint32_t r = begin; r < end; ++r) {
-    row_offsets[r] = running;
-    running += counts[r];
   }
 }
 
@@ -210,6 +218,7 @@ __global__ __launch_bounds__(256) void expand_bitmaps_kernel(const uint8_t* __re
                                                              uint64_t stride_bytes) {
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t row = blockIdx.x * 8 + warp;
+  chain_wait();
   if (row >= row_count) return;
   const uint32_t* bits = reinterpret_cast<const uint32_t*>(support + uint64_t(row) * stride_bytes);
   int32_t* out = block_indices + row_offsets[row];
@@ -306,11 +315,11 @@ extern "C" int risa_b200_select_retained_mass(const float* sorted_mass, const in
                         32 * kSelectRowsPerCta, 0, stream>>>(
       sorted_mass, order, counts, bitmaps, row_totals, uint32_t(row_count), uint32_t(key_blocks),
       theta);
-  offsets_and_summary_kernel<<<1, 256, 0, stream>>>(counts, row_totals, row_offsets, summary,
-                                                    uint32_t(row_count));
-  expand_bitmaps_kernel<<<(row_count + 7) / 8, 256, 0, stream>>>(
-      bitmaps, row_offsets, block_indices, uint32_t(row_count), uint32_t(key_blocks),
-      uint64_t(words) * 4);
+  launch_chained(offsets_and_summary_kernel, dim3(1), dim3(256), 0, stream, counts, row_totals,
+                 row_offsets, summary, uint32_t(row_count));
+  launch_chained(expand_bitmaps_kernel, dim3((row_count + 7) / 8), dim3(256), 0, stream, bitmaps,
+                 row_offsets, block_indices, uint32_t(row_count), uint32_t(key_blocks),
+                 uint64_t(words) * 4);
   return check_launch("select_retained_mass");
 }
 
@@ -322,10 +331,11 @@ extern "C" int risa_b200_pack_selected(const int32_t* counts, const uint32_t* bi
                "pack_selected: null tensor");
   RISA_REQUIRE(row_count > 0 && key_blocks > 0, "pack_selected: empty problem");
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-  offsets_and_summary_kernel<<<1, 256, 0, stream>>>(counts, row_totals, row_offsets, summary,
-                                                    uint32_t(row_count));
-  expand_bitmaps_kernel<<<(row_count + 7) / 8, 256, 0, stream>>>(
-      reinterpret_cast<const uint8_t*>(bitmaps), row_offsets, block_indices, uint32_t(row_count),
-      uint32_t(key_blocks), uint64_t(bitmap_words(uint32_t(key_blocks))) * 4);
+  launch_chained(offsets_and_summary_kernel, dim3(1), dim3(256), 0, stream, counts, row_totals,
+                 row_offsets, summary, uint32_t(row_count));
+  launch_chained(expand_bitmaps_kernel, dim3((row_count + 7) / 8), dim3(256), 0, stream,
+                 reinterpret_cast<const uint8_t*>(bitmaps), row_offsets, block_indices,
+                 uint32_t(row_count), uint32_t(key_blocks),
+                 uint64_t(bitmap_words(uint32_t(key_blocks))) * 4);
   return check_launch("pack_selected");
 }

@@ -67,8 +67,10 @@ def _construct_in_pass(quantized, theta, output_layout, rows, k_blocks):
         attn_mask=quantized.attn_mask, is_causal=quantized.is_causal)
     row_offsets = torch.empty(rows + 1, dtype=torch.int32, device=device)
     storage = torch.empty(rows * k_blocks, dtype=torch.int32, device=device)
-    summary = torch.empty(3, dtype=torch.float64, device=device)
+    # the kernel writes the summary to pinned host memory: no copy between its end and the read
+    summary = torch.empty(3, dtype=torch.float64, pin_memory=True)
     native.pack_selected(counts, bitmaps, totals, row_offsets, storage, summary, k_blocks, stream)
+    torch.cuda.current_stream(device).synchronize()
     selected_mass, total_mass, selected_blocks = summary.tolist()
     return (finish_output(output, quantized), row_offsets, storage[: int(selected_blocks)],
             selected_mass / max(total_mass, 1e-20))

@@ -93,3 +93,28 @@ def test_mask_tiles_give_the_bits_of_the_all_paths_kernel(dtype, head_dim, k_len
     assert torch.equal(own_lse.view(torch.int32), every_lse.view(torch.int32))
     assert own[:, :, 130].count_nonzero() == 0
     _backend._C.device_status()
+
+
+@pytest.mark.parametrize("rows", [1, 31, 32, 33, 255, 256, 257, 1024, 5000])
+@pytest.mark.parametrize("key_blocks", [1, 33, 70])
+def test_pack_selected_offsets_and_ids(rows, key_blocks):
+    """Offsets, ids and summary of counts whose slices end in every position of the scan."""
+    g = torch.Generator().manual_seed(rows)
+    kept = torch.rand(rows, key_blocks, generator=g) < 0.4
+    words = (key_blocks + 31) // 32
+    weights = 2 ** torch.arange(32, dtype=torch.int64)
+    bits = torch.nn.functional.pad(kept, (0, words * 32 - key_blocks)).view(rows, words, 32)
+    bitmaps = (bits.long() * weights).sum(-1)
+    bitmaps = torch.where(bitmaps >= 2**31, bitmaps - 2**32, bitmaps).int().cuda()
+    counts = kept.sum(-1).int().cuda()
+    totals = torch.ones(rows, 2, dtype=torch.float64, device="cuda")  # sums of ones are exact
+    offsets = torch.full((rows + 1,), -1, dtype=torch.int32, device="cuda")
+    ids = torch.full((rows * key_blocks,), -1, dtype=torch.int32, device="cuda")
+    summary = torch.zeros(3, dtype=torch.float64, pin_memory=True)
+    _backend._C.pack_selected(counts, bitmaps, totals, offsets, ids, summary, key_blocks,
+                              _backend.current_stream_ptr(counts.device))
+    torch.cuda.synchronize()
+    total = int(kept.sum())
+    assert offsets.tolist() == [0] + kept.sum(-1).cumsum(0).tolist()
+    assert torch.equal(ids[:total].cpu(), kept.nonzero()[:, 1].int())
+    assert (ids[total:] == -1).all() and summary.tolist() == [rows, rows, total]
