@@ -91,6 +91,7 @@ __device__ __forceinline__ int storage_position(int token) {
 // lanes of a group with two shuffle steps, after which a lane holds the whole 16-byte storage group
 // of one channel; neighbouring groups of a channel leave in the same store.  No shared memory and no
 // barrier per window, and key lengths need not be multiples of anything: missing tokens give code 0.
+// Rows are whole 16-token storage groups, not whole windows: each group's store has its own bound.
 //   absmax: a CTA walks `steps` pieces of 128 tokens x 64 channels, up to four in flight per lane.
 //   midpoint-affine: the residuals have an order of their own (slot t of `slots` sums tokens Lk-1-t,
 //   Lk-1-t-slots, ...), so a lane keeps four residue classes of tokens modulo `slots` -- a class is
@@ -271,7 +272,7 @@ __device__ __forceinline__ void v_codes_block(const VCodesJob& job, int part, in
 #pragma unroll
         for (int c = 0; c < 4; ++c) words[c] = pack4_s8(x[0][c], x[1][c], x[2][c], x[3][c]);
         transpose_words(words, lane);
-        if (base0 + kVPiece * u < end)
+        if (base0 + kVPiece * u + 16 * group < end)
           *reinterpret_cast<uint4*>(out + base0 + kVPiece * u) =
               make_uint4(words[0], words[1], words[2], words[3]);
       }
@@ -309,7 +310,7 @@ __device__ __forceinline__ void v_codes_block(const VCodesJob& job, int part, in
         words[c] = __byte_perm(__byte_perm(code[0][c], code[1][c], 0x0040),
                                __byte_perm(code[2][c], code[3][c], 0x0040), 0x5410);
       transpose_words(words, lane);
-      if (base < padded_len)
+      if (base + 16 * group < padded_len)
         *reinterpret_cast<uint4*>(out + base) = make_uint4(words[0], words[1], words[2], words[3]);
     }
 #pragma unroll

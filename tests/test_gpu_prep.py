@@ -192,6 +192,44 @@ def test_quantize_v_c_abi_head_dims_outside_the_kernel_set(ref, dim, lk, affine)
     assert int(guard.sum()) == 0
 
 
+@pytest.mark.parametrize("entry", ["quantize_v", "quantize_v_static"])
+@pytest.mark.parametrize("dim", [64, 128, 256])
+@pytest.mark.parametrize("lk,padded", [(9, 16), (48, 48), (41, 80), (260, 272), (500, 784),
+                                       (1040, 1040)])
+@pytest.mark.parametrize("affine", [False, True])
+def test_quantize_v_rows_of_an_odd_number_of_storage_groups(entry, dim, lk, padded, affine):
+    """The C-ABI takes rows of any whole number of 16-token groups (the Python runtime pads to 64 or
+    128).  The codes lie inside a larger buffer of sentinels, so that a store past a row is seen in the
+    next row and one past the last row in the sentinels; they are those of the runtime's longer rows."""
+    import ctypes
+
+    import risaattention_b200 as risa
+    from risaattention_b200 import _backend
+
+    b, hkv = 2, 3
+    g = torch.Generator(device="cuda").manual_seed(dim + lk)
+    v = (torch.randn(b, hkv, lk, dim, device="cuda", generator=g) + 0.7).bfloat16()
+    channels, around = b * hkv * dim, 4096
+    buffer = torch.full((around + channels * padded + around,), 77, dtype=torch.int8, device="cuda")
+    scale, center = torch.empty(channels, device="cuda"), torch.empty(channels, device="cuda")
+    C = _backend._ABI
+    ws = torch.empty(C.quantize_v_workspace_size(b, hkv, lk, dim), dtype=torch.uint8, device="cuda")
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    scratch = [p(ws), ws.numel()] if entry == "quantize_v" else []
+    C._check(getattr(C.lib, f"risa_b200_{entry}")(
+        p(v), ctypes.c_void_p(buffer.data_ptr() + around), p(scale), p(center), b, hkv, lk, dim, padded,
+        v.stride(0), v.stride(1), v.stride(2), 2, int(affine), None, *scratch,
+        torch.cuda.current_stream().cuda_stream))
+    want = risa.prequantize_int8_attention(
+        torch.zeros_like(v), v, v, v_quantization="midpoint_affine" if affine else "absmax")
+    assert (buffer[:around] == 77).all() and (buffer[-around:] == 77).all()
+    codes = buffer[around:-around].view(channels, padded)
+    shared = min(padded, want.v.shape[1])
+    assert torch.equal(codes[:, :shared], want.v[:, :shared])
+    assert codes[:, shared:].count_nonzero() == 0 and want.v[:, shared:].count_nonzero() == 0
+    assert torch.equal(scale, want.v_scale) and torch.equal(center, want.v_center)
+
+
 @pytest.mark.parametrize("case", [CASES[0], CASES[3], CASES[6]])
 @pytest.mark.parametrize("affine", [False, True])
 def test_separate_entry_points_equal_the_combined_call(case, affine):
