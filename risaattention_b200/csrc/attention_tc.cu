@@ -344,12 +344,18 @@ __device__ __forceinline__ float fmax_nan(float a, float b) {
 // select per score where maxima on integers and a second pass from tensor memory need two of each.
 // The values are those of the general path on the same tile (the scaled maximum is the maximum of the
 // scaled scores), so the bits are too.
-// UNCHECKED: scores may have become +inf or NaN (a non-finite bias hides its key, whatever its sign);
-// the maxima let both through, and only then are the scores gone over.
-template <bool UNCHECKED, typename Adjust>
+// UNCHECKED: scores may have become +inf or NaN, by a non-finite bias (which hides its key, whatever its
+// sign) or by non-finite operands or a bias whose product with log2(e) overflows (which do not).  The
+// maxima let both through; a warp that finds one takes the raw scores from tensor memory again, through
+// `rescore(raw, column, scale)`, which looks at each bias as the general path does.
+struct NoRescore {
+  __device__ __forceinline__ float operator()(float raw, int, float) const { return raw; }
+};
+template <bool UNCHECKED, typename Adjust, typename Rescore = NoRescore>
 __device__ __forceinline__ void softmax_tile_floats64(uint32_t tmem_row, const float (&sc)[4],
                                                       unsigned char* p_row, int swz, float2* stat,
-                                                      PackMultipliers mul, Adjust&& adjust) {
+                                                      PackMultipliers mul, Adjust&& adjust,
+                                                      Rescore&& rescore = Rescore{}) {
   uint32_t raw[64];
   tmem_load32(tmem_row, raw);
   tmem_load32(tmem_row + 32, raw + 32);
@@ -370,14 +376,30 @@ __device__ __forceinline__ void softmax_tile_floats64(uint32_t tmem_row, const f
   }
   float highest = UNCHECKED ? fmax_nan(fmax_nan(top[0], top[1]), fmax_nan(top[2], top[3]))
                             : fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
-  if (UNCHECKED && !(__float_as_uint(highest) < 0x7f800000u || __float_as_uint(highest) >= 0x80000000u)) {
+  if (UNCHECKED && __any_sync(0xffffffffu, !(highest < INFINITY))) {
+    // (one rolled copy that hands the scores back through tensor memory: the registers of the common
+    // case stay as they are)
     highest = -50000.0f;
+#pragma unroll 1
+    for (int c = 0; c < 64; c += 32) {
+      tmem_load32(tmem_row + c, raw);
+      tmem_load_wait();
+      tmem_regs_ready<32>(raw);
 #pragma unroll
-    for (int i = 0; i < 64; ++i) {
-      const uint32_t bits = __float_as_uint(x[i]);  // +inf, or NaN of either sign
-      if (bits - 0x7f800000u < 0x80000000u - 0x7f800000u || bits > 0xff800000u) x[i] = -INFINITY;
-      highest = fmaxf(highest, x[i]);
+      for (int i = 0; i < 32; ++i) {
+        const float s = rescore(static_cast<float>(int(raw[i])), c + i, sc[(i & 7) >> 1]);
+        highest = fmaxf(highest, s);
+        raw[i] = __float_as_uint(s);
+      }
+      tmem_store32(tmem_row + c, raw);
     }
+    tmem_store_wait();
+    tmem_load32(tmem_row, raw);
+    tmem_load32(tmem_row + 32, raw + 32);
+    tmem_load_wait();
+    tmem_regs_ready<64>(raw);
+#pragma unroll
+    for (int i = 0; i < 64; ++i) x[i] = __uint_as_float(raw[i]);
   }
   const float tile_m = highest - kU8Offset;
   uint32_t numer = 0;
@@ -1247,6 +1269,8 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
               for (int i = 0; i < 32; ++i)
                 if (c0 + i >= inside) x[i] = -INFINITY;
             }
+          }, [&](float raw, int column, float scale) {
+            return apply_mask(a, batch, head, row, tile * CTA_K + column, row_ok, raw, scale);
           });
         }
       } else if (kHasMasked && (!kHasUnmasked || a.mask != nullptr))

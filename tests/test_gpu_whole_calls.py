@@ -95,6 +95,37 @@ def test_mask_tiles_give_the_bits_of_the_all_paths_kernel(dtype, head_dim, k_len
     _backend._C.device_status()
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("head_dim", [64, 128, 256])
+@pytest.mark.parametrize("k_len", [64 + 1, 200, 1100])
+@pytest.mark.parametrize("what", ["largest_bias", "hiding_bias", "q", "k"])
+def test_mask_tiles_with_scores_that_are_not_finite(dtype, head_dim, k_len, what):
+    """A score that is not finite although its bias is -- infinite operands, or a bias whose product with
+    log2(e) overflows -- does not hide its key; a bias of +inf or NaN does.  As in the all-paths kernel."""
+    q, k, v = _inputs(head_dim, 300, k_len, torch.bfloat16)
+    g = torch.Generator(device="cuda").manual_seed(k_len)
+    wide = torch.randn(2, 4, 300, (k_len + 15) // 16 * 16, device="cuda", generator=g).to(dtype)
+    mask = wide[..., :k_len]
+    if what == "largest_bias":
+        mask[:, 1, 5, 7] = mask[:, 1, 140, k_len - 1] = torch.finfo(dtype).max
+        mask[:, 2, ::3, ::5] = torch.finfo(dtype).min
+    elif what == "hiding_bias":
+        mask[:, 1, 5, 7] = mask[:, 2, 299, k_len - 1] = float("inf")
+        mask[:, 1, 140, 63] = mask[:, 2, 37, 64] = float("nan")
+    else:
+        (q if what == "q" else k)[:, 1, 33, 9] = float("inf")
+    results = []
+    for path in (0, 2):
+        previous = _backend._C.set_attention_path(path)
+        try:
+            results.append(risa.int8_attention(q, k, v, attn_mask=mask, return_lse=True))
+        finally:
+            _backend._C.set_attention_path(previous)
+    for own, every in zip(*results):  # as bits: NaN equals NaN
+        assert torch.equal(own.view(torch.uint8), every.view(torch.uint8))
+    _backend._C.device_status()
+
+
 @pytest.mark.parametrize("rows", [1, 31, 32, 33, 255, 256, 257, 1024, 5000])
 @pytest.mark.parametrize("key_blocks", [1, 33, 70])
 def test_pack_selected_offsets_and_ids(rows, key_blocks):
