@@ -53,7 +53,7 @@ def int8_attention_from_host(query: torch.Tensor, key: torch.Tensor, value: torc
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     out_dtype = query.dtype
     if out is None:
-        out = torch.empty(query.shape, dtype=out_dtype, pin_memory=True)
+        out = torch.empty(query.shape, dtype=out_dtype, device="cpu", pin_memory=True)
     elif out.shape != query.shape or out.device.type != "cpu" or not out.is_contiguous():
         raise ValueError("out must be a contiguous CPU tensor of q's shape")
 

@@ -68,7 +68,7 @@ def _construct_in_pass(quantized, theta, output_layout, rows, k_blocks):
     row_offsets = torch.empty(rows + 1, dtype=torch.int32, device=device)
     storage = torch.empty(rows * k_blocks, dtype=torch.int32, device=device)
     # the kernel writes the summary to pinned host memory: no copy between its end and the read
-    summary = torch.empty(3, dtype=torch.float64, pin_memory=True)
+    summary = torch.empty(3, dtype=torch.float64, device="cpu", pin_memory=True)
     native.pack_selected(counts, bitmaps, totals, row_offsets, storage, summary, k_blocks, stream)
     torch.cuda.current_stream(device).synchronize()
     selected_mass, total_mass, selected_blocks = summary.tolist()

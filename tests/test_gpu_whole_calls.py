@@ -9,6 +9,7 @@ pytestmark = pytest.mark.gpu
 
 import risaattention_b200 as risa  # noqa: E402
 from risaattention_b200 import _backend, compare_native  # noqa: E402
+from risaattention_b200.host_pipeline import int8_attention_from_host  # noqa: E402
 
 
 def _inputs(head_dim, q_len, k_len, dtype, q_heads=4, kv_heads=2, batch=2, token_major=False):
@@ -149,3 +150,18 @@ def test_pack_selected_offsets_and_ids(rows, key_blocks):
     assert offsets.tolist() == [0] + kept.sum(-1).cumsum(0).tolist()
     assert torch.equal(ids[:total].cpu(), kept.nonzero()[:, 1].int())
     assert (ids[total:] == -1).all() and summary.tolist() == [rows, rows, total]
+
+
+def test_host_buffers_under_a_default_device_of_the_gpu():
+    """Construction reads its summary from pinned host memory, and the host pipeline returns it: both
+    name the host, so that ``torch.set_default_device`` does not move the buffer."""
+    q, k, v = _inputs(128, 300, 1500, torch.bfloat16)
+    out, pattern = risa.construct_sparse_int8_attention(q, k, v, theta=0.9)
+    host = [x.cpu().pin_memory() for x in (q, k, v)]
+    with torch.device("cuda"):
+        again, same = risa.construct_sparse_int8_attention(q, k, v, theta=0.9)
+        streamed = int8_attention_from_host(*host)
+    assert torch.equal(out, again)
+    assert torch.equal(pattern.row_offsets, same.row_offsets)
+    assert torch.equal(pattern.block_indices, same.block_indices)
+    assert not streamed.is_cuda and torch.equal(streamed, risa.int8_attention(q, k, v).cpu())
