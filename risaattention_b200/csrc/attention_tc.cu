@@ -100,7 +100,11 @@ struct SmemLayout {
   // tiles at head_dim 64 have eight of 64 columns, everything else four of 128.
   static constexpr int kBuffers = D == 64 ? 8 : 4;
   static constexpr int kBufferCols = 512 / kBuffers;
-  static constexpr int kSlots = D == 256 ? 3 : MASK == 2 ? 4 : kBuffers;  // P tiles and per-row statistics
+  // P tiles and per-row statistics.  Where the correction group takes tiles in pairs (64-key tiles of dense
+  // launches) it hands the slots of a pair back together, so three slots would leave two tiles at a time in
+  // the softmax of three groups: a head_dim-256 call of 8 heads, 130 queries and 4096 keys with a BF16
+  // mask that TMA cannot fetch took 486 us with three slots.
+  static constexpr int kSlots = D == 256 ? (CTA_K == 64 ? 4 : 3) : MASK == 2 ? 4 : kBuffers;
   static constexpr int kQBytes = kPanels * 128 * kPanelBytes;  // the Q tile
   static constexpr int kQStages =
       MODE == kDense && D != 256 && !(D == 128 && MASK == 2) ? 2 : 1;  // Q tiles held at once
