@@ -28,7 +28,8 @@
 // the row-per-thread kernel; without capture the denominator is kept in one partial instead of four.
 // Dense launches are resident: one CTA per SM walks (query block, head) units, the rings and the
 // accumulator buffers running on across units, so the next unit's loads, MMAs and softmax overlap the
-// previous unit's epilogue.  Capture and selection launch one CTA per unit.
+// previous unit's epilogue.  Launches with tile lists draw their units (SCHEDULE below).  Capture and
+// selection launch one CTA per unit.
 // Dense unmasked launches may cut the units of their last, partial wave into key-range parts (see
 // split_parts below): a part runs the same loop over its share of the key tiles and leaves its
 // unnormalised rows, maximum and denominator in scratch for tail_merge_kernel.
@@ -57,9 +58,13 @@ constexpr int kThreads = 640;
 constexpr int kSoftmaxGroups = 3;     // softmax warpgroups; tile it is handled by group it % 3
 constexpr int kIssueWarp = 16;        // producer; +1 issues Q.K^T (and owns tensor memory), +2 P.V
 constexpr int kMaxBuffers = 8;        // tensor-memory accumulator buffers (SmemLayout::kBuffers)
+constexpr int kUnitSlots = 4;         // drawn units on their way to the warps of a CTA
 // What a launch produces besides the output: nothing, the reference's capture workspace, or the
 // retained-mass selection of every query block.
 enum Mode : int { kDense = 0, kCapture = 1, kSelect = 2 };
+// How the resident CTAs of a dense launch come by their units: every gridDim.x-th one, the same with the
+// units of the last round cut into parts, or drawn one at a time (see attention_tc_kernel).
+enum Schedule : int { kRounds = 0, kSplit = 1, kDrawn = 2 };
 constexpr int kRegsLaunch = 96;        // what ptxas gives 640 threads (65536 / 640, multiple of 8)
 constexpr int kRegsSoftmax = 96, kRegsCorrection = 168, kRegsIssue = 24;
 // setmaxnreg redistributes the registers the CTA was launched with (threads x launch count); a
@@ -139,10 +144,13 @@ struct SmemLayout {
   static constexpr int out_stage = MODE == kDense ? v_affine + 2 * 128 * 4 : k;
   static constexpr int bars = v_affine + 2 * 128 * 4 +
                               (MODE == kDense ? 4 * 32 * kOutPitch * 16 : 0);  // 8-byte mbarriers
-  static constexpr int n_bars = 1 + 2 * kKStages + 2 * kVStages + 6 * kMaxBuffers + 2 + 3 + 6;
+  static constexpr int n_bars =
+      4 + 2 * kKStages + 2 * kVStages + 6 * kMaxBuffers + 2 * kSoftmaxGroups + 2 + 1 + 2 * kUnitSlots;
   static constexpr int tmem_slot = bars + n_bars * 8;
   static constexpr int gave_up = tmem_slot + 8;            // site of the first expired wait, or 0
-  static constexpr int total = tmem_slot + 16;
+  static constexpr int response = (tmem_slot + 16 + 15) & ~15;  // of a request for a pending CTA
+  static constexpr int units = response + 16;              // int [kUnitSlots]: drawn units
+  static constexpr int total = units + 4 * kUnitSlots;
   static constexpr size_t bytes = total + 1024;            // room to align the base to 1024
 };
 template <int MODE>
@@ -216,7 +224,9 @@ struct Bars {
                        SLOTFREE = PFULL + kMaxBuffers, OFULL = SLOTFREE + kMaxBuffers,
                        WFULL = OFULL + kMaxBuffers,
                        MFULL = WFULL + kMaxBuffers, MEMPTY = MFULL + kSoftmaxGroups,
-                       PAIRS = MEMPTY + kSoftmaxGroups;  // two: the selection epilogue's bulk copies
+                       PAIRS = MEMPTY + kSoftmaxGroups,  // two: the selection epilogue's bulk copies
+                       DRAWN = PAIRS + 2,                // answer to a request for a pending CTA
+                       UNITFULL = DRAWN + 1, UNITEMPTY = UNITFULL + kUnitSlots;
   // Tile it owns accumulator buffer it % kBuffers of tensor memory for its whole life: Q.K^T writes the
   // scores there (SFULL), the softmax group reads them, P.V then overwrites the same columns with the
   // tile's integer output (OFULL) and the correction group hands the buffer back once it has it in
@@ -725,13 +735,21 @@ __device__ __forceinline__ void softmax_tile_general(const AttentionArgs& a, int
 // -> 75.  Capture and selection use the idle rings after their last tile and keep a CTA per unit.
 // SPLIT: some units are key-range parts of a (query block, head) pair (an instantiation of its own:
 // the part's bookkeeping costs the tile loop registers, 75 -> 88 us in the last of the cases above).
-template <int MODE, int CTA_K, int D, int VARIANT = 0, bool SPLIT = false>
+// SCHEDULE: units of equal or known length are taken in rounds.  Where lengths are not known (tile lists)
+// a CTA draws its next unit: the grid has one CTA per unit, and the resident ones call off the launch of
+// CTAs that are still waiting and take their units (cluster launch control), so that, as with a CTA per
+// unit, the first SM to be free goes on.  Attention of 16 heads over 8192 keys, rows that keep 10 to 90 %
+// of their tiles: 320 us in rounds, 255 drawn; one row in twenty nearly full, the others at 10 %: 204 and
+// 130; all rows at half: 224 and 226.  (A CTA per unit: 282, 153 and 255.)
+template <int MODE, int CTA_K, int D, int VARIANT = 0, int SCHEDULE = kRounds>
 __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_mask,
     const AttentionArgs a) {
   constexpr bool CAPTURE = MODE != kDense;  // exact per-tile statistics and denominators
   constexpr bool PERSIST = !CAPTURE;
+  constexpr bool SPLIT = SCHEDULE == kSplit, DRAWN = SCHEDULE == kDrawn;
+  static_assert(PERSIST || SCHEDULE == kRounds, "schedules are those of dense launches");
   // Which softmax paths an instantiation holds (the host picks the instantiation, launch_tc):
   // 0 every path; 1 boolean per-query masks read as bits; 2 no mask, not causal, positive scale;
   // 3 causal without mask, positive scale; 4 any other per-query mask; 5 masks broadcast over the
@@ -828,6 +846,13 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       mbar_init(bar(Bars::MFULL + i), 1);
       mbar_init(bar(Bars::MEMPTY + i), 4);
     }
+    if constexpr (DRAWN) {
+      mbar_init(bar(Bars::DRAWN), 1);
+      for (int i = 0; i < kUnitSlots; ++i) {
+        mbar_init(bar(Bars::UNITFULL + i), 1);
+        mbar_init(bar(Bars::UNITEMPTY + i), kThreads / 32);
+      }
+    }
     mbar_init_fence();
   }
   if (warp == kIssueWarp + 1) tmem_alloc(sbase + L::tmem_slot, 512);
@@ -843,17 +868,36 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
   // Steps to the CTA's next unit; every role walks the same units on its own.  `round` units and
   // `base` tiles lie behind; tile it of the unit in hand is tile base + it of the CTA's rings.
   int round = 0, base = 0;
+  // Drawn units come through a ring of slots that the Q / K producer fills; -1 ends it.  Every warp reads
+  // every slot, also after a failure.
+  auto draw = [&] {
+    const int slot = round % kUnitSlots;
+    const bool there = mbar_wait_through(bar(Bars::UNITFULL + slot), (round / kUnitSlots) & 1, gave_up,
+                                         601);
+    // (by the shuffle the compiler sees that the number is the same in all lanes, and what is derived from
+    // it stays in uniform registers: 16 bytes of spills instead of 400)
+    unit = __shfl_sync(0xffffffffu,
+                       there ? *reinterpret_cast<volatile int*>(smem + L::units + 4 * slot) : -1, 0);
+    mbar_arrive_warp(bar(Bars::UNITEMPTY + slot));
+    ++round;
+    return unit >= 0;
+  };
   auto next_unit = [&] {
     if constexpr (!PERSIST) return false;
     base += seq.n_iter;
-    ++round;
-    const int turn = (round & 1) != 0 ? int(gridDim.x) - 1 - int(blockIdx.x) : int(blockIdx.x);
-    unit = round * int(gridDim.x) + turn;
-    if (unit >= a.units) return false;
+    if constexpr (DRAWN) {
+      if (!draw()) return false;
+    } else {
+      ++round;
+      const int turn = (round & 1) != 0 ? int(gridDim.x) - 1 - int(blockIdx.x) : int(blockIdx.x);
+      unit = round * int(gridDim.x) + turn;
+      if (unit >= a.units) return false;
+    }
     place();
     seq = tile_sequence<CTA_K>(a, bh, bx, n_q, n_k, CAPTURE, part, parts);
     return true;
   };
+  bool more = true;  // false: next_unit() has said that there is none
   float2* stats = reinterpret_cast<float2*>(smem + L::stats);
   uint16_t* sums = reinterpret_cast<uint16_t*>(smem + L::sums);
 
@@ -872,7 +916,33 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       RingPos<L::kKSt> ks;
       RingPos<L::kQStages> qs;
       int q_loads = 0, k_loads = 0;
-      bool ok = true;
+      bool ok = true, asked = false;
+      // The request for the next unit goes out with the last K tile of the unit in hand: early enough for
+      // the answer to be back before the warps run out of tiles, and no unit is taken while it could
+      // still start sooner elsewhere.
+      auto ask = [&] {
+        if (elect_one()) {
+          mbar_expect_tx(bar(Bars::DRAWN), 16);
+          request_pending_cta(sbase + L::response, bar(Bars::DRAWN));
+        }
+        __syncwarp();
+        asked = true;
+      };
+      auto hand_over = [&] {
+        int next = -1;
+        if (asked && mbar_wait_through(bar(Bars::DRAWN), round & 1, gave_up, 602)) {
+          next = pending_cta(sbase + L::response);
+          fence_async_smem();  // read before the next answer is written
+        }
+        asked = false;
+        const int slot = round % kUnitSlots;
+        mbar_wait_through(bar(Bars::UNITEMPTY + slot), ((round / kUnitSlots) & 1) ^ 1, gave_up, 603);
+        if (lane == 0) {
+          *reinterpret_cast<volatile int*>(smem + L::units + 4 * slot) = next;
+          mbar_arrive(bar(Bars::UNITFULL + slot));
+        }
+        __syncwarp();
+      };
       do {
         const int n_iter = uniform(seq.n_iter), row_q = uniform(bx * 128), slab_q = uniform(int(bh)),
                   slab_k = uniform(int(kvh));
@@ -889,7 +959,9 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
         __syncwarp();
         ++q_loads;
         qs.next();
+        if (DRAWN && n_iter == 0) ask();
         for (int it = 0; it < n_iter; ++it) {
+          if (DRAWN && it == n_iter - 1) ask();
           ok = mbar_wait<true>(bar(Bars::KEMPTY + ks.stage), ks.phase ^ 1, gave_up, 101);
           if (!__all_sync(0xffffffffu, ok)) break;
           const int row0 = seq.tile(it) * CTA_K;
@@ -905,8 +977,17 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
           ks.next();
         }
         if (!__all_sync(0xffffffffu, ok)) break;
-      } while (next_unit());
+        if constexpr (DRAWN) hand_over();
+        more = next_unit();
+      } while (more);
       if (!__all_sync(0xffffffffu, ok)) {
+        // a request on its way is waited for, its unit passed on (to be marked), and the ring is ended
+        if constexpr (DRAWN) {
+          while (more) {
+            hand_over();
+            more = draw();
+          }
+        }
         // drain: every issued load must land before shared memory can be released
         for (int j = max(0, q_loads - L::kQStages); j < q_loads; ++j)
           mbar_drain(bar(Bars::QFULL + j % L::kQStages), (j / L::kQStages) & 1);
@@ -966,7 +1047,8 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
           vs.next();
         }
         if (!__all_sync(0xffffffffu, ok)) break;
-      } while (next_unit());
+        more = next_unit();
+      } while (more);
       if (!__all_sync(0xffffffffu, ok)) {
         for (int j = max(0, v_loads - L::kVSt); j < v_loads; ++j)
           mbar_drain(bar(Bars::VFULL + j % L::kVSt), (j / L::kVSt) & 1);
@@ -1019,7 +1101,8 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
         if (PERSIST && elect_one()) mma_commit(bar(Bars::QEMPTY + qs.stage));
         __syncwarp();
         qs.next();
-      } while (next_unit());
+        more = next_unit();
+      } while (more);
     } else if (warp == kIssueWarp + 2) {
       // ---------------------------------------------------------------- MMA issue: P.V
       constexpr uint32_t idesc_pv = idesc_i8(false, true, L::kOut);
@@ -1052,8 +1135,11 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
           ob.next();
         }
         if (!__all_sync(0xffffffffu, ok)) break;
-      } while (next_unit());
+        more = next_unit();
+      } while (more);
     }
+    if constexpr (DRAWN)
+      while (more) more = draw();  // a role that failed still empties the ring
   } else if (wg < kSoftmaxGroups) {
     // ------------------------------------------------------------------ softmax of tiles it = wg, wg+3, ...
     // every group must end up at its constant: a group left at the launch count while another one
@@ -1379,7 +1465,11 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       }
     }
     b = it - seq.n_iter;
-    } while (ok && next_unit());
+    if (!ok) break;
+    more = next_unit();
+    } while (more);
+    if constexpr (DRAWN)
+      while (more) more = draw();
   } else {
     // ------------------------------------------------------------------ correction + epilogue
     regs_inc<kRegsCorrection>();
@@ -2037,10 +2127,10 @@ int sms_of_device(int device) {
   return sms;
 }
 
-template <int MODE, int CTA_K, int D, int VARIANT = 0, bool SPLIT = false>
+template <int MODE, int CTA_K, int D, int VARIANT = 0, int SCHEDULE = kRounds>
 int launch_tc(const AttentionArgs& a, const CUtensorMap& map_q, const CUtensorMap& map_k,
               const CUtensorMap& map_v, cudaStream_t stream, const CUtensorMap* map_mask = nullptr) {
-  auto kernel = attention_tc_kernel<MODE, CTA_K, D, VARIANT, SPLIT>;
+  auto kernel = attention_tc_kernel<MODE, CTA_K, D, VARIANT, SCHEDULE>;
   static thread_local int configured = -1;  // per instantiation, thread and device
   int device = -1;
   cudaGetDevice(&device);
@@ -2066,11 +2156,12 @@ int launch_tc(const AttentionArgs& a, const CUtensorMap& map_q, const CUtensorMa
   }
   const dim3 grid((a.q_len + 127) / 128, a.q_heads * SmemLayout<D, CTA_K, MODE, mask_ring(VARIANT)>::kHalves, a.batch);
   if constexpr (MODE == kDense) {
-    // resident CTAs, one per SM, over all units; the rest of the last round may be split into parts
+    // resident CTAs, one per SM, over all units; the rest of the last round may be split into parts.
+    // (Drawn units: one CTA per unit is launched, of which the resident ones call off most.)
     const int sms = sms_of_device(device), ctas = int(grid.x * grid.y * grid.z);
     AttentionArgs all = a;
     all.tail_begin = all.units = ctas;
-    if constexpr (SPLIT) {
+    if constexpr (SCHEDULE == kSplit) {
       const int rest = ctas % sms;
       all.tail_begin = ctas - rest;
       all.units = all.tail_begin + rest * a.tail_splits;
@@ -2078,13 +2169,17 @@ int launch_tc(const AttentionArgs& a, const CUtensorMap& map_q, const CUtensorMa
       const int parts = tail_split_factor(a, ctas, (a.k_len + CTA_K - 1) / CTA_K, sms);
       if (parts > 0) {
         all.tail_splits = parts;
-        return launch_tc<MODE, CTA_K, D, VARIANT, true>(all, map_q, map_k, map_v, stream);
+        return launch_tc<MODE, CTA_K, D, VARIANT, kSplit>(all, map_q, map_k, map_v, stream);
       }
     }
-    launch_chained(kernel, dim3(std::min(all.units, sms)), dim3(kThreads),
+    // lists give units of any length (variant 1 has none)
+    if constexpr (SCHEDULE == kRounds && VARIANT != 1)
+      if (a.row_offsets != nullptr || a.key_mask_tiles != nullptr)
+        return launch_tc<MODE, CTA_K, D, VARIANT, kDrawn>(a, map_q, map_k, map_v, stream, map_mask);
+    launch_chained(kernel, dim3(SCHEDULE == kDrawn ? all.units : std::min(all.units, sms)), dim3(kThreads),
                    SmemLayout<D, CTA_K, MODE, mask_ring(VARIANT)>::bytes, stream, map_q, map_k, map_v,
                    map_mask ? *map_mask : map_v, all);
-    if constexpr (SPLIT)
+    if constexpr (SCHEDULE == kSplit)
       launch_chained(tail_merge_kernel,
                      dim3(ctas % sms, SmemLayout<D, CTA_K, MODE, mask_ring(VARIANT)>::kOut / kMergeChannels), dim3(128), 0,
                      stream, all, SmemLayout<D, CTA_K, MODE, mask_ring(VARIANT)>::kHalves,
@@ -2178,7 +2273,7 @@ int attention_tc(const AttentionArgs& args, cudaStream_t stream, bool every_path
     // against the general path of variant 5, a batch of 4 padded sequences of 1500 keys, 16 heads of
     // 80 (run as 128) channels, whole call: 531 -> 252 us
     if (reads_mask_keys_as_bits(a))
-      return launch_tc<kDense, K, HD, 7>(a, map_q, map_k, map_v, stream);
+      return launch_tc<kDense, K, HD, 7, kDrawn>(a, map_q, map_k, map_v, stream);
     if (a.mask != nullptr)
       return a.mask_stride_q == 0 ? launch_tc<kDense, K, HD, 5>(a, map_q, map_k, map_v, stream)
                                   : launch_tc<kDense, K, HD, 4>(a, map_q, map_k, map_v, stream);

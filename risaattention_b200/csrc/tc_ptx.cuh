@@ -117,6 +117,23 @@ __device__ __forceinline__ bool mbar_drain(uint32_t bar, uint32_t parity,
   }
 }
 
+// The same limit for a hand-over that must be completed also after a failure (the give-up word does not
+// end it); expiring, it records its site and raises the give-up word.
+__device__ __forceinline__ bool mbar_wait_through(uint32_t bar, uint32_t parity, uint32_t gave_up,
+                                                  unsigned int site) {
+  uint32_t start, now;
+  asm volatile("mov.u32 %0, %globaltimer_lo;" : "=r"(start));
+  do {
+#pragma unroll 1
+    for (int i = 0; i < 16; ++i)
+      if (mbar_try_wait(bar, parity)) return true;
+    asm volatile("mov.u32 %0, %globaltimer_lo;" : "=r"(now));
+  } while (now - start < uint32_t(kWaitLimitNs));
+  atomicCAS(&g_wait_status, 0u, site);
+  asm volatile("st.volatile.shared::cta.u32 [%0], %1;" ::"r"(gave_up), "r"(site) : "memory");
+  return false;
+}
+
 // Waits for several phases at once: the tests are issued back to back so their latencies overlap
 // (in steady state all of them are already complete), then any that failed is waited for in turn.
 template <bool SPIN = false>
@@ -210,6 +227,34 @@ __device__ __forceinline__ void l2_prefetch_run(const void* address, uint32_t by
 }
 __device__ __forceinline__ void tma_prefetch_descriptor(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
+
+// ---- cluster launch control -----------------------------------------------------------------------
+// Asks the hardware to call off the launch of a CTA of this grid that has not started and to hand its
+// index to this one: 16 bytes arrive at `response` (shared memory, 16-byte aligned) and complete on the
+// mbarrier.  After an answer without an index no further request may be made.
+__device__ __forceinline__ void request_pending_cta(uint32_t response, uint32_t bar) {
+  asm volatile(
+      "clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+      ::"r"(response), "r"(bar)
+      : "memory");
+}
+// blockIdx.x of the CTA that was called off, or -1 if there was none.
+__device__ __forceinline__ int pending_cta(uint32_t response) {
+  int index;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      ".reg .b128 r;\n"
+      "ld.shared::cta.b128 r, [%1];\n"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n"
+      "mov.b32 %0, -1;\n"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, r;\n"
+      "}\n"
+      : "=r"(index)
+      : "r"(response)
+      : "memory");
+  return index;
 }
 
 // ---- tensor memory --------------------------------------------------------------------------------

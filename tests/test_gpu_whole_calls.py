@@ -165,3 +165,71 @@ def test_host_buffers_under_a_default_device_of_the_gpu():
     assert torch.equal(pattern.row_offsets, same.row_offsets)
     assert torch.equal(pattern.block_indices, same.block_indices)
     assert not streamed.is_cuda and torch.equal(streamed, risa.int8_attention(q, k, v).cpu())
+
+
+def _rows_of_any_length(heads, q_len, k_len, cta_k, scale, seed):
+    """A pattern whose rows keep from one tile to all of them."""
+    g = torch.Generator().manual_seed(seed)
+    q_blocks, tiles = -(-q_len // 128), -(-k_len // cta_k)
+    rows = heads * q_blocks
+    counts = torch.randint(1, tiles + 1, (rows,), generator=g)
+    kept = torch.rand(rows, tiles, generator=g).argsort(1).argsort(1) < counts[:, None]
+    offsets = torch.cat([torch.zeros(1, dtype=torch.long), counts.cumsum(0)])
+    return [risa.RetainedMassPattern(
+        row_offsets=(offsets[first:last + 1] - offsets[first]).int().cuda(),
+        block_indices=kept[first:last].nonzero()[:, 1].int().cuda(), batch_size=1,
+        q_heads=(last - first) // q_blocks, q_length=q_len, kv_length=k_len, query_block_size=128,
+        key_block_size=cta_k, attention_scale=scale, retained_mass_target=0.9,
+        measured_retained_mass=0.9)
+        for first, last in [(0, rows), *((h * q_blocks, (h + 1) * q_blocks) for h in range(heads))]]
+
+
+@pytest.mark.parametrize("head_dim,q_len,k_len", [(64, 300, 1000), (128, 700, 1500), (128, 300, 700),
+                                                  (256, 500, 1300), (128, 100, 4000)])
+def test_units_of_any_length_are_drawn(head_dim, q_len, k_len):
+    """Pattern rows of one to all tiles over many more units than SMs, on two streams at once and replayed
+    from a graph: the rows of each head alone, whose few units all start at once."""
+    heads = 150
+    q, k, v = _inputs(head_dim, q_len, k_len, torch.bfloat16, q_heads=heads, kv_heads=heads // 2, batch=1)
+    packed = risa.prequantize_int8_attention(q, k, v)
+    whole, *single = _rows_of_any_length(heads, q_len, k_len, packed.cta_k, packed.attention_scale, 5)
+    out = risa.int8_attention_from_prequantized(packed, sparse_pattern=whole)
+    for h in (0, 1, 74, 149):
+        alone = risa.sparse_int8_attention(q[:, h:h + 1], k[:, h // 2:h // 2 + 1],
+                                           v[:, h // 2:h // 2 + 1], single[h])
+        assert torch.equal(alone[0, 0], out[0, h])
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    results = []
+    for _ in range(3):
+        for stream in streams:
+            stream.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(stream):
+                results.append(risa.int8_attention_from_prequantized(packed, sparse_pattern=whole))
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        results.append(risa.int8_attention_from_prequantized(packed, sparse_pattern=whole))
+    results[-1].zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(out, x) for x in results)
+    _backend._C.device_status()
+
+
+@pytest.mark.parametrize("head_dim", [64, 128, 256])
+@pytest.mark.parametrize("dtype", [torch.bool, torch.bfloat16])
+def test_sequences_of_any_length_are_drawn(head_dim, dtype):
+    """A padded batch from no visible key at all to all of them, many units: each sequence alone."""
+    batch, q_len, k_len = 12, 400, 2100
+    q, k, v = _inputs(head_dim, q_len, k_len, torch.bfloat16, q_heads=8, kv_heads=4, batch=batch)
+    lengths = torch.tensor([2100, 0, 1, 127, 128, 129, 2099, 0, 1024, 64, 700, 2048], device="cuda")
+    mask = (torch.arange(k_len, device="cuda") < lengths[:, None])[:, None, None, :]
+    if dtype is not torch.bool:
+        mask = torch.zeros(mask.shape, device="cuda").masked_fill(~mask, float("-inf")).to(dtype)
+    out, lse = risa.int8_attention(q, k, v, attn_mask=mask, return_lse=True)
+    for i in range(batch):
+        alone, its_lse = risa.int8_attention(q[i:i + 1], k[i:i + 1], v[i:i + 1],
+                                             attn_mask=mask[i:i + 1], return_lse=True)
+        assert torch.equal(alone[0], out[i]) and torch.equal(its_lse[0], lse[i])
+    assert out[1].count_nonzero() == 0 and torch.isneginf(lse[1]).all()
+    _backend._C.device_status()
