@@ -201,7 +201,7 @@ int risa_b200_dense_attention(const void* q, const void* k, const void* v, void*
  * The same work as the entries above for callers that hold a whole call together, with three things
  * those do not have: inputs whose head dim `in_dim` (a multiple of 4) is narrower than the kernel's
  * `head_dim` are read as if padded with zeros, without a padded copy; outputs may be stored as FP32
- * (dtype_code 0: the bf16 values, `cols` channels per row); and the LSE may have a per-row shift
+ * (dtype_code 0: the bf16 values, `cols` channels per row, a multiple of 4); and the LSE may have a per-row shift
  * added where it is written.  The last two need the tensor-core kernel:
  * risa_b200_finishes_outputs() says whether it takes a shape on the calling thread.  Strides are in
  * elements, [batch, head, sequence].  No counterpart in the reference. */

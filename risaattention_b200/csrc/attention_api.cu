@@ -107,6 +107,8 @@ int run_attention(
                "risa_attention: sizes must be positive and q heads divisible by kv heads");
   RISA_REQUIRE(out_dtype_code == 1 || out_dtype_code == 2 || (out_dtype_code == 0 && out_cols > 0),
                "risa_attention: output_dtype_code must be 1 (fp16) or 2 (bf16)");
+  RISA_REQUIRE(out_dtype_code != 0 || (out_cols % 4 == 0 && out_cols <= head_dim),
+               "risa_attention: FP32 rows are a multiple of 4 channels wide, at most head_dim");
   RISA_REQUIRE(mask == nullptr || (mask_dtype_code >= 0 && mask_dtype_code <= 3),
                "risa_attention: attention mask must be bool, float16, bfloat16, or float32");
   RISA_REQUIRE(reinterpret_cast<uintptr_t>(q) % 16 == 0 && reinterpret_cast<uintptr_t>(k) % 16 == 0 &&

@@ -201,3 +201,38 @@ def test_one_call_allocation_matches_the_python_allocations(shape):
     for name in names:
         a, b = getattr(through_module, name), getattr(from_python, name)
         assert a.shape == b.shape and a.dtype == b.dtype and a.is_contiguous(), name
+
+
+@pytest.mark.parametrize("cols", [2, 6, 63, 68])
+def test_fp32_rows_of_a_width_the_kernel_cannot_store(cols):
+    """risa_b200_attend stores FP32 rows four channels at a time and none past the head dim; a width of
+    another kind is refused before anything is launched (addresses here are never followed)."""
+    import ctypes
+
+    class Operands(ctypes.Structure):
+        _fields_ = [("q", ctypes.c_void_p), ("k", ctypes.c_void_p), ("v", ctypes.c_void_p),
+                    ("q_strides", ctypes.c_int64 * 3), ("k_strides", ctypes.c_int64 * 3),
+                    ("v_strides", ctypes.c_int64 * 3),
+                    *((name, ctypes.c_int) for name in (
+                        "batch", "q_heads", "kv_heads", "q_len", "k_len", "head_dim", "in_dim",
+                        "cta_k", "dtype_code", "midpoint_affine")),
+                    ("kv_perm", ctypes.c_void_p)]
+
+    class Packed(ctypes.Structure):
+        _fields_ = [(name, ctypes.c_void_p) for name in (
+            "q_codes", "k_codes", "v_codes", "q_scale", "k_scale", "v_scale", "v_center", "anchors",
+            "workspace")] + [("workspace_bytes", ctypes.c_size_t)]
+
+    class Output(ctypes.Structure):
+        _fields_ = [("o", ctypes.c_void_p), ("o_strides", ctypes.c_int64 * 3),
+                    ("dtype_code", ctypes.c_int), ("cols", ctypes.c_int), ("lse", ctypes.c_void_p),
+                    ("lse_shift", ctypes.c_void_p)]
+
+    shape = Operands(batch=1, q_heads=1, q_len=4, kv_heads=1, k_len=256, head_dim=64, in_dim=64, cta_k=64)
+    packed = Packed(*([4096] * 9), 0)
+    out = Output(4096, (ctypes.c_int64 * 3)(4 * 64, 4 * 64, 64), 0, cols, None, None)
+    lib = _backend._ABI.lib
+    status = lib.risa_b200_attend(ctypes.byref(shape), ctypes.byref(packed), ctypes.byref(out),
+                                  ctypes.c_float(0.125), 0, None, None, -1, None, None, None, None,
+                                  ctypes.c_size_t(0), None)
+    assert status == 1 and b"multiple of 4 channels" in lib.risa_b200_last_error()
