@@ -201,8 +201,8 @@ int risa_b200_dense_attention(const void* q, const void* k, const void* v, void*
  * The same work as the entries above for callers that hold a whole call together, with three things
  * those do not have: inputs whose head dim `in_dim` (a multiple of 4) is narrower than the kernel's
  * `head_dim` are read as if padded with zeros, without a padded copy; outputs may be stored as FP32
- * (dtype_code 0: the bf16 values, `cols` channels per row, a multiple of 4); and the LSE may have a per-row shift
- * added where it is written.  The last two need the tensor-core kernel:
+ * (dtype_code 0: the bf16 values, `cols` channels per row, a multiple of 4); and the LSE may have a
+ * per-row shift added where it is written.  The last two need the tensor-core kernel:
  * risa_b200_finishes_outputs() says whether it takes a shape on the calling thread.  Strides are in
  * elements, [batch, head, sequence].  No counterpart in the reference. */
 typedef struct risa_b200_operands {
@@ -228,8 +228,9 @@ typedef struct risa_b200_attention_out {
   const float* lse_shift; /* added to lse, or NULL */
 } risa_b200_attention_out;
 int risa_b200_finishes_outputs(int head_dim, int cta_k, int k_len);
-/* Bytes of one block (256-byte aligned) that holds a call's packed operands, quantiser workspace and
- * last-wave parts; with `packed` non-NULL also fills in the addresses inside the block at `base`. */
+/* Bytes of one block (256-byte aligned) that holds a call's packed operands and quantiser workspace
+ * and, unless `tail` is NULL, its last-wave parts (a call with a mask or the causal rule has none);
+ * with `packed` non-NULL also fills in the addresses inside the block at `base`. */
 size_t risa_b200_packed_layout(const risa_b200_operands* shape, char* base, risa_b200_packed* packed,
                                void** tail, size_t* tail_bytes);
 /* lse_shift: [B,Hq,Lq] floats to receive the LSE correction of the K anchors, or NULL. */

@@ -437,10 +437,12 @@ extern "C" size_t risa_b200_packed_layout(const risa_b200_operands* shape, char*
   const size_t need = risa_b200_dense_scratch_size(shape->batch, shape->q_heads, shape->q_len,
                                                    shape->kv_heads, shape->k_len, shape->head_dim,
                                                    shape->cta_k);
-  if (need == 0 || packed == nullptr) return need;
+  if (need == 0) return 0;
   const DenseScratch s = dense_scratch_layout(shape->batch, shape->q_heads, shape->q_len,
                                               shape->kv_heads, shape->k_len, shape->head_dim,
                                               shape->cta_k);
+  const size_t bytes = tail ? s.total : s.tail;  // (the parts lie last)
+  if (packed == nullptr) return bytes;
   packed->q_codes = base + s.q_codes;
   packed->k_codes = base + s.k_codes;
   packed->v_codes = base + s.v_codes;
@@ -451,7 +453,9 @@ extern "C" size_t risa_b200_packed_layout(const risa_b200_operands* shape, char*
   packed->anchors = reinterpret_cast<int32_t*>(base + s.anchors);
   packed->workspace = base + s.v_work;
   packed->workspace_bytes = s.tail - s.v_work;
-  *tail = base + s.tail;
-  *tail_bytes = s.total - s.tail;
-  return need;
+  if (tail) {
+    *tail = base + s.tail;
+    *tail_bytes = s.total - s.tail;
+  }
+  return bytes;
 }

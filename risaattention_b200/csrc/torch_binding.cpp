@@ -606,12 +606,13 @@ py::tuple attention_call(const at::Tensor& q, const at::Tensor& k, const at::Ten
   const int64_t b = shape.batch, hq = shape.q_heads, lq = shape.q_len, dim = q.size(3);
   const bool finishes = risa_b200_finishes_outputs(head_dim, cta_k, shape.k_len) != 0;
   const Output out = output_for(q.options(), shape.dtype_code, b, hq, lq, head_dim, dim, finishes, false);
-  const size_t bytes = risa_b200_packed_layout(&shape, nullptr, nullptr, nullptr, nullptr);
-  const at::Tensor scratch = at::empty({int64_t(bytes)}, q.options().dtype(at::kByte));
-  risa_b200_packed packed;
   void* tail = nullptr;
   size_t tail_bytes = 0;
-  risa_b200_packed_layout(&shape, static_cast<char*>(scratch.data_ptr()), &packed, &tail, &tail_bytes);
+  void** parts = mask.has_value() || is_causal ? nullptr : &tail;  // only plain calls are ever cut
+  const size_t bytes = risa_b200_packed_layout(&shape, nullptr, nullptr, parts, nullptr);
+  const at::Tensor scratch = at::empty({int64_t(bytes)}, q.options().dtype(at::kByte));
+  risa_b200_packed packed;
+  risa_b200_packed_layout(&shape, static_cast<char*>(scratch.data_ptr()), &packed, parts, &tail_bytes);
   MaybeTensor lse, shift;
   if (return_lse) {
     lse = at::empty({b, hq, lq}, q.options().dtype(at::kFloat));

@@ -233,3 +233,29 @@ def test_sequences_of_any_length_are_drawn(head_dim, dtype):
         assert torch.equal(alone[0], out[i]) and torch.equal(its_lse[0], lse[i])
     assert out[1].count_nonzero() == 0 and torch.isneginf(lse[1]).all()
     _backend._C.device_status()
+
+
+def _split_shape(head_dim):
+    """160 units, 12 more than SMs, whose last ones are cut into key-range parts."""
+    q_len = 2000 if head_dim > 128 else 4000
+    kernel_dim = 256 if head_dim > 128 else 128
+    assert _backend._ABI.lib.risa_b200_attention_scratch_size(1, 5, q_len, 4000, kernel_dim, 128) > 0
+    return _inputs(head_dim, q_len, 4000, torch.float32, q_heads=5, kv_heads=5, batch=1)
+
+
+def test_calls_that_are_never_split_reserve_no_parts():
+    """The parts of a split last wave are room that only plain calls need."""
+    q, k, v = _split_shape(128)
+    parts = _backend._ABI.lib.risa_b200_attention_scratch_size(1, 5, 4000, 4000, 128, 128)
+    mask = torch.ones(1, 1, 1, 4000, dtype=torch.bool, device="cuda")
+
+    def peak(**options):
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        risa.int8_attention(q, k, v, **options)
+        return torch.cuda.max_memory_allocated() - before
+
+    plain = peak()
+    for options in ({"attn_mask": mask}, {"is_causal": True}):
+        assert peak(**options) <= plain - parts + 65536  # the tile list of the mask
