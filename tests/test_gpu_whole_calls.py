@@ -243,6 +243,22 @@ def _split_shape(head_dim):
     return _inputs(head_dim, q_len, 4000, torch.float32, q_heads=5, kv_heads=5, batch=1)
 
 
+@pytest.mark.parametrize("head_dim", [80, 128, 200, 256])
+def test_fp32_rows_and_shifted_lse_of_a_split_last_wave(head_dim):
+    """The launch that merges key-range parts stores FP32 rows of the caller's width and adds the LSE
+    shift: the bits of BF16 rows converted and of the shift added afterwards."""
+    q, k, v = _split_shape(head_dim)
+
+    def calls():
+        packed = risa.prequantize_int8_attention(q, k, v, return_lse=True)
+        nhd, lse = risa.int8_attention_from_prequantized(packed, output_layout="nhd", return_lse=True)
+        return [*risa.int8_attention(q, k, v, return_lse=True), nhd, lse, risa.int8_attention(q, k, v)]
+
+    for ours, want in zip(calls(), compare_native.with_native(_backend._ABI, calls)):
+        assert ours.dtype == want.dtype and torch.equal(ours, want)
+    _backend._C.device_status()
+
+
 def test_calls_that_are_never_split_reserve_no_parts():
     """The parts of a split last wave are room that only plain calls need."""
     q, k, v = _split_shape(128)
