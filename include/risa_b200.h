@@ -244,8 +244,9 @@ int risa_b200_attend(const risa_b200_operands* shape, const risa_b200_packed* pa
                      void* stream);
 
 /* Selects which attention kernel family calls made BY THE CALLING THREAD may use: 0 = automatic
- * (tensor-core kernel where it applies, in the instantiation for the call's class: no mask / causal
- * / boolean rows / other per-query masks / masks broadcast over queries), 1 = force the
+ * (tensor-core kernel where it applies, in the instantiation for the call's class: no mask, with or
+ * without a ragged last tile / causal / boolean, FP32 and 16-bit per-query masks whose tiles TMA can
+ * fetch / other per-query masks / boolean and additive masks broadcast over queries), 1 = force the
  * row-per-thread integer kernel, whose FP32 operation order equals the reference's (the on-device
  * cross-check of the tensor-core kernel), 2 = the tensor-core kernel with every softmax path
  * compiled in, whose bits the class-specific instantiations must reproduce (a diagnostic).

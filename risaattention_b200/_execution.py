@@ -68,7 +68,7 @@ def execute_dense_attention(q, k, v, *, scale=None, attn_mask=None, use_midpoint
     if call is not None:
         return _whole_call(call, q, k, v, attn_mask, None, scale, use_midpoint_affine, is_causal,
                            False)[0]
-    # a native surface without whole calls (an older build of the library under comparison)
+    # the separate steps, for a native surface without whole calls (the ctypes one)
     input_dtype = q.dtype
     q, k, v, original_head_dim, dim = pad_head_dim(q, k, v)
     attention_scale = resolve_scale(scale, original_head_dim)

@@ -104,7 +104,7 @@ def prequantize_int8_attention(q, k, v, *, scale=None, attn_mask=None, v_quantiz
             attention_scale=attention_scale, cta_k=key_block_size, attn_mask=attn_mask,
             v_quantization=v_quantization, is_causal=is_causal, lse_shift=lse_shift,
             kv_permuted=kv_permutation is not None)
-    # a native surface without whole calls (an older build of the library under comparison)
+    # the separate steps, for a native surface without whole calls (the ctypes one)
     q, k, v, original_head_dim, _ = pad_head_dim(q, k, v)
     attention_scale = resolve_scale(scale, original_head_dim)
     key_block_size = select_key_block_size(

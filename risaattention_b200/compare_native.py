@@ -10,7 +10,10 @@ extension module (benchmarks/compare_native.py:34-152).  Here the preserved buil
 library by name, so a second copy of the *module* would resolve to the library that is already
 loaded; a second copy of the *library* opened by path through the ctypes surface
 (:class:`risaattention_b200._backend._Native`) is a separate image.  To compare like with like the
-current library is driven through the same ctypes surface.
+current library is driven through the same ctypes surface.  That surface has the separate steps only --
+quantisation of padded copies, attention, conversion to FP32, LSE shift -- so the tool compares and times
+those kernels; what the extension's whole calls add (inputs read without a padded copy, FP32 rows and
+shifted LSE from the attention kernel) is compared with the separate steps by the GPU tests.
 
     python -m risaattention_b200.compare_native --baseline-library /keep/librisa_b200.so \\
         --case 1,16,4,4096,4096,128 --include-components --report comparison.json

@@ -249,8 +249,8 @@ struct Bars {
 // score (unmasked, non-causal calls); kScoresScaled multiplies first and subtracts the maximum
 // afterwards (causal calls, for their tiles below the diagonal) -- the positive scale keeps the
 // maximum of the products equal to the product of the integer maximum.
-// KEEPBITS (with kScoresScaled): a boolean per-query mask of the row arrives as one bit per key
-// (bit i of keep[c] = key 32 c + i is visible).  Hidden scores enter the maxima as INT_MIN, which the
+// KEEPBITS (with kScoresScaled): the visible keys of a boolean mask that all queries share arrive as
+// one bit per key (bit i of keep[c] = key 32 c + i is visible).  Hidden scores enter the maxima as INT_MIN, which the
 // -50000 floor of the pre-scaled arithmetic turns into the maximum a tile without a visible key
 // has, and go into the exponent pass as -inf, so their codes are zero: the arithmetic of the
 // general path on the same tile, without the trip through floats in tensor memory.
@@ -428,12 +428,6 @@ __device__ __forceinline__ void softmax_tile_floats64(uint32_t tmem_row, const f
   *stat = make_float2(tile_m, __uint_as_float(numer));
 }
 
-// The same block with 16-byte accesses, for masks whose keys are contiguous and whose rows start on
-// 16-byte boundaries (checked by the caller): a row of the block is 32 * ESIZE bytes = LPR chunks of
-// 16 bytes, so one warp-wide request covers 32 / LPR rows, and the block travels through the
-// staging area as 16-byte chunks.  Chunk j of row r is stored at position j ^ f(r) of its row, f
-// chosen per row width so that both the stores (lanes = chunks of a few rows) and the loads (lanes
-// = rows, same chunk) touch every bank once per quarter warp.
 // 32 mask entries held as packed words -> FP32 bit patterns: the additive bias, 0 for a kept
 // boolean entry, NaN for a boolean false.
 template <int ESIZE>
@@ -456,6 +450,12 @@ __device__ __forceinline__ void mask_words_to_bits(const AttentionArgs& a,
   }
 }
 
+// A block of 32 query rows x 32 keys with 16-byte accesses, for masks whose keys are contiguous and whose
+// rows start on 16-byte boundaries (checked by the caller, mask_block_rows): a row of the block is
+// 32 * ESIZE bytes = LPR chunks of 16 bytes, so one warp-wide request covers 32 / LPR rows, and the block
+// travels through the staging area as 16-byte chunks.  Chunk j of row r is stored at position j ^ f(r) of
+// its row, f chosen per row width so that both the stores (lanes = chunks of a few rows) and the loads
+// (lanes = rows, same chunk) touch every bank once per quarter warp.
 template <int ESIZE>
 __device__ __forceinline__ void mask_block_rows_vec(const AttentionArgs& a, const char* block,
                                                     int64_t row_step_bytes, uint32_t* stage,
@@ -722,10 +722,8 @@ __device__ __forceinline__ void softmax_tile_general(const AttentionArgs& a, int
   *stat = make_float2(tile_m, __uint_as_float(numer));
 }
 
-// BOOLROWS: the instantiation for dense calls with a boolean per-query mask whose rows can be read
-// as 16-byte pieces (chosen on the host, launch_tc): their tiles take the bit form of the fast path.
-// It is a kernel of its own so that the code of every other call stays exactly as it is -- the
-// register allocation of the tile loop reacts to any path that is compiled into it.
+// VARIANT: what softmax paths are compiled in (chosen on the host, attention_tc()); a kernel of its own for
+// each class of call, because the register allocation of the tile loop reacts to any path in it.
 // PERSIST (dense launches): the CTAs stay and take one (query block, head) unit after the other, and
 // every ring and barrier runs on across units.  A CTA of its own per unit costs about 6 us besides its
 // tiles (launch, barrier and tensor-memory set-up, first loads, a pipeline that fills and drains, the
@@ -775,7 +773,8 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
   const int lane = threadIdx.x & 31;
   const int wg = warp >> 2;
   const int n_k = (a.k_len + CTA_K - 1) / CTA_K, n_q = (a.q_len + 127) / 128;
-  // Units are ordered query block fastest, then (head, half), then batch.  With a split tail, units
+  // Units are ordered query block fastest, then (head, half), then batch -- in chunks of several heads, all
+  // heads of a chunk at one query block together, where chunk_heads() says so.  With a split tail, units
   // before tail_begin are whole (query block, head) pairs, the rest come in groups of tail_splits
   // parts of one pair each.
   int bx = blockIdx.x, by = blockIdx.y, batch = blockIdx.z, part = 0, parts = 1, tail_unit = -1;

@@ -7,7 +7,7 @@
 //   * a lane owns 16 contiguous channels of a row (four vector loads, one 16-byte code store),
 //     so only the three highest Hadamard stages need warp shuffles;
 //   * one CTA quantises a whole 128-row query block or a whole key tile, with the four key scale
-//     groups of the tile spread over its warps, so no lane holds more than 64 values.
+//     groups of the tile spread over its warps, so no lane holds more than 32 values.
 // This file is compiled with --use_fast_math on purpose: the reference's scale arithmetic
 // (x / 127.f, 1.f / x) is defined by that mode's approximate division and reciprocal.
 #include "prep_v_steps.cuh"
@@ -242,9 +242,9 @@ struct KJob {
   int in_dim;  // channels the input has; the head's channels from here on are zeros
 };
 
-// One item (key tile or half of its scale groups) by k_threads(D, CTA_K) consecutive threads.  `sub` is the index of that thread group
-// inside the CTA (0 when the CTA is exactly one group) and `tid` the thread's index inside the
-// group; groups of a CTA meet only at their own named barrier.
+// One item (key tile or half of its scale groups) by k_threads(D, CTA_K) consecutive threads.  `sub` is
+// the index of that thread group inside the CTA (0 when the CTA is exactly one group) and `tid` the
+// thread's index inside the group; groups of a CTA meet only at their own named barrier.
 template <typename T, int D, int CTA_K, int ROT>
 __device__ __forceinline__ void quantize_k_tile(const KJob& job, int item, int h, int b, int sub,
                                                 int tid) {

@@ -9,8 +9,10 @@
 // CTA all tokens of 8 channels, which leaves B*Hkv*D/8 CTAs (64 at B=1, Hkv=4, D=128) for 148 SMs.
 // Here three small kernels spread every channel over many CTAs:
 //   1. range:    coalesced row reads, per-(chunk, channel) min/max into scratch;
-//   2. quantise: each CTA owns 8 channels x a 128-slot slice of the residual order, reduces the
-//                chunk ranges itself, writes codes and its slots' residual sums;
+//   2. quantise: each CTA owns 64 channels x 128-token pieces (absmax) or four windows of residual
+//                slots (midpoint-affine), reduces the chunk ranges itself, writes codes and its slots'
+//                residual sums (prep_v_steps.cuh); head dims that are not whole 64-channel blocks
+//                take a kernel of 8 channels x 128 slots per CTA;
 //   3. finish:   (midpoint-affine only) combines the residual sums in the reference order.
 // Compiled with --use_fast_math like the reference so 1.f / x and x / float(L) lower identically.
 #include "prep_v_steps.cuh"
@@ -268,7 +270,7 @@ int risa_b200::v_quantize_jobs(const void* v, void* v_codes, float* v_scale, flo
       codes->parts = p.slots / 128;  // a CTA keeps four windows of 32 residue classes
     } else {
       // CTAs repeat the range reduction of their channels, so long sequences give them up to sixteen
-      // pieces each, as long as about two CTAs per SM remain
+      // pieces each, as long as about two CTAs for each of a B200's 148 SMs remain
       const int64_t blocks = int64_t(batch) * kv_heads * (head_dim / kVChannels);
       const int pieces = (padded_len + kVPiece - 1) / kVPiece;
       codes->steps = int(std::max<int64_t>(1, std::min<int64_t>(16, pieces * blocks / 296)));

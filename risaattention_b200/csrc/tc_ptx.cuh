@@ -144,16 +144,6 @@ __device__ __forceinline__ bool mbar_wait2(uint32_t b0, uint32_t p0, uint32_t b1
   return (r0 || mbar_wait<SPIN>(b0, p0, gave_up, site)) &&
          (r1 || mbar_wait<SPIN>(b1, p1, gave_up, site + 1));
 }
-template <bool SPIN = false>
-__device__ __forceinline__ bool mbar_wait3(uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1,
-                                           uint32_t b2, uint32_t p2, uint32_t gave_up,
-                                           unsigned int site) {
-  const bool r0 = mbar_test(b0, p0), r1 = mbar_test(b1, p1), r2 = mbar_test(b2, p2);
-  if (r0 & r1 & r2) return true;
-  return (r0 || mbar_wait<SPIN>(b0, p0, gave_up, site)) &&
-         (r1 || mbar_wait<SPIN>(b1, p1, gave_up, site + 1)) &&
-         (r2 || mbar_wait<SPIN>(b2, p2, gave_up, site + 2));
-}
 
 // One lane of a converged warp.
 __device__ __forceinline__ bool elect_one() {
