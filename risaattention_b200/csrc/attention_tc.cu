@@ -2171,9 +2171,10 @@ int launch_tc(const AttentionArgs& a, const CUtensorMap& map_q, const CUtensorMa
         return launch_tc<MODE, CTA_K, D, VARIANT, kSplit>(all, map_q, map_k, map_v, stream);
       }
     }
-    // lists give units of any length (variant 1 has none)
+    // Lists give units of any length (variant 1 has none).  With no more units than SMs there is nothing to
+    // draw, and the request and its hand-over would only lengthen the launch.
     if constexpr (SCHEDULE == kRounds && VARIANT != 1)
-      if (a.row_offsets != nullptr || a.key_mask_tiles != nullptr)
+      if ((a.row_offsets != nullptr || a.key_mask_tiles != nullptr) && ctas > sms)
         return launch_tc<MODE, CTA_K, D, VARIANT, kDrawn>(a, map_q, map_k, map_v, stream, map_mask);
     launch_chained(kernel, dim3(SCHEDULE == kDrawn ? all.units : std::min(all.units, sms)), dim3(kThreads),
                    SmemLayout<D, CTA_K, MODE, mask_ring(VARIANT)>::bytes, stream, map_q, map_k, map_v,
@@ -2272,7 +2273,7 @@ int attention_tc(const AttentionArgs& args, cudaStream_t stream, bool every_path
     // against the general path of variant 5, a batch of 4 padded sequences of 1500 keys, 16 heads of
     // 80 (run as 128) channels, whole call: 531 -> 252 us
     if (reads_mask_keys_as_bits(a))
-      return launch_tc<kDense, K, HD, 7, kDrawn>(a, map_q, map_k, map_v, stream);
+      return launch_tc<kDense, K, HD, 7>(a, map_q, map_k, map_v, stream);
     if (a.mask != nullptr)
       return a.mask_stride_q == 0 ? launch_tc<kDense, K, HD, 5>(a, map_q, map_k, map_v, stream)
                                   : launch_tc<kDense, K, HD, 4>(a, map_q, map_k, map_v, stream);
