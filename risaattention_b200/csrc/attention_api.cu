@@ -314,8 +314,15 @@ struct DenseScratch {
 
 constexpr size_t align256(size_t n) { return (n + 255) & ~size_t(255); }
 
+bool dense_scratch_shape(int batch, int q_heads, int q_len, int kv_heads, int k_len, int head_dim,
+                         int cta_k) {
+  return batch > 0 && q_heads > 0 && q_len > 0 && kv_heads > 0 && k_len > 0 &&
+         (cta_k == 64 || cta_k == 128) && (head_dim == 64 || head_dim == 128 || head_dim == 256);
+}
+
+// can_split: whether the call may split its last wave (no mask, not causal).
 DenseScratch dense_scratch_layout(int batch, int q_heads, int q_len, int kv_heads, int k_len,
-                                  int head_dim, int cta_k) {
+                                  int head_dim, int cta_k, bool can_split = true) {
   const size_t n_q = (size_t(q_len) + 127) / 128, n_k = (size_t(k_len) + cta_k - 1) / cta_k;
   const size_t channels = size_t(batch) * kv_heads * head_dim;
   DenseScratch s;
@@ -331,7 +338,9 @@ DenseScratch dense_scratch_layout(int batch, int q_heads, int q_len, int kv_head
   s.anchors = take(size_t(batch) * kv_heads * sizeof(int32_t));
   s.v_work = take(risa_b200_quantize_v_workspace_size(batch, kv_heads, k_len, head_dim));
   // parts of a split last wave (attention_tc.cu); nothing for shapes the rule leaves whole
-  s.tail = take(risa_b200_attention_scratch_size(batch, q_heads, q_len, k_len, head_dim, cta_k));
+  s.tail = at;
+  if (can_split)
+    take(risa_b200_attention_scratch_size(batch, q_heads, q_len, k_len, head_dim, cta_k));
   s.total = at;
   return s;
 }
@@ -340,9 +349,7 @@ DenseScratch dense_scratch_layout(int batch, int q_heads, int q_len, int kv_head
 
 extern "C" size_t risa_b200_dense_scratch_size(int batch, int q_heads, int q_len, int kv_heads,
                                                int k_len, int head_dim, int cta_k) {
-  if (batch <= 0 || q_heads <= 0 || q_len <= 0 || kv_heads <= 0 || k_len <= 0 ||
-      (cta_k != 64 && cta_k != 128) || (head_dim != 64 && head_dim != 128 && head_dim != 256))
-    return 0;
+  if (!dense_scratch_shape(batch, q_heads, q_len, kv_heads, k_len, head_dim, cta_k)) return 0;
   return dense_scratch_layout(batch, q_heads, q_len, kv_heads, k_len, head_dim, cta_k).total;
 }
 
@@ -434,15 +441,13 @@ extern "C" size_t risa_b200_packed_layout(const risa_b200_operands* shape, char*
                                           risa_b200_packed* packed, void** tail,
                                           size_t* tail_bytes) {
   using namespace risa_b200;
-  const size_t need = risa_b200_dense_scratch_size(shape->batch, shape->q_heads, shape->q_len,
-                                                   shape->kv_heads, shape->k_len, shape->head_dim,
-                                                   shape->cta_k);
-  if (need == 0) return 0;
+  if (!dense_scratch_shape(shape->batch, shape->q_heads, shape->q_len, shape->kv_heads, shape->k_len,
+                           shape->head_dim, shape->cta_k))
+    return 0;
   const DenseScratch s = dense_scratch_layout(shape->batch, shape->q_heads, shape->q_len,
                                               shape->kv_heads, shape->k_len, shape->head_dim,
-                                              shape->cta_k);
-  const size_t bytes = tail ? s.total : s.tail;  // (the parts lie last)
-  if (packed == nullptr) return bytes;
+                                              shape->cta_k, tail != nullptr);
+  if (packed == nullptr) return s.total;
   packed->q_codes = base + s.q_codes;
   packed->k_codes = base + s.k_codes;
   packed->v_codes = base + s.v_codes;
@@ -457,5 +462,5 @@ extern "C" size_t risa_b200_packed_layout(const risa_b200_operands* shape, char*
     *tail = base + s.tail;
     *tail_bytes = s.total - s.tail;
   }
-  return bytes;
+  return s.total;
 }
