@@ -55,7 +55,7 @@ B, HQ, HKV, D = 1, 16, 4, 128
 METRIC = "dense_equiv_int8_tops_32k_full_call"
 # DRAM bytes (read + written) of one attention_tc_kernel launch from an ncu capture of this script,
 # keyed by (sequence length, query heads on the GPU); other shapes report null.
-NCU_DRAM_BYTES_PER_LAUNCH = {(32768, 16): 101901824 + 99419136}
+NCU_DRAM_BYTES_PER_LAUNCH = {(32768, 16): 101431808 + 101752576}
 # kernels the library launches for one unmasked dense call with absmax V: (K anchor + V range + Q),
 # (K + V codes), attention
 KERNELS_PER_DENSE_CALL = 3
