@@ -768,8 +768,11 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t sbase = smem_u32(smem);
   // (the shuffle tells the compiler that the warp index is the same in all lanes; the capture and
-  // selection kernels lose 2-4 % to the register allocation that follows from it)
-  const int warp = CAPTURE ? int(threadIdx.x >> 5) : __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0);
+  // selection kernels lose 2-4 % to the register allocation that follows from it, the additive masks
+  // shared by all queries on 128-key tiles 4-8 %, on 64-key tiles they gain 9 %)
+  constexpr bool kPlainWarp = CAPTURE || (KEYMASK && CTA_K == 128);
+  const int thread_warp = int(threadIdx.x >> 5);
+  const int warp = kPlainWarp ? thread_warp : __shfl_sync(0xffffffffu, thread_warp, 0);
   const int lane = threadIdx.x & 31;
   const int wg = warp >> 2;
   const int n_k = (a.k_len + CTA_K - 1) / CTA_K, n_q = (a.q_len + 127) / 128;
