@@ -1555,7 +1555,10 @@ __global__ __launch_bounds__(kThreads, 1) void attention_tc_kernel(
     };
     // 64-key tiles are taken two at a time (P.V completes in order, so the second tile's accumulator
     // stands for both): wait, hand-over and loop cost as much as the fold of such a tile.
-    constexpr int kStep = !CAPTURE && CTA_K == 64 ? 2 : 1;
+    // (Not for additive masks shared by all queries with four buffers: their softmax is long, and slots that
+    // are handed back two at a time hold it up.  32 heads of 128 channels, 1024 x 900, B2, BF16 mask: 221 us
+    // in pairs, 214 one at a time.)
+    constexpr int kStep = !CAPTURE && CTA_K == 64 && !(KEYMASK && L::kBuffers == 4) ? 2 : 1;
     for (int it = 0; it < seq.n_iter && ok; it += kStep) {
       const int ring = base + it, slot = ring % L::kSlots;
       if constexpr (CAPTURE) {
